@@ -62,6 +62,10 @@ struct b2r_handle {
     bool gol_bytes = false;    // Game of Life: byte-SWAR kernel instead of bit-sliced cells
     bool adj_fused = true;     // adjoint: stress adjoint + lambda/mu gradients in one sweep
     bool gol_push = false;     // Game of Life: period-end passes fill the next period's halos (opt-in: slower so far)
+    // Game of Life on the whole domain's bit grid (gol_domain.cu): its two
+    // grids (null: no room, the block passes run) and the passes' plans
+    uint32_t* gol_grid = nullptr;
+    GolDomainPlans gol_plans;
     int gol_rows = 0;          // Game of Life several-generation pass: output rows per band at most (0 = 32)
     float* mat[3] = {};
     std::vector<float> src;     // per-step source increment of sxx/syy/szz (STAG)
@@ -78,6 +82,7 @@ struct b2r_handle {
     int* d_status = nullptr;
     long long ts = 0;
     bool halos_fresh = false;
+    bool halos_lost = false;     // stepped without the blocks' halos: a sub-step needs an exchange, mid-period too
     unsigned upmask = 0;         // fields uploaded since the last step while the halos were not fresh
     unsigned xmask = 0;          // fields exchanged by the caller at time step xts
     long long xts = -1;

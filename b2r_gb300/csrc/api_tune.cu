@@ -150,7 +150,7 @@ static b2r_status autotune_knobs(b2r_handle* h, int trial_steps, int best[3], do
     }
     const int save_cur = h->cur;
     const long long save_ts = h->ts;
-    const bool save_fresh = h->halos_fresh;
+    const bool save_fresh = h->halos_fresh, save_lost = h->halos_lost;
     // trials run as the stepping will (graph replay included, each
     // candidate's graphs captured in its warm run) and over whole periods:
     // a single period would not show what a choice costs at period ends
@@ -185,6 +185,7 @@ static b2r_status autotune_knobs(b2r_handle* h, int trial_steps, int best[3], do
     h->cur = save_cur;
     h->ts = save_ts;
     h->halos_fresh = save_fresh;
+    h->halos_lost = save_lost;
     // restore every field even after a failed trial; report the first failure
     cudaError_t rerr = cudaSuccess;
     for (int f = 0; f < nsave; ++f) {

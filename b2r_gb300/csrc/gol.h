@@ -30,6 +30,33 @@ cudaError_t launch_gol_bits_period(const uint8_t* in, uint8_t* out, const BlockL
                                    bool push_halos, cudaStream_t st, int rows = 0);
 int gol_bits_max_generations_per_pass();
 
+// gol_domain.cu: gens (>= 1) generations of the whole domain on a bit grid,
+// whatever the blocks: the interiors of `blocks` (one buffer of padded
+// blocks, updated in place; the shell is read from its edge blocks) are
+// packed into `bits` (2 * gol_domain_words words), stepped and unpacked.  The
+// halos between blocks are neither read nor written.  plans: the tiles and
+// generations per pass chosen for this domain, kept by the caller (zeroed at
+// first).
+constexpr int kGolDomainMaxGen = 8;   // generations per pass at most
+struct GolPass {
+    int nx, ny, nz, W;     // cells per axis of the bit grid (shell included), words per row
+    int periodic;
+    int G;                 // generations of this pass
+    int WX, XO, split;     // region words per row, output words, 1: a row is cut into x tiles
+    int Ty, Tz, PR, PZ;    // output rows / planes of a tile, region rows (even) / planes
+    int RP, RPZ;           // shared pitch of a row and of a plane (words)
+    int nzs;               // z segments of a CTA
+    int ntx, nty;
+    int threads;
+    size_t smem;
+};
+struct GolDomainPlans {
+    GolPass p[kGolDomainMaxGen + 1] = {};   // by generations to go (at most kGolDomainMaxGen); G = 0: not made yet
+};
+size_t gol_domain_words(const int env[3], int shell);
+cudaError_t launch_gol_domain(uint8_t* blocks, uint32_t* bits, const int env[3], int shell, const BlockLayout& L,
+                              int gens, GolDomainPlans& plans, cudaStream_t st);
+
 // z chunks per block of the several-generation pass (host side): the CTAs
 // (tiles x chunks) are dealt over `sms` SMs, the busiest SM holding
 // ceil(CTAs / sms) of them, each computing its chunk of nz planes plus about
