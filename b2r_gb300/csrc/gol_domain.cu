@@ -382,8 +382,9 @@ GolPass plan_pass(const GolPass& base, int left, int sms)
 {
     GolPass best = base;
     double best_cost = 1e300;
-    for (int G = std::min(kMaxG, left); G >= 1; --G) {
-        for (int PR = 4; PR <= kMaxPR; PR += kNR) {
+    for (int G : {4, 6, 8, 3, 5, 2, 1}) {
+        if (G > left) continue;
+        for (int PR = 4; PR <= kMaxPR; PR += PR < 24 ? kNR : 4) {
             const int Ty = PR - 2 * G;
             if (Ty < 1) continue;
             if (Ty >= base.ny + 4) break;
@@ -394,7 +395,13 @@ GolPass plan_pass(const GolPass& base, int left, int sms)
                 if (nzt > 1 && Tz == (base.nz + nzt - 2) / (nzt - 1)) continue;   // same tile as fewer chunks
                 const int PZ = Tz + 2 * G;
                 if (PZ > kMaxPZ) continue;
-                for (int nzs : {1, 2, 3, 4, 5, 6, 8, 12, 16}) {
+                if (Tz < 3 && base.nz > 8) break;
+                // no z split of this tile can beat the best so far
+                const double ctas_all = (double)base.ntx * nty * ((base.nz + Tz - 1) / Tz);
+                const double least = 6000.0 + 150.0 * G + ctas_all / sms * PR * base.WX *
+                                                              ((39.0 / 56.0) * (G * PZ - G * (G + 1)) + 0.55 * PZ);
+                if (least / G >= best_cost) continue;
+                for (int nzs : {4, 2, 3, 6, 8, 12, 16, 1}) {
                     const int th = base.WX * (PR / kNR) * nzs;
                     if (th > kMaxThreads || (nzs > 1 && Tz < nzs)) continue;
                     const size_t bytes = (size_t)2 * PZ * (PR + 2) * RP * 4;
@@ -404,18 +411,18 @@ GolPass plan_pass(const GolPass& base, int left, int sms)
                     const int fit = (int)std::min<size_t>(std::min(2048 / (warps * 32), 65536 / (warps * 32 * 64)),
                                                           (220 * 1024) / (bytes + 1024));
                     if (fit < 1) continue;
-                    long long busiest = (ctas + sms - 1) / sms;
-                    double cost = 0.0;
-                    while (busiest > 0) {
-                        const int n = (int)std::min<long long>(busiest, fit);
-                        busiest -= n;
-                        cost += (double)n * PZ * PR * base.WX * 0.55;                      // the load
+                    const long long busiest = (ctas + sms - 1) / sms;
+                    auto together = [&](int n) {   // n CTAs resident on the SM
+                        double c = (double)n * PZ * PR * base.WX * 0.55;               // the load
                         for (int g = 1; g <= G; ++g) {
                             const int sz = (PZ - 2 * g + nzs - 1) / nzs;
                             const double per = kNR * (25.0 * sz + 14.0 * (sz + 2)) + 12.0 * sz;   // per thread
-                            cost += std::max(n * warps * 32 * per / 56.0, per * 9.5) + 150.0;
+                            c += std::max(n * warps * 32 * per / 56.0, per * 9.5) + 150.0;
                         }
-                    }
+                        return c;
+                    };
+                    double cost = (double)(busiest / fit) * together(fit);
+                    if (busiest % fit) cost += together((int)(busiest % fit));
                     cost = (cost + 6000.0) / G;
                     if (cost < best_cost) {
                         best_cost = cost;
