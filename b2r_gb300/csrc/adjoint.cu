@@ -115,6 +115,7 @@ struct AdjS {
 __global__ void __launch_bounds__(kBX * kBY, B2R_EQWP_MINB)
 adj_velocity_kernel(AdjV A, const BlockLayout L, Tiles T)
 {
+    pdl_begin();
     const int nzc = T.nzc;
     const int blk = blockIdx.z / nzc, zc = blockIdx.z % nzc;
     const Win w = window(L, blk, zc, nzc, 2);
@@ -188,6 +189,7 @@ adj_velocity_kernel(AdjV A, const BlockLayout L, Tiles T)
 __global__ void __launch_bounds__(kBX * kBY, B2R_EQWP_MINB)
 adj_stress_kernel(AdjS A, const BlockLayout L, Tiles T)
 {
+    pdl_begin();
     const int nzc = T.nzc;
     const int blk = blockIdx.z / nzc, zc = blockIdx.z % nzc;
     const Win w = window(L, blk, zc, nzc, 4);
@@ -248,6 +250,7 @@ adj_stress_kernel(AdjS A, const BlockLayout L, Tiles T)
 __global__ void __launch_bounds__(kBX * kBY, B2R_EQWP_MINB)
 adj_grad_lm_kernel(AdjS A, const BlockLayout L, Tiles T)
 {
+    pdl_begin();
     const int nzc = T.nzc;
     const int blk = blockIdx.z / nzc, zc = blockIdx.z % nzc;
     const Win w = window(L, blk, zc, nzc, 4);
@@ -298,6 +301,7 @@ adj_grad_lm_kernel(AdjS A, const BlockLayout L, Tiles T)
 __global__ void __launch_bounds__(kBX * kBY, B2R_ADJ_FUSED_MINB)
 adj_stress_lm_kernel(AdjS A, const BlockLayout L, Tiles T)
 {
+    pdl_begin();
     const int nzc = T.nzc;
     const int blk = blockIdx.z / nzc, zc = blockIdx.z % nzc;
     const Win w = window(L, blk, zc, nzc, 4);
@@ -374,12 +378,14 @@ adj_stress_lm_kernel(AdjS A, const BlockLayout L, Tiles T)
 
 __global__ void rec_sample_kernel(const float* vy, const long long* idx, int nrec, float* out)
 {
+    pdl_begin();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r < nrec) out[r] = vy[idx[r]];
 }
 
 __global__ void rec_inject_kernel(float* vby, const long long* idx, int nrec, const float* res)
 {
+    pdl_begin();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r < nrec) atomicAdd(&vby[idx[r]], res[r]);
 }
@@ -418,16 +424,12 @@ inline int grid_for(long long work)
 
 cudaError_t adjoint_sample(const float* vy, const long long* d_idx, int nrec, float* out, cudaStream_t st)
 {
-    rec_sample_kernel<<<(nrec + 127) / 128, 128, 0, st>>>(vy, d_idx, nrec, out);
-    count_launches(1);
-    return cudaGetLastError();
+    return launch_pdl(rec_sample_kernel, (nrec + 127) / 128, 128, 0, st, vy, d_idx, nrec, out);
 }
 
 cudaError_t adjoint_inject(float* vby, const long long* d_idx, int nrec, const float* res, cudaStream_t st)
 {
-    rec_inject_kernel<<<(nrec + 127) / 128, 128, 0, st>>>(vby, d_idx, nrec, res);
-    count_launches(1);
-    return cudaGetLastError();
+    return launch_pdl(rec_inject_kernel, (nrec + 127) / 128, 128, 0, st, vby, d_idx, nrec, res);
 }
 
 // Reverse step n: q (from the later step) -> vb, w, g_b; then, unless n is
@@ -460,20 +462,13 @@ cudaError_t adjoint_step(float* const* tmp, const float* const* v_n, const float
     T.g_lam = g[0];
     T.g_mu = g[1];
     T.k = dt_h;
-    const Grid ga = stage_grid(L, 2), gb = stage_grid(L, 4);
-    adj_velocity_kernel<<<ga.g, ga.b, 0, st>>>(V, L, ga.t);
-    count_launches(1);
-    if (!last) {
-        if (fused) {
-            adj_stress_lm_kernel<<<gb.g, gb.b, 0, st>>>(T, L, gb.t);
-            count_launches(1);
-        } else {
-            adj_stress_kernel<<<gb.g, gb.b, 0, st>>>(T, L, gb.t);
-            adj_grad_lm_kernel<<<gb.g, gb.b, 0, st>>>(T, L, gb.t);
-            count_launches(2);
-        }
-    }
-    return cudaGetLastError();
+    // the fused sweep's CTAs are one per SM, the others B2R_EQWP_MINB
+    const Grid ga = stage_grid(L, 2), gb = stage_grid(L, 4, fused ? B2R_ADJ_FUSED_MINB : B2R_EQWP_MINB);
+    if (cudaError_t e = launch_pdl(adj_velocity_kernel, ga.g, ga.b, 0, st, V, L, ga.t)) return e;
+    if (last) return cudaSuccess;
+    if (fused) return launch_pdl(adj_stress_lm_kernel, gb.g, gb.b, 0, st, T, L, gb.t);
+    if (cudaError_t e = launch_pdl(adj_stress_kernel, gb.g, gb.b, 0, st, T, L, gb.t)) return e;
+    return launch_pdl(adj_grad_lm_kernel, gb.g, gb.b, 0, st, T, L, gb.t);
 }
 
 namespace {

@@ -11,6 +11,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <utility>
 
 #include "../../include/b2r.h"
 
@@ -138,6 +139,16 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
         : "memory");
 }
 
+// Programmatic dependent launch: wait for the launches before this one (their
+// writes are then visible), and let the next launch's CTAs take the room that
+// this one's tail leaves.  Both at the top of a kernel started by launch_pdl:
+// everything it reads or overwrites belongs to an earlier launch.
+__device__ __forceinline__ void pdl_begin()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+
 __device__ __forceinline__ void report(int* status, int code)
 {
     if (status) atomicCAS(status, 0, code);
@@ -196,6 +207,27 @@ cudaError_t kernel_setup(KernelSetup& ks, Kernel kern, int threads, size_t smem,
     if (total) *total = v * ks.sms[dev];
     return cudaSuccess;
 }
+
+#if defined(__CUDACC__)
+// Launch a kernel that starts with pdl_begin() as a programmatic dependent of
+// the launch before it on the stream.
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    count_launches(1);
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+#endif
 
 // A dynamic shared-memory limit that several launch shapes of one kernel
 // share: only ever raised, per device (the attribute belongs to the device

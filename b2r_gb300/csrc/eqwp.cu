@@ -33,6 +33,7 @@ using namespace eqk;
 __global__ void __launch_bounds__(kBX * kBY, B2R_EQWP_MINB)
 eqwp_ref_stress(FieldPtrs F, const BlockLayout L, int step_i, Tiles T, EqwpRefParams p)
 {
+    pdl_begin();
     const int nzc = T.nzc;
     const int blk = blockIdx.z / nzc, zc = blockIdx.z % nzc;
     const Win w = window(L, blk, zc, nzc, 4 * step_i + 2);
@@ -109,6 +110,7 @@ eqwp_ref_stress(FieldPtrs F, const BlockLayout L, int step_i, Tiles T, EqwpRefPa
 __global__ void __launch_bounds__(kBX * kBY, B2R_EQWP_MINB)
 eqwp_ref_velocity(FieldPtrs F, const BlockLayout L, int step_i, Tiles T, EqwpRefParams p, int ts)
 {
+    pdl_begin();
     const int nzc = T.nzc;
     const int blk = blockIdx.z / nzc, zc = blockIdx.z % nzc;
     const Win w = window(L, blk, zc, nzc, 4 * step_i + 4);
@@ -191,6 +193,7 @@ __global__ void __launch_bounds__(kBX * kBY, B2R_EQWP_MINB)
 eqwp_stag_velocity(FieldPtrs F, FieldPtrs O, MatPtrs M, const BlockLayout L, int step_i, Tiles T,
                    EqwpStagParams p, AccPtrs A)
 {
+    pdl_begin();
     const int blk = blockIdx.z / T.nzc, zc = blockIdx.z % T.nzc;
     stag_velocity_unit<ACC>(F, O, M, L, step_i, T, p, A, blk, zc, launch_pos());
 }
@@ -217,6 +220,7 @@ __global__ void __launch_bounds__(kBX * kBY, B2R_EQWP_MINB)
 eqwp_stag_stress(FieldPtrs F, FieldPtrs O, MatPtrs M, const BlockLayout L, int step_i, Tiles T,
                  EqwpStagParams p, float src_amp, int split)
 {
+    pdl_begin();
     const int blk = blockIdx.z / T.nzc, zc = blockIdx.z % T.nzc;
     const TilePos q = launch_pos();
     if (split) {
@@ -262,10 +266,8 @@ cudaError_t launch_eqwp_ref_substep(float* const* fld, const BlockLayout& L, int
     FieldPtrs F{};
     for (int f = 0; f < 10; ++f) F.p[f] = fld[f];
     const Grid ga = stage_grid(L, 4 * step_i + 2), gb = stage_grid(L, 4 * step_i + 4);
-    eqwp_ref_stress<<<ga.g, ga.b, 0, st>>>(F, L, step_i, ga.t, p);
-    eqwp_ref_velocity<<<gb.g, gb.b, 0, st>>>(F, L, step_i, gb.t, p, ts);
-    count_launches(2);
-    return cudaGetLastError();
+    if (cudaError_t e = launch_pdl(eqwp_ref_stress, ga.g, ga.b, 0, st, F, L, step_i, ga.t, p)) return e;
+    return launch_pdl(eqwp_ref_velocity, gb.g, gb.b, 0, st, F, L, step_i, gb.t, p, ts);
 }
 
 cudaError_t launch_eqwp_stag_substep(float* const* fld, float* const* mat, const BlockLayout& L,
@@ -278,10 +280,10 @@ cudaError_t launch_eqwp_stag_substep(float* const* fld, float* const* mat, const
     const Grid ga = stage_grid(L, 4 * step_i + 2), gb = stage_grid(L, 4 * step_i + 4);
     float amp = 0.f;
     if (p.src_host && ts >= 0 && ts < p.src_len) amp = p.src_host[ts];
-    eqwp_stag_velocity<false><<<ga.g, ga.b, 0, st>>>(F, F, M, L, step_i, ga.t, p, AccPtrs{});
-    eqwp_stag_stress<<<gb.g, gb.b, 0, st>>>(F, F, M, L, step_i, gb.t, p, amp, 0);
-    count_launches(2);
-    return cudaGetLastError();
+    if (cudaError_t e = launch_pdl(eqwp_stag_velocity<false>, ga.g, ga.b, 0, st, F, F, M, L, step_i, ga.t, p,
+                                   AccPtrs{}))
+        return e;
+    return launch_pdl(eqwp_stag_stress, gb.g, gb.b, 0, st, F, F, M, L, step_i, gb.t, p, amp, 0);
 }
 
 cudaError_t launch_eqwp_stag_stress(float* const* fld, float* const* mat, const BlockLayout& L, int step_i, int ts,
@@ -294,9 +296,7 @@ cudaError_t launch_eqwp_stag_stress(float* const* fld, float* const* mat, const 
     const Grid gb = stage_grid(L, 4 * step_i + 4);
     float amp = 0.f;
     if (p.src_host && ts >= 0 && ts < p.src_len) amp = p.src_host[ts];
-    eqwp_stag_stress<<<gb.g, gb.b, 0, st>>>(F, F, M, L, step_i, gb.t, p, amp, split);
-    count_launches(1);
-    return cudaGetLastError();
+    return launch_pdl(eqwp_stag_stress, gb.g, gb.b, 0, st, F, F, M, L, step_i, gb.t, p, amp, split);
 }
 
 cudaError_t launch_eqwp_stag_velocity(float* const* fld, float* const* mat, const BlockLayout& L, int step_i,
@@ -307,9 +307,7 @@ cudaError_t launch_eqwp_stag_velocity(float* const* fld, float* const* mat, cons
     MatPtrs M{};
     for (int m = 0; m < 3; ++m) M.p[m] = mat[m];
     const Grid ga = stage_grid(L, 4 * step_i + 2);
-    eqwp_stag_velocity<false><<<ga.g, ga.b, 0, st>>>(F, F, M, L, step_i, ga.t, p, AccPtrs{});
-    count_launches(1);
-    return cudaGetLastError();
+    return launch_pdl(eqwp_stag_velocity<false>, ga.g, ga.b, 0, st, F, F, M, L, step_i, ga.t, p, AccPtrs{});
 }
 
 cudaError_t launch_eqwp_stag_step_replay(const float* const* v_in, float* const* s, float* const* v_out,
@@ -329,11 +327,9 @@ cudaError_t launch_eqwp_stag_step_replay(const float* const* v_in, float* const*
     const Grid ga = stage_grid(L, 2), gb = stage_grid(L, 4);
     float amp = 0.f;
     if (p.src_host && ts >= 0 && ts < p.src_len) amp = p.src_host[ts];
-    eqwp_stag_velocity<true><<<ga.g, ga.b, 0, st>>>(F, O, M, L, 0, ga.t, p, A);
+    if (cudaError_t e = launch_pdl(eqwp_stag_velocity<true>, ga.g, ga.b, 0, st, F, O, M, L, 0, ga.t, p, A)) return e;
     // the stress stage reads the new velocities and updates the stresses in place
-    eqwp_stag_stress<<<gb.g, gb.b, 0, st>>>(O, O, M, L, 0, gb.t, p, amp, 0);
-    count_launches(2);
-    return cudaGetLastError();
+    return launch_pdl(eqwp_stag_stress, gb.g, gb.b, 0, st, O, O, M, L, 0, gb.t, p, amp, 0);
 }
 
 }  // namespace b2r

@@ -358,17 +358,41 @@ struct Grid {
     Tiles t;
 };
 
-#ifndef B2R_EQWP_CTAS
-#define B2R_EQWP_CTAS 24    // CTAs per SM a stage launch aims at (z chunks of the tiles)
-#endif
-#ifndef B2R_EQWP_ZMIN
-#define B2R_EQWP_ZMIN 16    // planes per z chunk at least
-#endif
+// Planes per z chunk of a stage launch of `tiles` tiles of nz planes.  A CTA
+// costs its SM about 0.8 us to start a chunk and 1.1 us per plane (0.55 us of
+// L1 wavefronts and the latency of a plane's loads), two resident ones 2.05
+// us per plane of both; the busiest SM holds ceil(CTAs / SMs) of them.  The
+// chunk length with the least busy busiest SM, at most 8 planes: longer
+// chunks lose the L2 hits between neighbouring tiles, until the launch is so
+// large (24 CTAs of 16 planes per SM) that the planes read twice by
+// neighbouring chunks cost more (512x512x256 in four blocks: 154 ms per 100
+// steps with 16 planes, 155.6 with 8).  Measured us per
+// elastic-wave step (two stages) against chunks of at least 16 planes: 32^3
+// 12.5 from 45, 64^3 13 from 49, 96^3 23 from 49, 128^3 56 from 82, 192^3 172
+// from 194, 256^3 361 from 388 (by planes 1, 2, 3, 4, 6, 8, 12, 16 there:
+// 426, 402, 370, 360, 354, 361, 373, 388).  per_sm: resident CTAs per SM.
+inline int stage_chunk(long long tiles, int nz, int per_sm)
+{
+    if (tiles * ((nz + 15) / 16) >= 24 * 152) return 16;
+    int best = 1;
+    double least = 1e300;
+    for (int lz = 1; lz <= 8 && lz <= nz; ++lz) {
+        const long long q = (tiles * ((nz + lz - 1) / lz) + 151) / 152;
+        const double alone = 0.85 + 1.1 * lz, pair = 0.75 + 2.05 * lz;
+        const double cost = per_sm >= 2 ? (q / 2) * pair + (q % 2) * alone : q * alone;
+        if (cost < least) {
+            least = cost;
+            best = lz;
+        }
+    }
+    return best;
+}
+
 #ifndef B2R_EQWP_YHALO
 #define B2R_EQWP_YHALO 0    // cost of a re-read halo row against a computed row, percent (0 measured best)
 #endif
 
-inline Grid stage_grid(const BlockLayout& L, int shrink)
+inline Grid stage_grid(const BlockLayout& L, int shrink, int per_sm = B2R_EQWP_MINB)
 {
     int lo[3] = {1 << 30, 1 << 30, 1 << 30}, hi[3] = {-1, -1, -1};
     for (int b = 0; b < L.nblk; ++b) {
@@ -406,12 +430,9 @@ inline Grid stage_grid(const BlockLayout& L, int shrink)
     const int tx = std::max(1, (G4 + bx - 1) / bx);
     const int ty = std::max(1, (Hy + by - 1) / by);
     const long long tiles = (long long)tx * ty * L.nblk;
-    const long long want = 152LL * B2R_EQWP_CTAS;
-    int nzc = (int)((want + tiles - 1) / tiles);
-    int maxc = (hi[2] - lo[2] + 1) / B2R_EQWP_ZMIN;
-    if (maxc < 1) maxc = 1;
-    if (nzc > maxc) nzc = maxc;
-    if (nzc < 1) nzc = 1;
+    const int nz = std::max(1, hi[2] - lo[2] + 1);
+    const int lz = stage_chunk(tiles, nz, per_sm);
+    const int nzc = (nz + lz - 1) / lz;
     r.t.nzc = nzc;
     r.g = dim3(tx, ty, L.nblk * nzc);
     return r;
