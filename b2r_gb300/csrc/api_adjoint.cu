@@ -69,7 +69,7 @@ b2r_status b2r_eqwp_misfit_gradient(b2r_handle* h, int nsteps, int nrec, const i
     b2r_status st;
     if ((st = adj_check(h)) != B2R_OK) return st;
     if (nsteps <= 0 || nrec <= 0 || !rec_xyz || !d_obs) return fail(h, B2R_ERR_ARG, "invalid receivers / steps");
-    const int K = ckpt_every > 0 ? ckpt_every : nsteps;
+    const int K = ckpt_every > 0 ? std::min(ckpt_every, nsteps) : nsteps;
     std::vector<long long> idx;
     if ((st = rec_offsets(h, nrec, rec_xyz, idx)) != B2R_OK) return st;
     const size_t fb = field_bytes(h);
@@ -280,13 +280,17 @@ b2r_status b2r_heat_record(b2r_handle* h, int nsteps, int nrec, const int* rec_x
     CK(h, cudaMalloc(&d_rec.p, sizeof(float) * (size_t)nrec * (nsteps > 0 ? nsteps : 1)));
     CK(h, cudaMemcpyAsync(d_idx.p, idx.data(), sizeof(long long) * nrec, cudaMemcpyHostToDevice, h->stream));
     const HeatLap c = heat_lap_of(h);
-    for (int n = 0; n < nsteps; ++n) {
-        float* in = static_cast<float*>(h->buf[h->cur]);
-        float* out = static_cast<float*>(h->buf[1 - h->cur]);
-        CK(h, launch_heat_kappa_step(in, out, h->mat[0], h->L, h->cfg.D, c, h->stream));
+    const long long* didx = (const long long*)d_idx.p;
+    float* rec = (float*)d_rec.p;
+    for (int n = 0; n < nsteps; ++n) {   // a step samples the receivers of the one before
+        CK(h, launch_heat_kappa_step(static_cast<float*>(h->buf[h->cur]), static_cast<float*>(h->buf[1 - h->cur]),
+                                     h->mat[0], h->L, h->cfg.D, c, didx, nrec,
+                                     n > 0 ? rec + (size_t)(n - 1) * nrec : nullptr, h->stream));
         h->cur = 1 - h->cur;
-        CK(h, adjoint_sample(out, (const long long*)d_idx.p, nrec, (float*)d_rec.p + (size_t)n * nrec, h->stream));
     }
+    if (nsteps > 0)
+        CK(h, adjoint_sample(static_cast<float*>(h->buf[h->cur]), didx, nrec, rec + (size_t)(nsteps - 1) * nrec,
+                             h->stream));
     h->ts += nsteps;
     CK(h, cudaMemcpyAsync(d_out, d_rec.p, sizeof(float) * (size_t)nrec * nsteps, cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
@@ -300,15 +304,20 @@ b2r_status b2r_heat_misfit_gradient(b2r_handle* h, int nsteps, int nrec, const i
     b2r_status st;
     if ((st = heat_adj_check(h)) != B2R_OK) return st;
     if (nsteps <= 0 || nrec <= 0 || !rec_xyz || !d_obs) return fail(h, B2R_ERR_ARG, "invalid receivers / steps");
-    const int K = ckpt_every > 0 ? ckpt_every : nsteps;
+    const int K = ckpt_every > 0 ? std::min(ckpt_every, nsteps) : nsteps;
     std::vector<long long> idx;
     if ((st = rec_offsets(h, nrec, rec_xyz, idx)) != B2R_OK) return st;
     const size_t fb = field_bytes(h);
     const size_t nseg = (size_t)(nsteps + K - 1) / K;
-    // workspace on the handle: checkpoints, replay slots 1..K, lam, y, FP64 gradient
-    const size_t fba = (fb + 255) & ~(size_t)255;
-    const size_t gba = ((size_t)h->L.bstride * sizeof(double) + 255) & ~(size_t)255;
-    const size_t need = (nseg + (size_t)K + 1 + 2) * fba + gba;
+    // workspace on the handle: checkpoints 1 .. nseg-1 (checkpoint 0 is the
+    // caller's field, which no step overwrites), segment states 1 .. K, lam,
+    // two y buffers, the FP64 gradient as stored and as returned, receivers
+    const auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t fba = up(fb), gb = (size_t)h->L.bstride * sizeof(double);
+    const size_t ncell = (size_t)h->cfg.env[0] * h->cfg.env[1] * h->cfg.env[2];
+    const size_t nstate = (nseg - 1) + (size_t)K;
+    const size_t rb = up(sizeof(float) * (size_t)nrec * nsteps), ib = up(sizeof(long long) * nrec);
+    const size_t need = (nstate + 3) * fba + up(gb) + up(ncell * sizeof(double)) + 2 * rb + ib;
     if (h->adj_ws_bytes < need) {
         if (h->adj_ws) cudaFree(h->adj_ws);
         h->adj_ws = nullptr;
@@ -320,40 +329,46 @@ b2r_status b2r_heat_misfit_gradient(b2r_handle* h, int nsteps, int nrec, const i
         h->adj_ws_bytes = need;
     }
     char* ws = static_cast<char*>(h->adj_ws);
-    std::vector<float*> ckpt(nseg), slot((size_t)K + 1);
-    for (auto& p : ckpt) p = reinterpret_cast<float*>(ws), ws += fba;
-    for (auto& p : slot) p = reinterpret_cast<float*>(ws), ws += fba;
-    float* lam = reinterpret_cast<float*>(ws);
-    ws += fba;
-    float* yb = reinterpret_cast<float*>(ws);
-    ws += fba;
-    double* g = reinterpret_cast<double*>(ws);
-    CK(h, cudaMemsetAsync(lam, 0, fb, h->stream));
-    CK(h, cudaMemsetAsync(yb, 0, fb, h->stream));
-    CK(h, cudaMemsetAsync(g, 0, (size_t)h->L.bstride * sizeof(double), h->stream));
-    // shell cells never change: every replay slot starts as the initial state
-    for (size_t k = 1; k < slot.size(); ++k)
-        CK(h, cudaMemcpyAsync(slot[k], h->buf[h->cur], fb, cudaMemcpyDeviceToDevice, h->stream));
-    DevBuf d_idx, d_rec, d_res;
-    CK(h, cudaMalloc(&d_idx.p, sizeof(long long) * nrec));
-    CK(h, cudaMalloc(&d_rec.p, sizeof(float) * (size_t)nrec * nsteps));
-    CK(h, cudaMalloc(&d_res.p, sizeof(float) * (size_t)nrec * nsteps));
-    CK(h, cudaMemcpyAsync(d_idx.p, idx.data(), sizeof(long long) * nrec, cudaMemcpyHostToDevice, h->stream));
-    const long long* didx = (const long long*)d_idx.p;
+    auto carve = [&](size_t bytes) {
+        char* p = ws;
+        ws += bytes;
+        return p;
+    };
+    float* const u0 = static_cast<float*>(h->buf[h->cur]);
+    float* const states = reinterpret_cast<float*>(carve(nstate * fba));
+    const long long fstride = (long long)(fba / sizeof(float));
+    auto ckpt = [&](long long sgi) { return sgi == 0 ? u0 : states + (sgi - 1) * fstride; };
+    auto slot = [&](int k) { return states + ((long long)nseg - 1 + k - 1) * fstride; };   // k = 1 .. K
+    float* const lam = reinterpret_cast<float*>(carve(fba));
+    float* yb[2];
+    for (float*& b : yb) b = reinterpret_cast<float*>(carve(fba));
+    double* const g = reinterpret_cast<double*>(carve(up(gb)));
+    double* const d_out = reinterpret_cast<double*>(carve(up(ncell * sizeof(double))));
+    float* const d_rec = reinterpret_cast<float*>(carve(rb));
+    float* const d_res = reinterpret_cast<float*>(carve(rb));
+    long long* const didx = reinterpret_cast<long long*>(carve(ib));
+    CK(h, cudaMemsetAsync(lam, 0, 3 * fba, h->stream));   // and both y
+    CK(h, cudaMemsetAsync(g, 0, gb, h->stream));
+    CK(h, cudaMemcpyAsync(didx, idx.data(), sizeof(long long) * nrec, cudaMemcpyHostToDevice, h->stream));
     const HeatLap c = heat_lap_of(h);
     const int D = h->cfg.D;
+    // shell cells never change: every state has the initial one's
+    CK(h, launch_heat_shell(u0, states, fstride, (int)nstate, h->L, D, h->stream));
 
-    // forward with checkpoints and receiver samples
-    for (int n = 0; n < nsteps; ++n) {
-        float* in = static_cast<float*>(h->buf[h->cur]);
-        float* out = static_cast<float*>(h->buf[1 - h->cur]);
-        if (n % K == 0) CK(h, cudaMemcpyAsync(ckpt[n / K], in, fb, cudaMemcpyDeviceToDevice, h->stream));
-        CK(h, launch_heat_kappa_step(in, out, h->mat[0], h->L, D, c, h->stream));
-        h->cur = 1 - h->cur;
-        CK(h, adjoint_sample(out, didx, nrec, (float*)d_rec.p + (size_t)n * nrec, h->stream));
-    }
+    // forward: state n is a checkpoint at multiples of K, its segment's slot
+    // in the last segment (which needs no replay), and one of two slots in
+    // turn otherwise; a step samples the receivers of the one before
+    const int n_last = (int)(nseg - 1) * K;
+    auto state = [&](int n) {
+        if (n % K == 0 && n < nsteps) return ckpt(n / K);
+        return slot(n > n_last ? n - n_last : 1 + n % 2);
+    };
+    for (int n = 0; n < nsteps; ++n)
+        CK(h, launch_heat_kappa_step(state(n), state(n + 1), h->mat[0], h->L, D, c, didx, nrec,
+                                     n > 0 ? d_rec + (size_t)(n - 1) * nrec : nullptr, h->stream));
+    CK(h, adjoint_sample(state(nsteps), didx, nrec, d_rec + (size_t)(nsteps - 1) * nrec, h->stream));
     std::vector<float> syn((size_t)nrec * nsteps), res((size_t)nrec * nsteps);
-    CK(h, cudaMemcpyAsync(syn.data(), d_rec.p, sizeof(float) * syn.size(), cudaMemcpyDeviceToHost, h->stream));
+    CK(h, cudaMemcpyAsync(syn.data(), d_rec, sizeof(float) * syn.size(), cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
     double J = 0.0;
     for (size_t i = 0; i < syn.size(); ++i) {
@@ -363,26 +378,27 @@ b2r_status b2r_heat_misfit_gradient(b2r_handle* h, int nsteps, int nrec, const i
     }
     if (misfit) *misfit = J;
     if (d_syn) std::copy(syn.begin(), syn.end(), d_syn);
-    CK(h, cudaMemcpyAsync(d_res.p, res.data(), sizeof(float) * res.size(), cudaMemcpyHostToDevice, h->stream));
+    CK(h, cudaMemcpyAsync(d_res, res.data(), sizeof(float) * res.size(), cudaMemcpyHostToDevice, h->stream));
 
-    // reverse sweep, segment by segment with recomputation
+    // reverse sweep, segment by segment, each but the last replayed first
+    int cur = 0;   // y buffer of the step
     for (long long sgi = (long long)nseg - 1; sgi >= 0; --sgi) {
         const int n0 = (int)sgi * K;
         const int n1 = std::min(nsteps, n0 + K);
-        auto u_at = [&](int k) -> float* { return k == 0 ? ckpt[sgi] : slot[(size_t)k]; };
-        for (int n = n0; n < n1; ++n)
-            CK(h, launch_heat_kappa_step(u_at(n - n0), u_at(n - n0 + 1), h->mat[0], h->L, D, c, h->stream));
+        auto u_at = [&](int k) { return k == 0 ? ckpt(sgi) : slot(k); };
+        if (sgi < (long long)nseg - 1)
+            for (int n = n0; n + 1 < n1; ++n)
+                CK(h, launch_heat_kappa_step(u_at(n - n0), u_at(n - n0 + 1), h->mat[0], h->L, D, c, didx, 0, nullptr,
+                                             h->stream));
         for (int n = n1 - 1; n >= n0; --n) {
-            CK(h, adjoint_inject(lam, didx, nrec, (const float*)d_res.p + (size_t)n * nrec, h->stream));
-            CK(h, launch_heat_adjoint_step(lam, yb, u_at(n - n0), h->mat[0], g, h->L, D, c, h->stream));
+            CK(h, launch_heat_adjoint_inject(lam, yb[cur], h->mat[0], didx, nrec, d_res + (size_t)n * nrec, h->stream));
+            CK(h, launch_heat_adjoint_step(lam, yb[cur], yb[1 - cur], u_at(n - n0), h->mat[0], g, h->L, D, c, h->stream));
+            cur = 1 - cur;
         }
     }
     if (grad_kappa) {
-        const size_t ncell = (size_t)h->cfg.env[0] * h->cfg.env[1] * h->cfg.env[2];
-        DevBuf d_out;
-        CK(h, cudaMalloc(&d_out.p, ncell * sizeof(double)));
-        CK(h, adjoint_grad_out(g, nullptr, 0, h->L, (double*)d_out.p, h->stream));
-        CK(h, cudaMemcpyAsync(grad_kappa, d_out.p, ncell * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        CK(h, adjoint_grad_out(g, nullptr, 0, h->L, d_out, h->stream));
+        CK(h, cudaMemcpyAsync(grad_kappa, d_out, ncell * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     }
     CK(h, cudaStreamSynchronize(h->stream));
     h->ts = nsteps;

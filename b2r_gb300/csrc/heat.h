@@ -16,16 +16,26 @@ HeatCoef heat_coef(int D, double alpha_dt, double dx, double dy, double dz);
 // L u = w0*u + sum_k wx[k-1]*(u[x-k]+u[x+k]) + ...; the conductivity-scaled
 // step u' = u + kappa * L u on the interior window of one block, and one
 // reverse step of its adjoint (lam: adjoint of u^{n+1}, updated to that of
-// u^n; yb: scratch, zero outside the window; g += lam * L u^n in FP64).
+// u^n; y zero outside the window; g += lam * L u^n in FP64).
 struct HeatLap {
     float w0;
     float wx[4], wy[4], wz[4];
 };
 HeatLap heat_lap(int D, double alpha_dt, double dx, double dy, double dz);
+// launch_heat_kappa_step also samples the receivers of `in` (element offsets
+// rec) into rec_out unless that is null.  launch_heat_adjoint_step: lam and g
+// in place, y = kappa * lam read, y_next written; launch_heat_adjoint_inject
+// adds the residuals at the receivers to lam and refreshes y there.
+// launch_heat_shell copies src's fixed shell into n fields `stride` elements
+// apart.
 cudaError_t launch_heat_kappa_step(const float* in, float* out, const float* kappa, const BlockLayout& L, int D,
-                                   const HeatLap& c, cudaStream_t st);
-cudaError_t launch_heat_adjoint_step(float* lam, float* yb, const float* u, const float* kappa, double* g,
-                                     const BlockLayout& L, int D, const HeatLap& c, cudaStream_t st);
+                                   const HeatLap& c, const long long* rec, int nrec, float* rec_out, cudaStream_t st);
+cudaError_t launch_heat_adjoint_step(float* lam, const float* y, float* y_next, const float* u, const float* kappa,
+                                     double* g, const BlockLayout& L, int D, const HeatLap& c, cudaStream_t st);
+cudaError_t launch_heat_adjoint_inject(float* lam, float* y, const float* kappa, const long long* rec, int nrec,
+                                       const float* res, cudaStream_t st);
+cudaError_t launch_heat_shell(const float* src, float* dst, long long stride, int n, const BlockLayout& L, int D,
+                              cudaStream_t st);
 cudaError_t launch_fill(float* p, size_t n, float v, cudaStream_t st);
 // TMA box of one ring slot (cells): width and height for radius D.
 int heat_box_w();

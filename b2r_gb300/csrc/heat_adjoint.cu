@@ -13,100 +13,190 @@
 //   y         = kappa * lam on W, 0 elsewhere
 //   lam      += L^T y = L y                   on W   (L is symmetric)
 // u^n is replayed from checkpoints every K steps.
+//
+// Measured (radius 2, 160x144x128, 200 steps, checkpoints every 50, 64
+// receivers, the whole gradient call): 10.1 ms, from 61 with a thread per
+// column over the whole z axis, the reverse step in two sweeps, and a
+// separate launch for every receiver sample.
 #include <algorithm>
 #include <vector>
 
 #include "b2r_common.cuh"
+#include "eqwp_tile.cuh"
 #include "heat.h"
 
 namespace b2r {
 
 namespace {
 
-// L u at one cell (D compile time): w0 u + sum_k (wx_k (u[x+k] + u[x-k]) +
-// wy_k (...) + wz_k (...))
-template <int D>
-__device__ __forceinline__ float lap(const float* u, long long P, long long S, const HeatLap& c)
-{
-    float acc = c.w0 * u[0];
-#pragma unroll
-    for (int k = 1; k <= D; ++k) {
-        acc += c.wx[k - 1] * (u[k] + u[-k]);
-        acc += c.wy[k - 1] * (u[k * P] + u[-k * P]);
-        acc += c.wz[k - 1] * (u[k * S] + u[-k * S]);
-    }
-    return acc;
-}
+using namespace eqk;   // a thread's 4 cells, z chunks, masked float4 reads and writes (eqwp_tile.cuh)
 
-struct Win3 {
-    int lo[3], hi[3];
+// A field whose stencil a thread needs while it marches z: the 2D+1 planes of
+// its 4 cells in a register queue, x neighbours from the float4s on both
+// sides of the row and y neighbours from the rows +-1 .. +-D, through L1.
+template <int D>
+struct LapField {
+    const float* p;            // the thread's cells in plane 0
+    float4 q[2 * D + 1];
+    __device__ __forceinline__ void begin(const float* f, int zs, long long S)
+    {
+        p = f;
+#pragma unroll
+        for (int k = 0; k < 2 * D; ++k) q[k + 1] = ld4(p + (long long)(zs - D + k) * S);
+    }
+    // L u of the 4 cells at plane z (element offset o); planes in increasing
+    // order.  w0 u + sum_k (wx_k (u[x+k] + u[x-k]) + wy_k (...) + wz_k (...)):
+    // the first x product rounded, w0 u and then every other product fused
+    // onto the running sum, in this order in every kernel.
+    __device__ __forceinline__ void lap(long long o, long long P, long long S, const HeatLap& c, float (&acc)[4])
+    {
+#pragma unroll
+        for (int k = 0; k < 2 * D; ++k) q[k] = q[k + 1];
+        q[2 * D] = ld4(p + o + D * S);
+        const float4 l = ld4(p + o - 4), m = q[D], r = ld4(p + o + 4);
+        float4 ym[D], yp[D];
+#pragma unroll
+        for (int k = 1; k <= D; ++k) {
+            ym[k - 1] = ld4(p + o - k * P);
+            yp[k - 1] = ld4(p + o + k * P);
+        }
+        const float v[12] = {l.x, l.y, l.z, l.w, m.x, m.y, m.z, m.w, r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float a = __fmaf_rn(c.w0, v[4 + j], __fmul_rn(c.wx[0], __fadd_rn(v[5 + j], v[3 + j])));
+#pragma unroll
+            for (int k = 1; k <= D; ++k) {
+                if (k > 1) a = __fmaf_rn(c.wx[k - 1], __fadd_rn(v[4 + j + k], v[4 + j - k]), a);
+                a = __fmaf_rn(c.wy[k - 1], __fadd_rn(cmp(yp[k - 1], j), cmp(ym[k - 1], j)), a);
+                a = __fmaf_rn(c.wz[k - 1], __fadd_rn(cmp(q[D + k], j), cmp(q[D - k], j)), a);
+            }
+            acc[j] = a;
+        }
+    }
 };
 
-// thread = one (x, y) column of the window, marching z
+// One conductivity-scaled step.  rec_out (may be null): the receivers of
+// `in`, that is of the step before, sampled on the way.
 template <int D>
-__global__ void heat_kappa_step_kernel(const float* __restrict__ in, float* __restrict__ out,
-                                       const float* __restrict__ kappa, const BlockLayout L, HeatLap c,
-                                       Win3 w)
+__global__ void __launch_bounds__(kBX * kBY)
+heat_kappa_step_kernel(const float* __restrict__ in, float* __restrict__ out, const float* __restrict__ kappa,
+                       const BlockLayout L, const HeatLap c, const Tiles T, const long long* __restrict__ rec, int nrec,
+                       float* __restrict__ rec_out)
 {
-    const int x = w.lo[0] + blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = w.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
-    if (x > w.hi[0] || y > w.hi[1]) return;
+    pdl_begin();
+    if (rec_out && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
+        for (int r = threadIdx.y * blockDim.x + threadIdx.x; r < nrec; r += blockDim.x * blockDim.y)
+            rec_out[r] = in[rec[r]];
+    const Win w = window(L, 0, blockIdx.z, T.nzc, L.H);
+    Cell cell;
+    if (!cell_setup(L, w, 0, cell, T.x0, T.y0)) return;
     const long long P = L.P, S = L.plane;
-    const long long col = (long long)y * P + L.xoff + x;
-    for (int z = w.lo[2]; z <= w.hi[2]; ++z) {
-        const long long i = col + (long long)z * S;
-        out[i] = in[i] + kappa[i] * lap<D>(in + i, P, S, c);
+    LapField<D> u;
+    u.begin(in + cell.base, w.zs, S);
+    for (int z = w.zs; z <= w.ze; ++z) {
+        const long long o = (long long)z * S;
+        const float4 kap = ld4(kappa + cell.base + o);
+        float a[4];
+        u.lap(o, P, S, c, a);
+        const float4 m = u.q[D];
+        const float nv[4] = {__fmaf_rn(kap.x, a[0], m.x), __fmaf_rn(kap.y, a[1], m.y), __fmaf_rn(kap.z, a[2], m.z),
+                             __fmaf_rn(kap.w, a[3], m.w)};
+        st4(out + cell.base + o, cell, nv);
     }
 }
 
-// y = kappa * lam on W (0 elsewhere, never written there); g += lam * L u^n
+// One reverse step in one sweep: with lam the adjoint of u^{n+1} (receivers
+// added) and y = kappa lam on W, 0 elsewhere,
+//     g += lam * (L u^n),  lam += L y,  y_next = kappa lam.
+// lam and g are read and written by their own thread only; y, whose stencil
+// the neighbours need, goes from one buffer to the other.  40 B per cell (u,
+// y, lam and kappa read, lam and y written, g read and written in FP64)
+// against 52 in two sweeps.
 template <int D>
-__global__ void heat_adj_y_kernel(const float* __restrict__ lam, const float* __restrict__ u,
-                                  const float* __restrict__ kappa, float* __restrict__ yb, double* g,
-                                  const BlockLayout L, HeatLap c, Win3 w)
+__global__ void __launch_bounds__(kBX * kBY, 2)
+heat_adj_step_kernel(float* __restrict__ lam, const float* __restrict__ y, float* __restrict__ y_next,
+                     const float* __restrict__ un, const float* __restrict__ kappa, double* __restrict__ g,
+                     const BlockLayout L, const HeatLap c, const Tiles T)
 {
-    const int x = w.lo[0] + blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = w.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
-    if (x > w.hi[0] || y > w.hi[1]) return;
+    pdl_begin();
+    const Win w = window(L, 0, blockIdx.z, T.nzc, L.H);
+    Cell cell;
+    if (!cell_setup(L, w, 0, cell, T.x0, T.y0)) return;
     const long long P = L.P, S = L.plane;
-    const long long col = (long long)y * P + L.xoff + x;
-    for (int z = w.lo[2]; z <= w.hi[2]; ++z) {
-        const long long i = col + (long long)z * S;
-        const float l = lam[i];
-        yb[i] = kappa[i] * l;
-        g[i] += (double)(l * lap<D>(u + i, P, S, c));
+    LapField<D> u, yb;
+    u.begin(un + cell.base, w.zs, S);
+    yb.begin(y + cell.base, w.zs, S);
+    for (int z = w.zs; z <= w.ze; ++z) {
+        const long long o = (long long)z * S;
+        const float4 kap = ld4(kappa + cell.base + o);
+        const float4 l4 = rd4(lam + cell.base + o, cell);
+        double2* gp = reinterpret_cast<double2*>(g + cell.base + o);   // x groups start on 4 elements
+        double2 g0 = make_double2(0.0, 0.0), g1 = g0;
+        if (cell.all) {
+            g0 = gp[0];
+            g1 = gp[1];
+        }
+        float au[4], ay[4];
+        u.lap(o, P, S, c, au);
+        yb.lap(o, P, S, c, ay);
+        float nl[4], ny[4];
+        double inc[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float l = cmp(l4, j);
+            inc[j] = (double)__fmul_rn(l, au[j]);
+            nl[j] = __fadd_rn(l, ay[j]);
+            ny[j] = __fmul_rn(cmp(kap, j), nl[j]);
+        }
+        st4(lam + cell.base + o, cell, nl);
+        st4(y_next + cell.base + o, cell, ny);
+        if (cell.all) {
+            gp[0] = make_double2(g0.x + inc[0], g0.y + inc[1]);
+            gp[1] = make_double2(g1.x + inc[2], g1.y + inc[3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (cell.vx[j]) g[cell.base + o + j] += inc[j];
+        }
     }
 }
 
-// lam += L y on W
-template <int D>
-__global__ void heat_adj_lam_kernel(float* __restrict__ lam, const float* __restrict__ yb, const BlockLayout L,
-                                    HeatLap c, Win3 w)
+// The residuals of a step into lam at the receivers, and y = kappa lam there
+// (one CTA: receivers that share a cell are all added before y is formed).
+__global__ void heat_adj_inject_kernel(float* lam, float* y, const float* kappa, const long long* rec, int nrec,
+                                       const float* res)
 {
-    const int x = w.lo[0] + blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = w.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
-    if (x > w.hi[0] || y > w.hi[1]) return;
-    const long long P = L.P, S = L.plane;
-    const long long col = (long long)y * P + L.xoff + x;
-    for (int z = w.lo[2]; z <= w.hi[2]; ++z) {
-        const long long i = col + (long long)z * S;
-        lam[i] += lap<D>(yb + i, P, S, c);
-    }
+    pdl_begin();
+    for (int r = threadIdx.x; r < nrec; r += blockDim.x) atomicAdd(&lam[rec[r]], res[r]);
+    __syncthreads();
+    for (int r = threadIdx.x; r < nrec; r += blockDim.x)
+        y[rec[r]] = __fmul_rn(kappa[rec[r]], *(volatile float*)&lam[rec[r]]);
 }
 
-Win3 interior(const BlockLayout& L)
+// The fixed shell of `src` (the D cells around the window on every axis, the
+// only cells outside it that a stencil reads) into n buffers `stride`
+// elements apart.  A warp takes one row of one buffer.
+__global__ void heat_shell_kernel(const float* __restrict__ src, float* __restrict__ dst, long long stride, int n,
+                                  const BlockLayout L, int D)
 {
-    Win3 w;
-    for (int a = 0; a < 3; ++a) {
-        w.lo[a] = L.H;
-        w.hi[a] = L.n[a] - 1 - L.H;
+    const int lane = threadIdx.x & 31;
+    const int lo[3] = {L.H - D, L.H - D, L.H - D};
+    const int e[3] = {L.B[0] + 2 * D, L.B[1] + 2 * D, L.B[2] + 2 * D};
+    const long long rows = (long long)e[1] * e[2] * n;
+    for (long long i = blockIdx.x * 8LL + (threadIdx.x >> 5); i < rows; i += gridDim.x * 8LL) {
+        const int y = (int)(i % e[1]);
+        const long long r = i / e[1];
+        const int z = (int)(r % e[2]);
+        const long long o = (long long)(lo[2] + z) * L.plane + (long long)(lo[1] + y) * L.P + L.xoff + lo[0];
+        float* d = dst + (r / e[2]) * stride + o;
+        const bool whole = y < D || y >= e[1] - D || z < D || z >= e[2] - D;
+        if (whole) {
+            for (int x = lane; x < e[0]; x += 32) d[x] = src[o + x];
+        } else if (lane < 2 * D) {
+            const int x = lane < D ? lane : e[0] - 2 * D + lane;
+            d[x] = src[o + x];
+        }
     }
-    return w;
-}
-
-dim3 col_grid(const Win3& w, dim3 b)
-{
-    return dim3((w.hi[0] - w.lo[0] + 1 + b.x - 1) / b.x, (w.hi[1] - w.lo[1] + 1 + b.y - 1) / b.y);
 }
 
 __global__ void fill_kernel(float* p, size_t n, float v)
@@ -154,30 +244,39 @@ HeatLap heat_lap(int D, double alpha_dt, double dx, double dy, double dz)
     }
 
 cudaError_t launch_heat_kappa_step(const float* in, float* out, const float* kappa, const BlockLayout& L, int D,
-                                   const HeatLap& c, cudaStream_t st)
+                                   const HeatLap& c, const long long* rec, int nrec, float* rec_out, cudaStream_t st)
 {
-    const Win3 w = interior(L);
-    const dim3 b(32, 8), g = col_grid(w, b);
-#define CALL(DD) heat_kappa_step_kernel<DD><<<g, b, 0, st>>>(in, out, kappa, L, c, w)
+    const Grid g = stage_grid(L, L.H);
+#define CALL(DD) return launch_pdl(heat_kappa_step_kernel<DD>, g.g, g.b, 0, st, in, out, kappa, L, c, g.t, rec, nrec, rec_out)
     B2R_HEAT_ADJ_DISPATCH(D, CALL)
 #undef CALL
-    count_launches(1);
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
-cudaError_t launch_heat_adjoint_step(float* lam, float* yb, const float* u, const float* kappa, double* g,
-                                     const BlockLayout& L, int D, const HeatLap& c, cudaStream_t st)
+cudaError_t launch_heat_adjoint_step(float* lam, const float* y, float* y_next, const float* u, const float* kappa,
+                                     double* g, const BlockLayout& L, int D, const HeatLap& c, cudaStream_t st)
 {
-    const Win3 w = interior(L);
-    const dim3 b(32, 8), gr = col_grid(w, b);
-#define CALL(DD)                                                                        \
-    do {                                                                                \
-        heat_adj_y_kernel<DD><<<gr, b, 0, st>>>(lam, u, kappa, yb, g, L, c, w);         \
-        heat_adj_lam_kernel<DD><<<gr, b, 0, st>>>(lam, yb, L, c, w);                    \
-    } while (0)
+    const Grid gr = stage_grid(L, L.H);
+#define CALL(DD) return launch_pdl(heat_adj_step_kernel<DD>, gr.g, gr.b, 0, st, lam, y, y_next, u, kappa, g, L, c, gr.t)
     B2R_HEAT_ADJ_DISPATCH(D, CALL)
 #undef CALL
-    count_launches(2);
+    return cudaSuccess;
+}
+
+cudaError_t launch_heat_adjoint_inject(float* lam, float* y, const float* kappa, const long long* rec, int nrec,
+                                       const float* res, cudaStream_t st)
+{
+    return launch_pdl(heat_adj_inject_kernel, 1, std::min(1024, (nrec + 31) / 32 * 32), 0, st, lam, y, kappa, rec, nrec,
+                      res);
+}
+
+cudaError_t launch_heat_shell(const float* src, float* dst, long long stride, int n, const BlockLayout& L, int D,
+                              cudaStream_t st)
+{
+    if (n <= 0) return cudaSuccess;
+    const long long rows = (long long)(L.B[1] + 2 * D) * (L.B[2] + 2 * D) * n;
+    heat_shell_kernel<<<(unsigned)std::min<long long>((rows + 7) / 8, 152LL * 32), 256, 0, st>>>(src, dst, stride, n, L, D);
+    count_launches(1);
     return cudaGetLastError();
 }
 
