@@ -392,7 +392,8 @@ inline int stage_chunk(long long tiles, int nz, int per_sm)
 #define B2R_EQWP_YHALO 0    // cost of a re-read halo row against a computed row, percent (0 measured best)
 #endif
 
-inline Grid stage_grid(const BlockLayout& L, int shrink, int per_sm = B2R_EQWP_MINB)
+inline Grid stage_grid(const BlockLayout& L, int shrink, int per_sm = B2R_EQWP_MINB,
+                       int (*chunk)(long long tiles, int nz, int per_sm) = stage_chunk)
 {
     int lo[3] = {1 << 30, 1 << 30, 1 << 30}, hi[3] = {-1, -1, -1};
     for (int b = 0; b < L.nblk; ++b) {
@@ -431,7 +432,7 @@ inline Grid stage_grid(const BlockLayout& L, int shrink, int per_sm = B2R_EQWP_M
     const int ty = std::max(1, (Hy + by - 1) / by);
     const long long tiles = (long long)tx * ty * L.nblk;
     const int nz = std::max(1, hi[2] - lo[2] + 1);
-    const int lz = stage_chunk(tiles, nz, per_sm);
+    const int lz = chunk(tiles, nz, per_sm);
     const int nzc = (nz + lz - 1) / lz;
     r.t.nzc = nzc;
     r.g = dim3(tx, ty, L.nblk * nzc);

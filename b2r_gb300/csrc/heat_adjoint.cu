@@ -215,6 +215,29 @@ cudaError_t launch_fill(float* p, size_t n, float v, cudaStream_t st)
     return cudaGetLastError();
 }
 
+// Planes per z chunk, as stage_chunk (eqwp_tile.cuh) with these kernels'
+// costs: a chunk's start about one plane's latency, a plane of a lone CTA
+// 1.075 and of n resident ones 0.9 + 0.175 n (per_sm of them fit).  Measured
+// on the whole gradient by forward / reverse planes: radius 2, 160x144x128,
+// 11.1 ms at 8/8, 10.2 at 6/8 and 8/6, 10.4 at 8/4; 64x72x60 2.97 at 8/8,
+// 1.90 at 1/8, 2.32 at 8/1; radius 3, 100x90x110, 3.54 at 8/8, 3.20 at 8/4,
+// 3.60 at 8/1.
+static int heat_chunk(long long tiles, int nz, int per_sm)
+{
+    int best = 1;
+    double least = 1e300;
+    for (int lz = 1; lz <= 8 && lz <= nz; ++lz) {
+        const long long q = (tiles * ((nz + lz - 1) / lz) + 151) / 152;
+        auto together = [&](long long n) { return n > 0 ? 1.0 + lz * (0.9 + 0.175 * (double)n) : 0.0; };
+        const double cost = (double)(q / per_sm) * together(per_sm) + together(q % per_sm);
+        if (cost < least) {
+            least = cost;
+            best = lz;
+        }
+    }
+    return best;
+}
+
 HeatLap heat_lap(int D, double alpha_dt, double dx, double dy, double dz)
 {
     static const double cw[5][5] = {
@@ -246,7 +269,7 @@ HeatLap heat_lap(int D, double alpha_dt, double dx, double dy, double dz)
 cudaError_t launch_heat_kappa_step(const float* in, float* out, const float* kappa, const BlockLayout& L, int D,
                                    const HeatLap& c, const long long* rec, int nrec, float* rec_out, cudaStream_t st)
 {
-    const Grid g = stage_grid(L, L.H);
+    const Grid g = stage_grid(L, L.H, D <= 2 ? 4 : 3, heat_chunk);
 #define CALL(DD) return launch_pdl(heat_kappa_step_kernel<DD>, g.g, g.b, 0, st, in, out, kappa, L, c, g.t, rec, nrec, rec_out)
     B2R_HEAT_ADJ_DISPATCH(D, CALL)
 #undef CALL
@@ -256,7 +279,7 @@ cudaError_t launch_heat_kappa_step(const float* in, float* out, const float* kap
 cudaError_t launch_heat_adjoint_step(float* lam, const float* y, float* y_next, const float* u, const float* kappa,
                                      double* g, const BlockLayout& L, int D, const HeatLap& c, cudaStream_t st)
 {
-    const Grid gr = stage_grid(L, L.H);
+    const Grid gr = stage_grid(L, L.H, D == 1 ? 3 : 2, heat_chunk);
 #define CALL(DD) return launch_pdl(heat_adj_step_kernel<DD>, gr.g, gr.b, 0, st, lam, y, y_next, u, kappa, g, L, c, gr.t)
     B2R_HEAT_ADJ_DISPATCH(D, CALL)
 #undef CALL
