@@ -5,6 +5,7 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <fstream>
 #include <new>
@@ -36,6 +37,7 @@ struct b2r_handle {
     CUtensorMap tmap2[2];       // boxes of the two-step kernel (D = 1)
     CUtensorMap tmap3[2];       // boxes of the several-step kernel's 128 x 32 tiles (D = 1) or of the radius-2 two-step kernel
     CUtensorMap tmap4[2];       // boxes of its 64 x 64 tiles
+    CUtensorMap tmapr[3][2];    // boxes of heat_rows.cu for two, three and four steps per pass (D = 1)
     HeatCoef hc{};
     HeatTune tune{};
     // elastic wave: fields and material
@@ -176,6 +178,7 @@ b2r_status ensure_kappa(b2r_handle* h);
 b2r_status ensure_staging(b2r_handle* h, size_t bytes);
 b2r_status build_heat_maps(b2r_handle* h);
 int heat_pass_steps(const b2r_handle* h, int i, int left);
+int heat_own_steps(const b2r_handle* h);
 int gol_pass_gens(const b2r_handle* h, int i, int left);
 b2r_status check_status(b2r_handle* h);
 b2r_status exchange_all(b2r_handle* h, bool staged, cudaStream_t xst = nullptr);   // xst: another stream than the handle's

@@ -14,14 +14,14 @@ b2r_status b2r_set_tuning(b2r_handle* h, int key, int value)
     case B2R_TUNE_ZCHUNK: h->tune.zchunk = value; break;
     case B2R_TUNE_CTAS_PER_SM: h->tune.ctas_per_sm = value; break;
     case B2R_TUNE_PDL: h->tune.pdl = value != 0; break;
-    case B2R_TUNE_TBLOCK: h->tune.tblock = value; break;
-    case B2R_TUNE_ZCHUNK2: h->tune.zchunk2 = value; break;
+    case B2R_TUNE_TBLOCK: h->tune.tblock = value; h->tune.own = false; break;
+    case B2R_TUNE_ZCHUNK2: h->tune.zchunk2 = value; h->tune.own = false; break;
     case B2R_TUNE_EQWP_FUSED: h->eqwp_fused = value != 0; break;
     case B2R_TUNE_GOL_BYTES: h->gol_bytes = value != 0; break;
     case B2R_TUNE_ADJ_FUSED: h->adj_fused = value != 0; break;
     case B2R_TUNE_GOL_PUSH: h->gol_push = value != 0; break;
-    case B2R_TUNE_TB16: h->tune.tb16 = value != 0; break;
-    case B2R_TUNE_TB_NARROW: h->tune.tbn = value != 0; break;
+    case B2R_TUNE_TB16: h->tune.tb16 = value != 0; h->tune.own = false; break;
+    case B2R_TUNE_TB_NARROW: h->tune.tbn = value != 0; h->tune.own = false; break;
     case B2R_TUNE_TB_R2: h->tune.r2 = value != 0; break;
     case B2R_TUNE_EQWP_TMA: h->eqwp_tma = value != 0; break;
     case B2R_TUNE_EQWP_OVERLAP: h->eqwp_overlap = value != 0; break;

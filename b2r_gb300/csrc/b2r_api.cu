@@ -108,6 +108,10 @@ b2r_status build_heat_maps(b2r_handle* h)
              !make_block_tmap(&h->tmap3[b], h->buf[b], h->L, 4, heat_tb_box_w(0), heat_tb_box_h(0), 1) ||
              !make_block_tmap(&h->tmap4[b], h->buf[b], h->L, 4, heat_tb_box_w(1), heat_tb_box_h(1), 1)))
             return fail(h, B2R_ERR_CUDA, "cuTensorMapEncodeTiled failed for the heat field");
+        if (h->cfg.D == 1)
+            for (int k = 0; k < 3; ++k)
+                if (!make_block_tmap(&h->tmapr[k][b], h->buf[b], h->L, 4, heat_rows_box_w(), heat_rows_box_h(2 + k), 1))
+                    return fail(h, B2R_ERR_CUDA, "cuTensorMapEncodeTiled failed for the heat field");
         if (h->cfg.D == 2 &&
             !make_block_tmap(&h->tmap3[b], h->buf[b], h->L, 4, heat_tb2_box_w(), heat_tb2_box_h(), 1))
             return fail(h, B2R_ERR_CUDA, "cuTensorMapEncodeTiled failed for the heat field");
@@ -115,12 +119,19 @@ b2r_status build_heat_maps(b2r_handle* h)
     return B2R_OK;
 }
 
+// Steps per HBM pass of radius 1 unless a knob says otherwise.
+int heat_own_steps(const b2r_handle* h)
+{
+    (void)h;
+    return getenv("HR") ? atoi(getenv("HR")) : 3;
+}
+
 // Steps per HBM pass the heat schedule allows: radius 1 up to tblock (<= 4),
 // radius 2 two (tblock >= 2); 1 = the one-step sweep.
 int heat_max_pass_steps(const b2r_handle* h)
 {
     if (h->cfg.model != B2R_MODEL_HEAT || h->tune.tblock < 2) return 1;
-    if (h->cfg.D == 1) return std::min(h->tune.tblock, 4);
+    if (h->cfg.D == 1) return h->tune.own ? heat_own_steps(h) : std::min(h->tune.tblock, 4);
     return h->cfg.D == 2 && h->tune.r2 ? 2 : 1;
 }
 
@@ -397,6 +408,10 @@ b2r_status advance(b2r_handle* h, int n)
             if (h->cfg.D == 2) {
                 CK(h, launch_heat_substep_tb2(&h->tmap3[h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L, i,
                                               h->hc, h->d_status, h->stream, h->tune.zchunk2));
+                h->cur = 1 - h->cur;
+            } else if (h->tune.own) {
+                CK(h, launch_heat_rows(k, &h->tmapr[k - 2][h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L, i,
+                                       h->hc, h->d_status, h->stream));
                 h->cur = 1 - h->cur;
             } else if (k == 2 && !h->tune.tb16) {
                 if ((st = substep2(h, i)) != B2R_OK) return st;
