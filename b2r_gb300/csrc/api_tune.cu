@@ -246,13 +246,14 @@ b2r_status b2r_autotune(b2r_handle* h, int trial_steps, int best[3], double* bes
     HeatTune bestT = h->tune;
     float bestMs = 1e30f;
     b2r_status st = B2R_OK;
-    // candidates: the several-step sweeps (radius 1: two, three and four steps
-    // per pass) by z-chunk, then the one-step sweep by z-chunk x persistent
+    // candidates: the library's own rule for radius 1, the several-step sweeps
+    // (radius 1: two, three and four steps per pass) by z-chunk, then the one-step sweep by z-chunk x persistent
     // CTAs per SM x PDL.  Every trial advances a multiple of 12 time steps,
     // so that each schedule runs whole passes.
     struct Cand { int tb, zc2, zc, cp, pdl, tb16, tbn, r2 = 0; };
     std::vector<Cand> cands;
     if (h->cfg.D == 1) {
+        cands.push_back({0, 0, 0, 0, 1, 0, 0});   // the library's own rule
         for (int z2 : {4, 8, 16, 32, 64}) cands.push_back({2, z2, 0, 0, 1, 0, 0});
         for (int tbn = 0; tbn < 2; ++tbn) {
             for (int z2 : {0, 32, 96}) cands.push_back({2, z2, 0, 0, 1, 1, tbn});
@@ -273,7 +274,8 @@ b2r_status b2r_autotune(b2r_handle* h, int trial_steps, int best[3], double* bes
         h->tune.tb16 = cd.tb16;
         h->tune.tbn = cd.tbn;
         h->tune.r2 = cd.r2;
-        h->tune.tblock = cd.tb;
+        h->tune.own = cd.tb == 0;
+        h->tune.tblock = cd.tb == 0 ? 2 : cd.tb;
         h->tune.zchunk2 = cd.zc2;
         h->tune.zchunk = cd.zc;
         h->tune.ctas_per_sm = cd.cp;

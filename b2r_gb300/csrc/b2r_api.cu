@@ -119,11 +119,17 @@ b2r_status build_heat_maps(b2r_handle* h)
     return B2R_OK;
 }
 
-// Steps per HBM pass of radius 1 unless a knob says otherwise.
+// Steps per HBM pass of radius 1 unless a knob says otherwise: three on four
+// rows per thread (heat_rows.cu, whose tiles are 120 x 44 cells), or two in
+// two-row tiles where the blocks are too small to fill those (128^3: 5.2 us
+// per step against 7.0; 64^3: 4.4 against 2.8; four blocks of 24x20x32 cells
+// 6.5 against 4.9).
 int heat_own_steps(const b2r_handle* h)
 {
-    (void)h;
-    return getenv("HR") ? atoi(getenv("HR")) : 3;
+    if (h->L.B[0] < 96 || h->L.B[1] < 40 || (long long)h->L.B[0] * h->L.B[1] * h->L.B[2] < 1000000) return 2;
+    // a period of four steps between exchanges is one pass of four, not three
+    // and one (512^3 torus in 2x2x2 blocks: 136 us per step, 157 as 3 + 1)
+    return (h->L.nblk > 1 || h->L.periodic) && h->cfg.R == 4 ? 4 : 3;
 }
 
 // Steps per HBM pass the heat schedule allows: radius 1 up to tblock (<= 4),
@@ -409,7 +415,7 @@ b2r_status advance(b2r_handle* h, int n)
                 CK(h, launch_heat_substep_tb2(&h->tmap3[h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L, i,
                                               h->hc, h->d_status, h->stream, h->tune.zchunk2));
                 h->cur = 1 - h->cur;
-            } else if (h->tune.own) {
+            } else if (h->tune.own && heat_own_steps(h) > 2) {
                 CK(h, launch_heat_rows(k, &h->tmapr[k - 2][h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L, i,
                                        h->hc, h->d_status, h->stream));
                 h->cur = 1 - h->cur;

@@ -183,7 +183,7 @@ heat_rows_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ ou
     float* const ring = reinterpret_cast<float*>(smem_raw + ((128 - (smem_u32(smem_raw) & 127)) & 127));
     RCtx<T, NW> c;
     c.tid = threadIdx.x;
-    c.warp = c.tid >> 5;
+    c.warp = __shfl_sync(0xffffffffu, c.tid >> 5, 0);   // uniform over the warp, and known to be
     const int lane = c.tid & 31;
     c.xch = ring + kSlots * Cfg::SLOT;
     c.bar = reinterpret_cast<uint64_t*>(c.xch + (T - 1) * 2 * Cfg::XE);

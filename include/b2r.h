@@ -134,7 +134,8 @@ enum {
     B2R_TUNE_CTAS_PER_SM = 2,  /* 0 = one CTA per unit, k = persistent k CTAs per SM */
     B2R_TUNE_PDL = 3,          /* programmatic dependent launch on / off */
     B2R_TUNE_TBLOCK = 4,       /* time steps per pass: heat of radius 1 takes up to tblock (2, 3
-                                  or 4; default 2) steps per HBM pass and Game of Life
+                                  or 4; default 2, or three on large blocks until this or another
+                                  knob of the several-step sweeps is set) steps per HBM pass and Game of Life
                                   (bit-sliced cells, tblock >= 2) up to four generations per L2
                                   pass, never across a halo exchange; byte cells need >= 4;
                                   1 = one step per pass */
