@@ -37,6 +37,7 @@ struct b2r_handle {
     CUtensorMap tmap3[2];       // boxes of the several-step kernel's 128 x 32 tiles (D = 1) or of the radius-2 two-step kernel
     CUtensorMap tmap4[2];       // boxes of its 64 x 64 tiles
     CUtensorMap tmapr[3][2];    // boxes of heat_rows.cu for two, three and four steps per pass (D = 1)
+    CUtensorMap tmapf[2][3];    // boxes of heat_far.cu's three tile heights
     HeatCoef hc{};
     HeatTune tune{};
     // elastic wave: fields and material

@@ -11,9 +11,9 @@ b2r_status b2r_set_tuning(b2r_handle* h, int key, int value)
 {
     if (!h) return fail(nullptr, B2R_ERR_ARG, "null handle");
     switch (key) {
-    case B2R_TUNE_ZCHUNK: h->tune.zchunk = value; break;
-    case B2R_TUNE_CTAS_PER_SM: h->tune.ctas_per_sm = value; break;
-    case B2R_TUNE_PDL: h->tune.pdl = value != 0; break;
+    case B2R_TUNE_ZCHUNK: h->tune.zchunk = value; h->tune.own = false; break;
+    case B2R_TUNE_CTAS_PER_SM: h->tune.ctas_per_sm = value; h->tune.own = false; break;
+    case B2R_TUNE_PDL: h->tune.pdl = value != 0; h->tune.own = false; break;
     case B2R_TUNE_TBLOCK: h->tune.tblock = value; h->tune.own = false; break;
     case B2R_TUNE_ZCHUNK2: h->tune.zchunk2 = value; h->tune.own = false; break;
     case B2R_TUNE_EQWP_FUSED: h->eqwp_fused = value != 0; break;
@@ -22,7 +22,7 @@ b2r_status b2r_set_tuning(b2r_handle* h, int key, int value)
     case B2R_TUNE_GOL_PUSH: h->gol_push = value != 0; break;
     case B2R_TUNE_TB16: h->tune.tb16 = value != 0; h->tune.own = false; break;
     case B2R_TUNE_TB_NARROW: h->tune.tbn = value != 0; h->tune.own = false; break;
-    case B2R_TUNE_TB_R2: h->tune.r2 = value != 0; break;
+    case B2R_TUNE_TB_R2: h->tune.r2 = value != 0; h->tune.own = false; break;
     case B2R_TUNE_EQWP_TMA: h->eqwp_tma = value != 0; break;
     case B2R_TUNE_EQWP_OVERLAP: h->eqwp_overlap = value != 0; break;
     case B2R_TUNE_GOL_ROWS: h->gol_rows = value < 0 ? 0 : value; break;
@@ -246,14 +246,14 @@ b2r_status b2r_autotune(b2r_handle* h, int trial_steps, int best[3], double* bes
     HeatTune bestT = h->tune;
     float bestMs = 1e30f;
     b2r_status st = B2R_OK;
-    // candidates: the library's own rule for radius 1, the several-step sweeps
+    // candidates: the library's own rule, the several-step sweeps
     // (radius 1: two, three and four steps per pass) by z-chunk, then the one-step sweep by z-chunk x persistent
     // CTAs per SM x PDL.  Every trial advances a multiple of 12 time steps,
     // so that each schedule runs whole passes.
     struct Cand { int tb, zc2, zc, cp, pdl, tb16, tbn, r2 = 0; };
     std::vector<Cand> cands;
+    cands.push_back({0, 0, 0, 0, 1, 0, 0});   // the library's own rule
     if (h->cfg.D == 1) {
-        cands.push_back({0, 0, 0, 0, 1, 0, 0});   // the library's own rule
         for (int z2 : {4, 8, 16, 32, 64}) cands.push_back({2, z2, 0, 0, 1, 0, 0});
         for (int tbn = 0; tbn < 2; ++tbn) {
             for (int z2 : {0, 32, 96}) cands.push_back({2, z2, 0, 0, 1, 1, tbn});

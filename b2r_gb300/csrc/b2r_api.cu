@@ -112,6 +112,9 @@ b2r_status build_heat_maps(b2r_handle* h)
             for (int k = 0; k < 3; ++k)
                 if (!make_block_tmap(&h->tmapr[k][b], h->buf[b], h->L, 4, heat_rows_box_w(), heat_rows_box_h(2 + k), 1))
                     return fail(h, B2R_ERR_CUDA, "cuTensorMapEncodeTiled failed for the heat field");
+        for (int k = 0; k < 3; ++k)
+            if (!make_block_tmap(&h->tmapf[b][k], h->buf[b], h->L, 4, heat_far_box_w(), heat_far_box_h(h->cfg.D, k), 1))
+                return fail(h, B2R_ERR_CUDA, "cuTensorMapEncodeTiled failed for the heat field");
         if (h->cfg.D == 2 &&
             !make_block_tmap(&h->tmap3[b], h->buf[b], h->L, 4, heat_tb2_box_w(), heat_tb2_box_h(), 1))
             return fail(h, B2R_ERR_CUDA, "cuTensorMapEncodeTiled failed for the heat field");
@@ -271,7 +274,11 @@ b2r_status substep(b2r_handle* h, int i, bool xnext)
     h->upmask = 0;
     switch (h->cfg.model) {
     case B2R_MODEL_HEAT:
-        CK(h, launch_heat_substep(&h->tmap[h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L,
+        if (h->tune.own)
+            CK(h, launch_heat_far(h->tmapf[h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L, h->cfg.D, i, h->hc,
+                                  h->d_status, h->stream));
+        else
+            CK(h, launch_heat_substep(&h->tmap[h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L,
                                   h->cfg.D, i, h->hc, h->d_status, h->stream, h->tune));
         h->cur = 1 - h->cur;
         return B2R_OK;

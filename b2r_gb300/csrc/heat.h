@@ -47,8 +47,8 @@ struct HeatTune {
     int zchunk = 0;        // output planes per work unit; 0 = 16 (fewer for small grids)
     int ctas_per_sm = 0;   // 0 = one CTA per unit; k > 0 = persistent, k CTAs per SM
     int pdl = 1;           // programmatic dependent launch on the stream
-    bool own = true;       // radius 1: the library's own rule for the steps per pass and their kernel
-                           // (heat_rows.cu); false once a knob of the several-step kernels is set
+    bool own = true;       // the library's own rule for the kernel (heat_far.cu, on large blocks of radius 1
+                           // heat_rows.cu) and the steps per pass; false once one of the knobs below is set
     int tblock = 2;        // time steps per HBM pass: radius 1 (2 = heat2.cu, 3-4 = heat_tb.cu), radius 2 (2 = heat_tb2.cu, with r2)
     int zchunk2 = 0;       // output planes per unit of the several-step kernels (0 = 16 / 64)
     int tb16 = 0;          // two steps per pass: 0 = heat2.cu (8-warp CTAs), 1 = heat_tb.cu (16 warps)
@@ -93,5 +93,12 @@ int heat_rows_box_w();
 int heat_rows_box_h(int T);
 cudaError_t launch_heat_rows(int T, const CUtensorMap* tin, float* out, const BlockLayout& L, int step_i,
                              const HeatCoef& c, int* status, cudaStream_t st);
+
+// One sub-step of radius D = 1 .. 4 (heat_far.cu).  tin: three tensor maps
+// over the input, with boxes of heat_far_box_w() x heat_far_box_h(D, k) cells.
+int heat_far_box_w();
+int heat_far_box_h(int D, int k);
+cudaError_t launch_heat_far(const CUtensorMap* tin, float* out, const BlockLayout& L, int D, int step_i,
+                            const HeatCoef& c, int* status, cudaStream_t st);
 
 }  // namespace b2r

@@ -1,0 +1,320 @@
+// heat_far.cu -- one heat time step of radius 1..4.
+//
+// The sweep of heat.cu with what bounds it taken out of its way.  There, the plane loop could not be unrolled by the queue's depth at radius
+// 4 without spilling, so the queue moved 64 registers per plane, and all
+// eight warps met at a barrier per plane.  Here
+//   * a CTA is one producer warp, which streams the input planes by TMA into
+//     a ring of shared planes, and 15, 11 or 7 consumer warps; planes are handed over
+//     by two mbarriers per slot (loaded; read by every consumer warp), so no
+//     warp waits for another one's arithmetic and the warps drift apart by
+//     the depth of the ring;
+//   * with 16 warps per SM a consumer thread has the registers for the 2D+1
+//     planes of its 4 cells of 2 rows and the loop unrolled by them, so the
+//     queue turns by names;
+//   * the y neighbours of the two rows are read pair by pair as the radius
+//     grows, each row once for both.
+// A thread's cells run the sweep's operations in its order (heat_unit.cuh):
+// the same bits.
+//
+// Measured (us per step against heat.cu's default schedule): 512^3 radius 2
+// 168 from 191 (798 GLUPS, 0.94 of the copy rate at one read and one write per
+// cell), radius 3 175 from 237, radius 4 188 from 275; 256^3 radius 4 29.6
+// from 41.7; 128^3 radius 2 5.0 from 8.4; 64^3 radius 3 4.2 from 6.0; 32^3
+// radius 2 3.3 from 5.2.
+//
+// Every wait is bounded; a warp that gives up reports
+// DEV_TIMEOUT and leaves, and so does every warp that waits for it.
+#include "b2r_common.cuh"
+#include "heat.h"
+
+namespace b2r {
+namespace {
+
+constexpr int kTW = 128;             // output cells per tile row
+
+// NC consumer warps, two output rows each
+template <int D, int NC>
+struct FCfg {
+    static constexpr int TH = 2 * NC, THR = 32 * (NC + 1);
+    static constexpr int BW = kTW + 8, BH = TH + 2 * D;    // TMA box (cells)
+    static constexpr int SLOT = (BW * BH + 31) / 32 * 32;   // floats per ring slot (a multiple of 128 bytes)
+    static constexpr int S = D + 4;                         // ring slots: D + 1 planes in use, three ahead
+    static constexpr size_t SMEM = (size_t)S * SLOT * 4 + 2 * S * 8 + 128;
+};
+
+struct FSched {
+    int ntx, nty, nzc, Lz;
+};
+
+__device__ __forceinline__ float4 f4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+template <int D, int NC>
+struct FCtx {
+    float4 q[2 * D + 1][2];     // planes p-2D .. p by slot (pr mod 2D+1), rows
+    const float* ring;          // + the thread's first cell of its first row
+    uint64_t *full, *empty;
+    float* dst;                 // the thread's cells of the next output plane
+    long long plane;
+    int P, np;
+    unsigned m0, m1;            // cells stored of each row
+    bool lane0;
+};
+
+// Input plane pr (slot PH = pr mod 2D+1 of the queue); from pr = 2D on also
+// the output plane D planes back.  False if the wait gave up.
+template <int D, int NC, int PH>
+__device__ __forceinline__ bool f_iter(FCtx<D, NC>& c, const HeatCoef& C, int pr, int slot, int phase, int cslot)
+{
+    using Cfg = FCfg<D, NC>;
+    constexpr int N = 2 * D + 1, BW = Cfg::BW;
+    if (!mbar_wait_bounded(&c.full[slot], phase)) return false;
+    {
+        const float* pl = c.ring + slot * Cfg::SLOT;
+        c.q[PH][0] = f4(pl);
+        c.q[PH][1] = f4(pl + BW);
+    }
+    if (pr >= 2 * D) {
+        constexpr int CE = (PH + N - D) % N;                // the centre plane
+        const float* pc = c.ring + cslot * Cfg::SLOT;
+        const float4 c0 = c.q[CE][0], c1 = c.q[CE][1];
+        const float4 l0 = f4(pc - 4), r0 = f4(pc + 4), l1 = f4(pc + BW - 4), r1 = f4(pc + BW + 4);
+        const float v0[12] = {l0.x, l0.y, l0.z, l0.w, c0.x, c0.y, c0.z, c0.w, r0.x, r0.y, r0.z, r0.w};
+        const float v1[12] = {l1.x, l1.y, l1.z, l1.w, c1.x, c1.y, c1.z, c1.w, r1.x, r1.y, r1.z, r1.w};
+        const float2 a0 = make_float2(C.a0, C.a0);
+        float2 lo0 = __fmul2_rn(a0, make_float2(c0.x, c0.y)), hi0 = __fmul2_rn(a0, make_float2(c0.z, c0.w));
+        float2 lo1 = __fmul2_rn(a0, make_float2(c1.x, c1.y)), hi1 = __fmul2_rn(a0, make_float2(c1.z, c1.w));
+        float4 below = c0, above = c1;                      // rows -(k-1) and k of the pair
+#pragma unroll
+        for (int k = 1; k <= D; ++k) {
+            const float4 yb = f4(pc - k * BW), ya = f4(pc + (k + 1) * BW);   // rows -k and k+1
+            const float4 zm0 = c.q[(CE + N - k) % N][0], zp0 = c.q[(CE + k) % N][0];
+            const float4 zm1 = c.q[(CE + N - k) % N][1], zp1 = c.q[(CE + k) % N][1];
+            const float2 cx = make_float2(C.ax[k - 1], C.ax[k - 1]), cy = make_float2(C.ay[k - 1], C.ay[k - 1]),
+                         cz = make_float2(C.az[k - 1], C.az[k - 1]);
+            lo0 = __ffma2_rn(cx, make_float2(v0[4 - k] + v0[4 + k], v0[5 - k] + v0[5 + k]), lo0);
+            hi0 = __ffma2_rn(cx, make_float2(v0[6 - k] + v0[6 + k], v0[7 - k] + v0[7 + k]), hi0);
+            lo1 = __ffma2_rn(cx, make_float2(v1[4 - k] + v1[4 + k], v1[5 - k] + v1[5 + k]), lo1);
+            hi1 = __ffma2_rn(cx, make_float2(v1[6 - k] + v1[6 + k], v1[7 - k] + v1[7 + k]), hi1);
+            // row 0: rows -k and k; row 1: rows 1-k and 1+k
+            lo0 = __ffma2_rn(cy, __fadd2_rn(make_float2(yb.x, yb.y), make_float2(above.x, above.y)), lo0);
+            hi0 = __ffma2_rn(cy, __fadd2_rn(make_float2(yb.z, yb.w), make_float2(above.z, above.w)), hi0);
+            lo1 = __ffma2_rn(cy, __fadd2_rn(make_float2(below.x, below.y), make_float2(ya.x, ya.y)), lo1);
+            hi1 = __ffma2_rn(cy, __fadd2_rn(make_float2(below.z, below.w), make_float2(ya.z, ya.w)), hi1);
+            lo0 = __ffma2_rn(cz, __fadd2_rn(make_float2(zm0.x, zm0.y), make_float2(zp0.x, zp0.y)), lo0);
+            hi0 = __ffma2_rn(cz, __fadd2_rn(make_float2(zm0.z, zm0.w), make_float2(zp0.z, zp0.w)), hi0);
+            lo1 = __ffma2_rn(cz, __fadd2_rn(make_float2(zm1.x, zm1.y), make_float2(zp1.x, zp1.y)), lo1);
+            hi1 = __ffma2_rn(cz, __fadd2_rn(make_float2(zm1.z, zm1.w), make_float2(zp1.z, zp1.w)), hi1);
+            below = yb;
+            above = ya;
+        }
+        const float4 o0 = make_float4(lo0.x, lo0.y, hi0.x, hi0.y), o1 = make_float4(lo1.x, lo1.y, hi1.x, hi1.y);
+        float* d = c.dst;
+        if (c.m0 == 15u) *reinterpret_cast<float4*>(d) = o0;
+        else if (c.m0) {
+            if (c.m0 & 1u) d[0] = o0.x;
+            if (c.m0 & 2u) d[1] = o0.y;
+            if (c.m0 & 4u) d[2] = o0.z;
+            if (c.m0 & 8u) d[3] = o0.w;
+        }
+        d += c.P;
+        if (c.m1 == 15u) *reinterpret_cast<float4*>(d) = o1;
+        else if (c.m1) {
+            if (c.m1 & 1u) d[0] = o1.x;
+            if (c.m1 & 2u) d[1] = o1.y;
+            if (c.m1 & 4u) d[2] = o1.z;
+            if (c.m1 & 8u) d[3] = o1.w;
+        }
+        c.dst += c.plane;
+    }
+    if (pr >= D) {              // plane pr - D is read: its slot may be refilled
+        __syncwarp();
+        if (c.lane0) mbar_arrive(&c.empty[cslot]);
+    }
+    return true;
+}
+
+template <int D, int NC, int PH>
+__device__ __forceinline__ bool f_round(FCtx<D, NC>& c, const HeatCoef& C, int& pr, int& slot, int& phase, int& cslot)
+{
+    using Cfg = FCfg<D, NC>;
+    if (pr >= c.np) return true;
+    if (!f_iter<D, NC, PH>(c, C, pr, slot, phase, cslot)) return false;
+    if (pr >= D && ++cslot == Cfg::S) cslot = 0;
+    ++pr;
+    if (++slot == Cfg::S) slot = 0, phase ^= 1;
+    if constexpr (PH + 1 < 2 * D + 1) return f_round<D, NC, PH + 1>(c, C, pr, slot, phase, cslot);
+    return true;
+}
+
+template <int D, int NC>
+__global__ void __launch_bounds__(32 * (NC + 1), NC <= 7 ? 2 : 1)
+heat_far_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ out, const BlockLayout L,
+                const int step_i, const HeatCoef C, const FSched sch, int* __restrict__ status)
+{
+    using Cfg = FCfg<D, NC>;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    float* const ring = reinterpret_cast<float*>(smem_raw + ((128 - (smem_u32(smem_raw) & 127)) & 127));
+    uint64_t* const full = reinterpret_cast<uint64_t*>(ring + Cfg::S * Cfg::SLOT);
+    uint64_t* const empty = full + Cfg::S;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < Cfg::S; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], NC);
+        }
+        fence_mbar_init();
+    }
+    __syncthreads();
+    pdl_begin();
+
+    int u = blockIdx.x;
+    const int tx = u % sch.ntx;
+    u /= sch.ntx;
+    const int ty = u % sch.nty;
+    u /= sch.nty;
+    const int zc = u % sch.nzc, blk = u / sch.nzc;
+    const int edge = edge_bits(L, blk);
+    int lo[3], hi[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) stage_region(L, edge, a, D * (step_i + 1), lo[a], hi[a]);
+    const int xs0 = ((L.xoff + D) & ~3) + tx * kTW;     // storage x of tile column 0
+    const int y0 = D + ty * Cfg::TH;                        // block y of tile row 0
+    if (xs0 - L.xoff > hi[0] || xs0 + kTW - 1 - L.xoff < lo[0] || y0 > hi[1] || y0 + Cfg::TH - 1 < lo[1]) return;
+    const int zs = max(D + zc * sch.Lz, lo[2]), ze = min(D + (zc + 1) * sch.Lz - 1, hi[2]);
+    if (zs > ze) return;
+    const int first = zs - D, np = ze + D - first + 1;  // input planes
+
+    if (warp == NC) {                                // the producer
+        if (lane != 0) return;
+        int slot = 0, phase = 0;
+        bool ok = true;
+        int i = 0;
+        for (; i < np; ++i) {
+            if (i >= Cfg::S && !mbar_wait_bounded(&empty[slot], phase ^ 1)) {
+                ok = false;
+                break;
+            }
+            mbar_expect_tx(&full[slot], Cfg::BW * Cfg::BH * 4);
+            tma_load_4d(ring + slot * Cfg::SLOT, &tin, xs0 - 4, y0 - D, first + i, blk, &full[slot]);
+            if (++slot == Cfg::S) slot = 0, phase ^= 1;
+        }
+        if (!ok) {                                      // the loads in flight land before the CTA leaves (bounded)
+            report(status, DEV_TIMEOUT);
+            for (int k = max(0, i - Cfg::S); k < i; ++k)
+                mbar_wait_bounded(&full[k % Cfg::S], (k / Cfg::S) & 1, 100000000ull);
+        }
+        return;
+    }
+    FCtx<D, NC> c;
+    c.full = full;
+    c.empty = empty;
+    c.plane = L.plane;
+    c.P = L.P;
+    c.np = np;
+    c.lane0 = lane == 0;
+    c.ring = ring + (D + 2 * warp) * Cfg::BW + 4 + 4 * lane;
+    const int y = y0 + 2 * warp, xb = xs0 + 4 * lane - L.xoff;
+    unsigned m = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) m |= (xb + j >= lo[0] && xb + j <= hi[0] ? 1u : 0u) << j;
+    c.m0 = y >= lo[1] && y <= hi[1] ? m : 0u;
+    c.m1 = y + 1 >= lo[1] && y + 1 <= hi[1] ? m : 0u;
+    c.dst = out + (long long)blk * L.bstride + (long long)zs * L.plane + (long long)y * L.P + xs0 + 4 * lane;
+    int pr = 0, slot = 0, phase = 0, cslot = 0;
+    while (pr < np)
+        if (!f_round<D, NC, 0>(c, C, pr, slot, phase, cslot)) {
+            if (lane == 0) report(status, DEV_TIMEOUT);
+            return;
+        }
+}
+
+// Tile height and z chunk of a launch: the least busy busiest SM.  A unit of
+// lz planes costs lz + 2D planes and about two more until the ring is full; a
+// plane about 0.07 + 0.0222 us per row of the tile (radius 4, 512^3: 0.737 us
+// for 30 rows, 0.567 for 22, 0.709 for two tiles of 14).  Measured us per step
+// for 30 / 22 / 14 rows: radius 4, 512^3 197 / 207 / 188, 160^3 14.4 / 13.3 /
+// 14.2, 128^3 8.1 / 6.9 / 7.9; radius 2, 100x90x80 4.5 / 4.1 / 4.4, 32^3 4.3 /
+// 3.8 / 3.4.
+struct FPlan {
+    int rows = 0, lz = 0;
+    double cost = 1e300;
+};
+FPlan f_plan(const BlockLayout& L, int D, int ntx, int sms)
+{
+    FPlan best;
+    const int NZ = L.n[2] - 2 * D, NY = L.n[1] - 2 * D;
+    for (int rows : {30, 22, 14}) {
+        const long long tiles = (long long)ntx * ((NY + rows - 1) / rows) * L.nblk;
+        const int slots = rows == 14 ? 2 * sms : sms;
+        const double one = 0.07 + 0.0222 * rows;
+        for (int n = 1; n <= NZ; ++n) {
+            const int lz = (NZ + n - 1) / n;
+            if (n > 1 && lz < 3) break;
+            const long long units = tiles * ((NZ + lz - 1) / lz);
+            // two CTAs of 14 rows share an SM, or one has it alone
+            const double plane = rows > 14 ? one : (units > sms ? 1.85 : 1.4) * one;
+            const double cost = (double)((units + slots - 1) / slots) * (lz + 2 * D + 2) * plane;
+            if (cost < best.cost) best = FPlan{rows, lz, cost};
+        }
+    }
+    return best;
+}
+
+template <int D, int NC>
+cudaError_t launch_f(const CUtensorMap* tin, float* out, const BlockLayout& L, int ntx, int lz, int step_i,
+                     const HeatCoef& c, int* status, cudaStream_t st)
+{
+    using Cfg = FCfg<D, NC>;
+    static KernelSetup setup;
+    if (cudaError_t e = kernel_setup(setup, heat_far_kernel<D, NC>, Cfg::THR, Cfg::SMEM, nullptr, nullptr)) return e;
+    FSched sch;
+    sch.ntx = ntx;
+    sch.nty = (L.n[1] - 2 * D + Cfg::TH - 1) / Cfg::TH;
+    sch.Lz = lz;
+    sch.nzc = (L.n[2] - 2 * D + lz - 1) / lz;
+    return launch_pdl(heat_far_kernel<D, NC>, (unsigned)((long long)ntx * sch.nty * sch.nzc * L.nblk), Cfg::THR,
+                      Cfg::SMEM, st, *tin, out, L, step_i, c, sch, status);
+}
+
+template <int D>
+cudaError_t launch_d(const CUtensorMap* tin, float* out, const BlockLayout& L, int step_i, const HeatCoef& c,
+                     int* status, cudaStream_t st)
+{
+    int dev = 0, sms = 0;
+    cudaError_t e;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    const int xs_begin = (L.xoff + D) & ~3;
+    const int ntx = (L.xoff + L.n[0] - D - xs_begin + kTW - 1) / kTW;
+    const FPlan p = f_plan(L, D, ntx, sms);
+    // rows of the tile by the tensor map's box: tin[0], [1], [2] for 30, 22, 14
+    switch (p.rows) {
+    case 30: return launch_f<D, 15>(&tin[0], out, L, ntx, p.lz, step_i, c, status, st);
+    case 22: return launch_f<D, 11>(&tin[1], out, L, ntx, p.lz, step_i, c, status, st);
+    default: return launch_f<D, 7>(&tin[2], out, L, ntx, p.lz, step_i, c, status, st);
+    }
+}
+
+}  // namespace
+
+int heat_far_box_w() { return kTW + 8; }
+int heat_far_box_h(int D, int k) { return (k == 0 ? 30 : k == 1 ? 22 : 14) + 2 * D; }
+
+cudaError_t launch_heat_far(const CUtensorMap* tin, float* out, const BlockLayout& L, int D, int step_i,
+                            const HeatCoef& c, int* status, cudaStream_t st)
+{
+    switch (D) {
+    case 1: return launch_d<1>(tin, out, L, step_i, c, status, st);
+    case 2: return launch_d<2>(tin, out, L, step_i, c, status, st);
+    case 3: return launch_d<3>(tin, out, L, step_i, c, status, st);
+    case 4: return launch_d<4>(tin, out, L, step_i, c, status, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace b2r

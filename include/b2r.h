@@ -128,7 +128,9 @@ b2r_status b2r_step(b2r_handle* h, int nsteps);
  * CUDA graphs captured on first use (heat and Game of Life, when the handle
  * has a non-default stream).  Default on; results are identical either way. */
 b2r_status b2r_set_graphs(b2r_handle* h, int enable);
-/* Launch-schedule knobs of the heat sweep (the autotuner's search space). */
+/* Launch-schedule knobs (the autotuner's search space).  Until one of the heat
+ * knobs is set, a heat domain runs on the kernel that the library's own rule
+ * picks; setting one selects the sweep that the knob belongs to. */
 enum {
     B2R_TUNE_ZCHUNK = 1,       /* planes per work unit of the one-step sweep (0 = 16) */
     B2R_TUNE_CTAS_PER_SM = 2,  /* 0 = one CTA per unit, k = persistent k CTAs per SM */
