@@ -1,13 +1,14 @@
 // batch.cu -- many independent heat instances of uneven sizes and stencil
-// orders advanced in ONE persistent launch driven by a device work queue.
+// orders advanced in persistent launches (one per stencil order) driven by
+// device work queues.
 //
 // No reference counterpart (the reference runs one model per MPI rank); each
 // instance is a single-block heat domain with a fixed shell, stepped with the
 // scheme of heat-3D.cu:228-231/315-318/410-413/514-517 exactly as the plain
 // sweep does, so results are bit-identical to per-instance plain runs.
 //
-// Work items (round t, instance k, unit u) go through the device work queue
-// of work_queue.cuh.  A round is one time step of an instance on one-step
+// Work items (round t, instance k, unit u) go through device work queues
+// (work_queue.cuh).  A round is one time step of an instance on one-step
 // units (heat_unit.cuh, tile shape per instance) or two of an instance on
 // two-step units (heat2_unit.cuh, radius 1; the last round of an odd step
 // count takes one), chosen per (order, size class) by the autotuner.
@@ -19,6 +20,7 @@
 #include <vector>
 
 #include "heat2_unit.cuh"
+#include "heat_far.cuh"
 #include "heat_unit.cuh"
 #include "work_queue.cuh"
 
@@ -74,6 +76,7 @@ struct InstDev {
     int lpr;                             // its lanes per tile row (kLpr[shape])
     int tb;                              // time steps per unit: 1, or 2 (shape kTwoStep)
     int rounds;                          // rounds of units: nsteps / tb, rounded up
+    int done0;                           // its counters: one per z chunk, or one (two-step kernel)
 };
 
 struct BatchArgs {
@@ -81,11 +84,195 @@ struct BatchArgs {
     const CUtensorMap* maps;             // 2 per instance: buffer 0, buffer 1
     const unsigned long long* items;     // the queue: work items in claim order
     unsigned long long* head;            // next item (zeroed per run)
-    unsigned* done;                      // finished units per instance (zeroed per run)
+    unsigned* done;                      // finished units per instance and z chunk (zeroed per run)
     int* status;
     long long total;
 };
 
+// ---------------------------------------------------------------- one step per unit
+// The default kernel (no instance on two-step units): CTAs of one producer
+// warp and kQC consumer warps (heat_far.cuh), two per SM.  The producer claims
+// items, waits for an item's instance to finish the round before, and streams
+// the unit's planes into the ring while the consumers still work on the units
+// before it, so neither the claim, nor the wait, nor filling the ring stops
+// them.  A consumer warp reads the next unit's description (a ring of four,
+// written before the unit's first plane is loaded; a unit has at least three
+// planes and the ring of planes eight, so the producer is never four units
+// ahead), runs it, and counts itself into the instance's counter.  An item
+// still waits only for items claimed before it, whose CTAs' consumers need
+// nothing but their ring, so the queue cannot deadlock.
+//
+// Measured, 64 instances of edges 32..192, radii 1..4, 50..500 steps: 49.2 ms
+// with upload and download from 94.4 (478 GLUPS alone from 242; 50.6 ms with
+// one counter per instance instead of one per z chunk; z chunks of 8, 12, 20,
+// 32 planes instead of 16: 55, 50, 52, 59 ms).  All 64 with radius 1 / 2 / 3 /
+// 4: 653 / 610 / 513 / 404 GLUPS.
+//
+// One launch and one queue per radius in the batch: with all radii in one
+// kernel the four unrolled plane loops share one register allocation and
+// spill (radius 2: 313 GLUPS alone in such a kernel).  The launches run on
+// streams of their own, so one's CTAs take the room that another's tail
+// leaves.
+//
+constexpr int kQC = 7, kQS = 8;
+constexpr int kQThreads = 32 * (kQC + 1);
+constexpr int kQTileY[3] = {2 * kQC, 4 * kQC, 8 * kQC};     // rows of a tile by shape
+constexpr int q_slot(int D, int s) { return (4 * kLpr[s] + 8) * (kQTileY[s] + 2 * D); }
+constexpr int kQSlot = (cmax(cmax(q_slot(4, 0), q_slot(4, 1)), q_slot(4, 2)) + 31) / 32 * 32;
+constexpr size_t kQSmem = size_t(kQS) * kQSlot * sizeof(float) + 2 * kQS * sizeof(uint64_t) + 128;
+
+__device__ __forceinline__ float* q_ring(unsigned char* smem_raw)   // TMA destinations are 128-byte aligned
+{
+    return reinterpret_cast<float*>(smem_raw + ((128 - (smem_u32(smem_raw) & 127)) & 127));
+}
+
+struct QUnit {
+    int k, t, u;           // instance (-1: no more units), round, unit
+};
+
+// Ring positions after the unit (packed), or -1 if a wait gave up.  Not
+// inlined: a register allocation of its own does not spill (radius 4).
+template <int D>
+__device__ __noinline__ int consume_unit(const InstDev& in, int t, int u, uint32_t coef, int pos)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    float* const ring = q_ring(smem_raw);    // found again here, so that its loads are known to be shared ones
+    farx::FCtx<D, kQS, kQSlot, 0> c;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    uint64_t* const full = reinterpret_cast<uint64_t*>(ring + kQS * kQSlot);
+    uint64_t* const empty = full + kQS;
+    int slot = pos & 15, phase = (pos >> 4) & 1, cslot = pos >> 5;
+    const int tx = u % in.ntx, r = u / in.ntx, ty = r % in.nty, zc = r / in.nty;
+    const int lpr = in.lpr, lg = lpr == 32 ? 5 : (lpr == 16 ? 4 : 3);
+    const int lx = lane & (lpr - 1);
+    const int row = 2 * ((warp << (5 - lg)) + (lane >> lg));     // the thread's first row in the tile
+    const BlockLayout& L = in.L;
+    const int zs = D + zc * in.Lz, ze = min(D + (zc + 1) * in.Lz - 1, L.n[2] - 1 - D);
+    const int xs = ((L.xoff + D) & ~3) + tx * 4 * lpr + 4 * lx, y = D + ty * (2 * kQC << (5 - lg)) + row;
+    c.full = full;
+    c.empty = empty;
+    c.plane = L.plane;
+    c.P = L.P;
+    c.np = ze - zs + 1 + 2 * D;
+    c.bw = 4 * lpr + 8;
+    c.lane0 = lane == 0;
+    c.ring = ring + (D + row) * c.bw + 4 + 4 * lx;
+    unsigned m = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        m |= (xs + j - L.xoff >= D && xs + j - L.xoff <= L.n[0] - 1 - D ? 1u : 0u) << j;
+    c.m0 = y <= L.n[1] - 1 - D ? m : 0u;
+    c.m1 = y + 1 <= L.n[1] - 1 - D ? m : 0u;
+    c.dst = in.buf[(t + 1) & 1] + (long long)zs * L.plane + (long long)y * L.P + xs;
+    return farx::f_unit(c, farx::SharedCoef{coef}, slot, phase, cslot) ? slot | (phase << 4) | (cslot << 5) : -1;
+}
+
+template <int D>
+__global__ void __launch_bounds__(kQThreads, 2) batch_far_kernel(const BatchArgs a)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ QUnit s_unit[4];
+    __shared__ float2 s_coef[4][farx::kCoefPairs];
+    float* const ring = q_ring(smem_raw);
+    uint64_t* const full = reinterpret_cast<uint64_t*>(ring + kQS * kQSlot);
+    uint64_t* const empty = full + kQS;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kQS; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], kQC);
+        }
+        fence_mbar_init();
+    }
+    __syncthreads();
+    if (warp == kQC) {                       // the producer
+        int slot = 0, phase = 0;
+        long long i = 0;                     // planes issued
+        bool ok = true;
+        long long next = lane == 0 ? (long long)atomicAdd(a.head, 1ull) : 0;
+        for (int j = 0; ok; ++j) {
+            QUnit q{-1, 0, 0};
+            next = __shfl_sync(0xffffffffu, next, 0);
+            if (next < a.total) wq::unpack_item(a.items[next], q.t, q.k, q.u);
+            if (q.k < 0) {                   // no more units: a phase without a plane says so
+                if (lane == 0) {
+                    if (i >= kQS) ok = mbar_wait_bounded(&empty[slot], phase ^ 1);
+                    if (ok) {
+                        s_unit[j & 3] = q;
+                        farx::mbar_arrive(&full[slot]);
+                    }
+                }
+                break;
+            }
+            const InstDev& in = a.inst[q.k];
+            const int bw = 4 * in.lpr + 8, th = 2 * kQC * (32 / in.lpr), tiles = in.ntx * in.nty;
+            const int tx = q.u % in.ntx, r = q.u / in.ntx, ty = r % in.nty, zc = r / in.nty;
+            if (lane == 0) next = (long long)atomicAdd(a.head, 1ull);
+            if (q.t > 0) {
+                // the round before of the chunks this one reads (and whose
+                // readers it overwrites): a counter per lane
+                const int reach = (D + in.Lz - 1) / in.Lz;
+                for (int c = max(0, zc - reach) + lane; ok && c <= min(in.nzc - 1, zc + reach); c += 32)
+                    ok = wq::wait_done(&a.done[in.done0 + c], (unsigned)q.t * (unsigned)tiles * (unsigned)kQC);
+                ok = __all_sync(0xffffffffu, ok);
+            }
+            if (lane == 0) {
+                const int zs = D + zc * in.Lz, ze = min(D + (zc + 1) * in.Lz - 1, in.L.n[2] - 1 - D);
+                const int np = ze - zs + 1 + 2 * D, xs0 = ((in.L.xoff + D) & ~3) + tx * 4 * in.lpr;
+                const unsigned bytes = (unsigned)(bw * (th + 2 * D)) * 4u;
+                const CUtensorMap* map = &a.maps[2 * q.k + (q.t & 1)];
+                asm volatile("fence.proxy.async.global;" ::: "memory");   // what the other lanes waited for, too
+                for (int p = 0; p < np && ok; ++p, ++i) {
+                    if (i >= kQS) ok = mbar_wait_bounded(&empty[slot], phase ^ 1);
+                    if (!ok) break;
+                    if (p == 0) {            // the unit's description and weights, before its first plane
+                        s_unit[j & 3] = q;
+                        s_coef[j & 3][0] = make_float2(in.C.a0, in.C.a0);
+#pragma unroll
+                        for (int d = 0; d < 4; ++d) {
+                            s_coef[j & 3][3 * d + 1] = make_float2(in.C.ax[d], in.C.ax[d]);
+                            s_coef[j & 3][3 * d + 2] = make_float2(in.C.ay[d], in.C.ay[d]);
+                            s_coef[j & 3][3 * d + 3] = make_float2(in.C.az[d], in.C.az[d]);
+                        }
+                    }
+                    mbar_expect_tx(&full[slot], bytes);
+                    tma_load_4d(ring + slot * kQSlot, map, xs0 - 4, ty * th, zs - D + p, 0, &full[slot]);
+                    if (++slot == kQS) slot = 0, phase ^= 1;
+                }
+            }
+            ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+        }
+        if (!ok && lane == 0) {              // the loads in flight land before the CTA leaves (bounded)
+            report(a.status, DEV_TIMEOUT);
+            for (long long g = i > kQS ? i - kQS : 0; g < i; ++g)
+                mbar_wait_bounded(&full[g % kQS], (int)(g / kQS) & 1, 100000000ull);
+        }
+        return;
+    }
+    int pos = 0;                             // ring positions: slot, phase, slot to release next
+    for (int j = 0;; ++j) {
+        // the producer's own wait may take 2 s
+        bool ok = mbar_wait_bounded(&full[pos & 15], (pos >> 4) & 1, 4000000000ull);
+        const QUnit q = s_unit[j & 3];
+        if (ok) {
+            if (q.k < 0) return;
+            const InstDev& in = a.inst[q.k];
+            pos = consume_unit<D>(in, q.t, q.u, smem_u32(s_coef[j & 3]), pos);
+            ok = pos >= 0;
+        }
+        if (!ok) {
+            if (lane == 0) report(a.status, DEV_TIMEOUT);
+            return;
+        }
+        __syncwarp();                        // the warp's stores of this unit, then its count
+        if (lane == 0) {
+            const InstDev& in = a.inst[q.k];
+            wq::release_done(&a.done[in.done0 + q.u / (in.ntx * in.nty)]);
+        }
+    }
+}
+
+// ---------------------------------------------------------------- with two-step units
 // the four unit bodies are inlined into the kernel (measured faster than
 // separate calls, whose calling convention spills the register queues)
 #ifdef B2R_BATCH_NOINLINE
@@ -166,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, B2R_BATCH_MINB) batch_kernel(const B
             wq::unpack_item(a.items[item], t, k, u);
             int ok = 1;
             // wait for round t-1 of this instance (bounded)
-            if (t > 0) ok = wq::wait_done(&a.done[k], (unsigned)t * (unsigned)a.inst[k].units) ? 1 : 0;
+            if (t > 0) ok = wq::wait_done(&a.done[a.inst[k].done0], (unsigned)t * (unsigned)a.inst[k].units) ? 1 : 0;
             s_t = t;
             s_k = k;
             s_u = u;
@@ -202,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, B2R_BATCH_MINB) batch_kernel(const B
             return;
         }
         __syncthreads();                     // every store of this unit is issued
-        if (threadIdx.x == 0) wq::release_done(&a.done[k]);
+        if (threadIdx.x == 0) wq::release_done(&a.done[in.done0]);
     }
 }
 
@@ -225,14 +412,24 @@ struct b2r_batch {
     long long items_cap = 0;
     unsigned long long* d_head = nullptr;
     unsigned* d_done = nullptr;
+    int ndone = 0;                   // its counters
     int* d_status = nullptr;
     float* staging = nullptr;
     size_t staging_bytes = 0;
     int maxrounds = 0;               // rounds of the current schedule's longest instance
     long long total = 0;
     int lz_policy = 16;              // z chunk cap per unit (autotuned)
-    int grid[2] = {0, 0};            // persistent grid (every resident slot) per kernel variant
+    int grid[5] = {};                // persistent grid (every resident slot): radius 1..4, with two-step units
     bool two = false;                // some instance runs on two-step units
+    // launches of a run: one per radius (instances sched[first .. first + n), queue d_items + at),
+    // or one for all with two-step units
+    struct Launch {
+        int D, first, n;
+        long long at, total;
+    };
+    std::vector<Launch> runs;
+    cudaStream_t side[3] = {};       // the second to fourth launch's streams
+    cudaEvent_t fork = nullptr, join[3] = {};
     size_t smem = 0;                 // ring + the two-step units' planes
     cudaGraphExec_t gexec = nullptr;
     cudaStream_t gstream = nullptr;
@@ -268,7 +465,7 @@ long long plane_cells(const b2r_batch* b, int k, int s)
     const BlockLayout& L = in.L;
     const int D = in.D;
     const int X = L.xoff + L.n[0] - D - ((L.xoff + D) & ~3), Y = L.n[1] - 2 * D;
-    const int tw = 4 * kLpr[s], th = kTileY[D][s];
+    const int tw = 4 * kLpr[s], th = b->two ? kTileY[D][s] : kQTileY[s];
     return (long long)((X + tw - 1) / tw) * tw * ((Y + th - 1) / th) * th;
 }
 
@@ -303,6 +500,8 @@ b2r_status build_schedule(b2r_batch* b);
 // its shape sh[k] (two-step units for radius 1 only)
 b2r_status apply_shapes(b2r_batch* b, const std::vector<int>& sh)
 {
+    b->two = false;
+    for (int k = 0; k < b->n; ++k) b->two = b->two || (sh[k] == kTwoStep && b->host[k].D == 1);
     for (int k = 0; k < b->n; ++k) {
         InstDev& in = b->host[k];
         const BlockLayout& L = in.L;
@@ -320,11 +519,11 @@ b2r_status apply_shapes(b2r_batch* b, const std::vector<int>& sh)
         } else {
             in.tb = 1;
             const int X = L.xoff + L.n[0] - D - ((L.xoff + D) & ~3), Y = L.n[1] - 2 * D;
-            const int tw = 4 * kLpr[s], th = kTileY[D][s];
+            const int tw = 4 * kLpr[s], th = b->two ? kTileY[D][s] : kQTileY[s];
             in.ntx = (X + tw - 1) / tw;
             in.nty = (Y + th - 1) / th;
             bw = tw + 8;
-            bh = kBoxH[D][s];
+            bh = b->two ? kBoxH[D][s] : kQTileY[s] + 2 * D;
         }
         in.rounds = (in.nsteps + in.tb - 1) / in.tb;
         for (int f = 0; f < 2; ++f)
@@ -346,18 +545,21 @@ b2r_status build_schedule(b2r_batch* b)
 {
     b->sched.resize(b->n);
     for (int k = 0; k < b->n; ++k) b->sched[k] = k;
-    std::stable_sort(b->sched.begin(), b->sched.end(),
-                     [&](int x, int y) { return b->host[x].rounds > b->host[y].rounds; });
+    std::stable_sort(b->sched.begin(), b->sched.end(), [&](int x, int y) {
+        const InstDev &p = b->host[x], &q = b->host[y];
+        return !b->two && p.D != q.D ? p.D > q.D : p.rounds > q.rounds;
+    });
     std::vector<InstDev> dev(b->n);
     std::vector<CUtensorMap> maps(2 * b->n);
     b->maxrounds = 0;
-    b->two = false;
+    int ndone = 0;
     for (int j = 0; j < b->n; ++j) {
         InstDev& in = b->host[b->sched[j]];
-        b->two = b->two || in.tb == 2;
         in.Lz = std::min(in.NZ, b->lz_policy > 0 ? b->lz_policy : in.NZ);
         in.nzc = (in.NZ + in.Lz - 1) / in.Lz;
         in.units = in.ntx * in.nty * in.nzc;
+        in.done0 = ndone;
+        ndone += b->two ? 1 : in.nzc;
         dev[j] = in;
         maps[2 * j] = b->maps[2 * b->sched[j]];
         maps[2 * j + 1] = b->maps[2 * b->sched[j] + 1];
@@ -365,15 +567,31 @@ b2r_status build_schedule(b2r_batch* b)
     }
     // no run of this batch may still read the queue or the descriptors
     BCK(cudaDeviceSynchronize(), "waiting for the batch's runs");
+    if (ndone > b->ndone) {
+        cudaFree(b->d_done);
+        b->d_done = nullptr;
+        b->ndone = 0;
+        BCK(cudaMalloc(&b->d_done, sizeof(unsigned) * ndone), "counter allocation");
+        b->ndone = ndone;
+    }
     std::vector<int> rounds(b->n), units(b->n);
     for (int j = 0; j < b->n; ++j) {
         rounds[j] = dev[j].rounds;
         units[j] = dev[j].units;
     }
-    std::vector<unsigned long long> items;
-    if (!wq::round_major_items(rounds.data(), units.data(), b->n, items))
-        return bfail(B2R_ERR_ARG, "the batch queue is too long (an instance with more than 2^24 units or "
-                                  "rounds, or more than 2^28 work items): split the batch");
+    std::vector<unsigned long long> items, part;
+    b->runs.clear();
+    for (int first = 0; first < b->n;) {
+        int n = 1;
+        while (first + n < b->n && (b->two || dev[first + n].D == dev[first].D)) ++n;
+        if (!wq::round_major_items(rounds.data() + first, units.data() + first, n, part) ||
+            items.size() + part.size() > (size_t)1 << 28)
+            return bfail(B2R_ERR_ARG, "the batch queue is too long (an instance with more than 2^24 units or "
+                                      "rounds, or more than 2^28 work items): split the batch");
+        b->runs.push_back({dev[first].D, first, n, (long long)items.size(), (long long)part.size()});
+        items.insert(items.end(), part.begin(), part.end());
+        first += n;
+    }
     b->total = (long long)items.size();
     if (b->total > b->items_cap) {
         cudaFree(b->d_items);
@@ -397,19 +615,35 @@ b2r_status build_schedule(b2r_batch* b)
 
 b2r_status enqueue_run(b2r_batch* b, cudaStream_t st)
 {
-    BCK(cudaMemsetAsync(b->d_head, 0, sizeof(unsigned long long), st), "reset queue");
-    BCK(cudaMemsetAsync(b->d_done, 0, sizeof(unsigned) * b->n, st), "reset counters");
-    BatchArgs a;
-    a.inst = b->d_inst;
-    a.maps = b->d_maps;
-    a.items = b->d_items;
-    a.head = b->d_head;
-    a.done = b->d_done;
-    a.status = b->d_status;
-    a.total = b->total;
-    if (b->two) batch_kernel<true><<<b->grid[1], kThreads, b->smem, st>>>(a);
-    else batch_kernel<false><<<b->grid[0], kThreads, b->smem, st>>>(a);
-    BCK(cudaGetLastError(), "batch launch");
+    BCK(cudaMemsetAsync(b->d_head, 0, 4 * sizeof(unsigned long long), st), "reset queue");
+    BCK(cudaMemsetAsync(b->d_done, 0, sizeof(unsigned) * b->ndone, st), "reset counters");
+    if (b->runs.size() > 1) BCK(cudaEventRecord(b->fork, st), "batch launch");
+    for (size_t r = 0; r < b->runs.size(); ++r) {
+        const b2r_batch::Launch& u = b->runs[r];
+        cudaStream_t s = r == 0 ? st : b->side[r - 1];
+        if (r > 0) BCK(cudaStreamWaitEvent(s, b->fork, 0), "batch launch");
+        BatchArgs a;
+        a.inst = b->d_inst + u.first;
+        a.maps = b->d_maps + 2 * u.first;
+        a.items = b->d_items + u.at;
+        a.head = b->d_head + r;
+        a.done = b->d_done;
+        a.status = b->d_status;
+        a.total = u.total;
+        if (b->two) batch_kernel<true><<<b->grid[4], kThreads, b->smem, s>>>(a);
+        else
+            switch (u.D) {
+            case 1: batch_far_kernel<1><<<b->grid[0], kQThreads, kQSmem, s>>>(a); break;
+            case 2: batch_far_kernel<2><<<b->grid[1], kQThreads, kQSmem, s>>>(a); break;
+            case 3: batch_far_kernel<3><<<b->grid[2], kQThreads, kQSmem, s>>>(a); break;
+            default: batch_far_kernel<4><<<b->grid[3], kQThreads, kQSmem, s>>>(a); break;
+            }
+        BCK(cudaGetLastError(), "batch launch");
+        if (r > 0) {
+            BCK(cudaEventRecord(b->join[r - 1], s), "batch launch");
+            BCK(cudaStreamWaitEvent(st, b->join[r - 1], 0), "batch launch");
+        }
+    }
     return B2R_OK;
 }
 
@@ -478,11 +712,16 @@ b2r_status b2r_batch_create(const b2r_batch_item* items, int n, b2r_batch** out)
     }
     if (cudaMalloc(&b->d_inst, sizeof(InstDev) * n) != cudaSuccess ||
         cudaMalloc(&b->d_maps, sizeof(CUtensorMap) * 2 * n) != cudaSuccess ||
-        cudaMalloc(&b->d_head, sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc(&b->d_done, sizeof(unsigned) * n) != cudaSuccess ||
+        cudaMalloc(&b->d_head, 4 * sizeof(unsigned long long)) != cudaSuccess ||
         cudaMalloc(&b->d_status, sizeof(int)) != cudaSuccess)
         return bail(bfail(B2R_ERR_OOM, "batch table allocation failed"));
     cudaMemset(b->d_status, 0, sizeof(int));
+    for (int k = 0; k < 3; ++k)
+        if (cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming) != cudaSuccess)
+            return bail(bfail(B2R_ERR_CUDA, "batch streams"));
+    if (cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess)
+        return bail(bfail(B2R_ERR_CUDA, "batch streams"));
     // persistent grid: every resident slot
     b->smem = kSmem + 16 + kSmemS1;
     int dev = 0, sms = 0;
@@ -492,13 +731,16 @@ b2r_status b2r_batch_create(const b2r_batch_item* items, int n, b2r_batch** out)
         // the limit is per function and device: only ever raised, so that a
         // batch with a smaller schedule does not lower it under one created
         // before it
-        static SmemLimit limit[2];
-        const void* fns[2] = {(const void*)batch_kernel<false>, (const void*)batch_kernel<true>};
-        for (int v = 0; v < 2; ++v) {
+        static SmemLimit limit[5];
+        const void* fns[5] = {(const void*)batch_far_kernel<1>, (const void*)batch_far_kernel<2>,
+                              (const void*)batch_far_kernel<3>, (const void*)batch_far_kernel<4>,
+                              (const void*)batch_kernel<true>};
+        for (int v = 0; v < 5; ++v) {
             int occ = 0;
-            if (raise_smem_limit(limit[v], fns[v], b->smem) != cudaSuccess)
+            const size_t smem = v < 4 ? kQSmem : b->smem;
+            if (raise_smem_limit(limit[v], fns[v], smem) != cudaSuccess)
                 return bail(bfail(B2R_ERR_CUDA, "smem attribute"));
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fns[v], kThreads, b->smem);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fns[v], v < 4 ? kQThreads : kThreads, smem);
             b->grid[v] = std::max(1, occ) * std::max(1, sms);
         }
     }
@@ -513,6 +755,11 @@ b2r_status b2r_batch_destroy(b2r_batch* b)
 {
     if (!b) return B2R_OK;
     if (b->gexec) cudaGraphExecDestroy(b->gexec);
+    for (int k = 0; k < 3; ++k) {
+        if (b->side[k]) cudaStreamDestroy(b->side[k]);
+        if (b->join[k]) cudaEventDestroy(b->join[k]);
+    }
+    if (b->fork) cudaEventDestroy(b->fork);
     for (auto& in : b->host)
         for (int s = 0; s < 2; ++s)
             if (in.buf[s]) cudaFree(in.buf[s]);
@@ -583,7 +830,7 @@ b2r_status b2r_batch_run(b2r_batch* b, void* stream, int use_graph)
         b2r_status s = enqueue_run(b, st);
         if (s != B2R_OK) return s;
     }
-    count_launches(1);
+    count_launches((long long)b->runs.size());
     return B2R_OK;
 }
 

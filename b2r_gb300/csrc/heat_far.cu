@@ -24,11 +24,12 @@
 //
 // Every wait is bounded; a warp that gives up reports
 // DEV_TIMEOUT and leaves, and so does every warp that waits for it.
-#include "b2r_common.cuh"
-#include "heat.h"
+#include "heat_far.cuh"
 
 namespace b2r {
 namespace {
+
+using namespace farx;
 
 constexpr int kTW = 128;             // output cells per tile row
 
@@ -45,111 +46,6 @@ struct FCfg {
 struct FSched {
     int ntx, nty, nzc, Lz;
 };
-
-__device__ __forceinline__ float4 f4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-template <int D, int NC>
-struct FCtx {
-    float4 q[2 * D + 1][2];     // planes p-2D .. p by slot (pr mod 2D+1), rows
-    const float* ring;          // + the thread's first cell of its first row
-    uint64_t *full, *empty;
-    float* dst;                 // the thread's cells of the next output plane
-    long long plane;
-    int P, np;
-    unsigned m0, m1;            // cells stored of each row
-    bool lane0;
-};
-
-// Input plane pr (slot PH = pr mod 2D+1 of the queue); from pr = 2D on also
-// the output plane D planes back.  False if the wait gave up.
-template <int D, int NC, int PH>
-__device__ __forceinline__ bool f_iter(FCtx<D, NC>& c, const HeatCoef& C, int pr, int slot, int phase, int cslot)
-{
-    using Cfg = FCfg<D, NC>;
-    constexpr int N = 2 * D + 1, BW = Cfg::BW;
-    if (!mbar_wait_bounded(&c.full[slot], phase)) return false;
-    {
-        const float* pl = c.ring + slot * Cfg::SLOT;
-        c.q[PH][0] = f4(pl);
-        c.q[PH][1] = f4(pl + BW);
-    }
-    if (pr >= 2 * D) {
-        constexpr int CE = (PH + N - D) % N;                // the centre plane
-        const float* pc = c.ring + cslot * Cfg::SLOT;
-        const float4 c0 = c.q[CE][0], c1 = c.q[CE][1];
-        const float4 l0 = f4(pc - 4), r0 = f4(pc + 4), l1 = f4(pc + BW - 4), r1 = f4(pc + BW + 4);
-        const float v0[12] = {l0.x, l0.y, l0.z, l0.w, c0.x, c0.y, c0.z, c0.w, r0.x, r0.y, r0.z, r0.w};
-        const float v1[12] = {l1.x, l1.y, l1.z, l1.w, c1.x, c1.y, c1.z, c1.w, r1.x, r1.y, r1.z, r1.w};
-        const float2 a0 = make_float2(C.a0, C.a0);
-        float2 lo0 = __fmul2_rn(a0, make_float2(c0.x, c0.y)), hi0 = __fmul2_rn(a0, make_float2(c0.z, c0.w));
-        float2 lo1 = __fmul2_rn(a0, make_float2(c1.x, c1.y)), hi1 = __fmul2_rn(a0, make_float2(c1.z, c1.w));
-        float4 below = c0, above = c1;                      // rows -(k-1) and k of the pair
-#pragma unroll
-        for (int k = 1; k <= D; ++k) {
-            const float4 yb = f4(pc - k * BW), ya = f4(pc + (k + 1) * BW);   // rows -k and k+1
-            const float4 zm0 = c.q[(CE + N - k) % N][0], zp0 = c.q[(CE + k) % N][0];
-            const float4 zm1 = c.q[(CE + N - k) % N][1], zp1 = c.q[(CE + k) % N][1];
-            const float2 cx = make_float2(C.ax[k - 1], C.ax[k - 1]), cy = make_float2(C.ay[k - 1], C.ay[k - 1]),
-                         cz = make_float2(C.az[k - 1], C.az[k - 1]);
-            lo0 = __ffma2_rn(cx, make_float2(v0[4 - k] + v0[4 + k], v0[5 - k] + v0[5 + k]), lo0);
-            hi0 = __ffma2_rn(cx, make_float2(v0[6 - k] + v0[6 + k], v0[7 - k] + v0[7 + k]), hi0);
-            lo1 = __ffma2_rn(cx, make_float2(v1[4 - k] + v1[4 + k], v1[5 - k] + v1[5 + k]), lo1);
-            hi1 = __ffma2_rn(cx, make_float2(v1[6 - k] + v1[6 + k], v1[7 - k] + v1[7 + k]), hi1);
-            // row 0: rows -k and k; row 1: rows 1-k and 1+k
-            lo0 = __ffma2_rn(cy, __fadd2_rn(make_float2(yb.x, yb.y), make_float2(above.x, above.y)), lo0);
-            hi0 = __ffma2_rn(cy, __fadd2_rn(make_float2(yb.z, yb.w), make_float2(above.z, above.w)), hi0);
-            lo1 = __ffma2_rn(cy, __fadd2_rn(make_float2(below.x, below.y), make_float2(ya.x, ya.y)), lo1);
-            hi1 = __ffma2_rn(cy, __fadd2_rn(make_float2(below.z, below.w), make_float2(ya.z, ya.w)), hi1);
-            lo0 = __ffma2_rn(cz, __fadd2_rn(make_float2(zm0.x, zm0.y), make_float2(zp0.x, zp0.y)), lo0);
-            hi0 = __ffma2_rn(cz, __fadd2_rn(make_float2(zm0.z, zm0.w), make_float2(zp0.z, zp0.w)), hi0);
-            lo1 = __ffma2_rn(cz, __fadd2_rn(make_float2(zm1.x, zm1.y), make_float2(zp1.x, zp1.y)), lo1);
-            hi1 = __ffma2_rn(cz, __fadd2_rn(make_float2(zm1.z, zm1.w), make_float2(zp1.z, zp1.w)), hi1);
-            below = yb;
-            above = ya;
-        }
-        const float4 o0 = make_float4(lo0.x, lo0.y, hi0.x, hi0.y), o1 = make_float4(lo1.x, lo1.y, hi1.x, hi1.y);
-        float* d = c.dst;
-        if (c.m0 == 15u) *reinterpret_cast<float4*>(d) = o0;
-        else if (c.m0) {
-            if (c.m0 & 1u) d[0] = o0.x;
-            if (c.m0 & 2u) d[1] = o0.y;
-            if (c.m0 & 4u) d[2] = o0.z;
-            if (c.m0 & 8u) d[3] = o0.w;
-        }
-        d += c.P;
-        if (c.m1 == 15u) *reinterpret_cast<float4*>(d) = o1;
-        else if (c.m1) {
-            if (c.m1 & 1u) d[0] = o1.x;
-            if (c.m1 & 2u) d[1] = o1.y;
-            if (c.m1 & 4u) d[2] = o1.z;
-            if (c.m1 & 8u) d[3] = o1.w;
-        }
-        c.dst += c.plane;
-    }
-    if (pr >= D) {              // plane pr - D is read: its slot may be refilled
-        __syncwarp();
-        if (c.lane0) mbar_arrive(&c.empty[cslot]);
-    }
-    return true;
-}
-
-template <int D, int NC, int PH>
-__device__ __forceinline__ bool f_round(FCtx<D, NC>& c, const HeatCoef& C, int& pr, int& slot, int& phase, int& cslot)
-{
-    using Cfg = FCfg<D, NC>;
-    if (pr >= c.np) return true;
-    if (!f_iter<D, NC, PH>(c, C, pr, slot, phase, cslot)) return false;
-    if (pr >= D && ++cslot == Cfg::S) cslot = 0;
-    ++pr;
-    if (++slot == Cfg::S) slot = 0, phase ^= 1;
-    if constexpr (PH + 1 < 2 * D + 1) return f_round<D, NC, PH + 1>(c, C, pr, slot, phase, cslot);
-    return true;
-}
 
 template <int D, int NC>
 __global__ void __launch_bounds__(32 * (NC + 1), NC <= 7 ? 2 : 1)
@@ -210,7 +106,7 @@ heat_far_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ out
         }
         return;
     }
-    FCtx<D, NC> c;
+    FCtx<D, Cfg::S, Cfg::SLOT, Cfg::BW> c;
     c.full = full;
     c.empty = empty;
     c.plane = L.plane;
@@ -225,12 +121,8 @@ heat_far_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ out
     c.m0 = y >= lo[1] && y <= hi[1] ? m : 0u;
     c.m1 = y + 1 >= lo[1] && y + 1 <= hi[1] ? m : 0u;
     c.dst = out + (long long)blk * L.bstride + (long long)zs * L.plane + (long long)y * L.P + xs0 + 4 * lane;
-    int pr = 0, slot = 0, phase = 0, cslot = 0;
-    while (pr < np)
-        if (!f_round<D, NC, 0>(c, C, pr, slot, phase, cslot)) {
-            if (lane == 0) report(status, DEV_TIMEOUT);
-            return;
-        }
+    int slot = 0, phase = 0, cslot = 0;
+    if (!f_unit(c, ParamCoef{C}, slot, phase, cslot) && lane == 0) report(status, DEV_TIMEOUT);
 }
 
 // Tile height and z chunk of a launch: the least busy busiest SM.  A unit of

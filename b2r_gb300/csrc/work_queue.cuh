@@ -7,7 +7,8 @@
 // item with one atomicAdd on a head counter.  Before reading round t of instance
 // k it waits until done[k] >= t * units[k] (every unit of round t-1 of that
 // instance has finished), runs the unit and bumps done[k] with a release
-// reduction.  Items are claimed in increasing order and an item only waits
+// reduction.  (The heat batch's default kernel counts warps per z chunk
+// instead and waits for the chunks that a unit reads.)  Items are claimed in increasing order and an item only waits
 // on smaller items, which are held by running CTAs, so the queue cannot
 // deadlock; every wait is bounded (2 s) and reports B2R_ERR_TIMEOUT.
 #pragma once

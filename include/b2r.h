@@ -345,7 +345,8 @@ b2r_status b2r_heat_misfit_gradient(b2r_handle* h, int nsteps, int nrec, const i
 
 /* ---- batched instances (no reference counterpart) ------------------------ */
 /* Many independent single-block heat domains of uneven sizes and stencil
- * orders advanced in one persistent launch driven by a device work queue of
+ * orders advanced in persistent launches, one per stencil order in the batch
+ * (one for all with two-step units), each driven by a device work queue of
  * (time step, instance, tile chunk) items, replayable from a CUDA graph.
  * Each instance is a domain array with a fixed shell of D cells
  * ((env+2D) cells per axis, reference layout) stepped nsteps times with the
@@ -368,7 +369,7 @@ b2r_status b2r_batch_upload(b2r_batch* b, int i, const float* src, int src_is_de
 /* Result of instance i after its nsteps (synchronous for host dst). */
 b2r_status b2r_batch_download(b2r_batch* b, int i, float* dst, int dst_is_device,
                               void* cuda_stream);
-/* Run every instance to its nsteps: one persistent launch (plus two counter
+/* Run every instance to its nsteps: the persistent launches (plus two counter
  * resets), captured once into a CUDA graph and replayed when use_graph != 0
  * and the stream is not the legacy default stream.  Asynchronous. */
 b2r_status b2r_batch_run(b2r_batch* b, void* cuda_stream, int use_graph);
@@ -378,8 +379,9 @@ b2r_status b2r_batch_synchronize(b2r_batch* b, void* cuda_stream);
 int64_t b2r_batch_lups(const b2r_batch* b);
 /* Planes per work unit along z (0 = whole column). */
 b2r_status b2r_batch_set_zchunk(b2r_batch* b, int zchunk);
-/* Tile shape of the instances: 128 x 16, 64 x 32 or 32 x 64 cells (x by
- * y, for D <= 2; half the rows for D >= 3), by width 128, 64 or 32, for
+/* Tile shape of the instances: 128 x 14, 64 x 28 or 32 x 56 cells (x by y;
+ * with two-step units in the batch 16, 32 or 64 rows, half as many for D >= 3),
+ * by width 128, 64 or 32, for
  * every instance; 0 gives each instance the shape that computes the fewest
  * cells of its planes (the default at creation).  Instances of different
  * shapes share the one launch.  b2r_batch_tile returns the width shared by
