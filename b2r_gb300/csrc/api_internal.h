@@ -40,6 +40,9 @@ struct b2r_handle {
     CUtensorMap tmapf[2][3];    // boxes of heat_far.cu's three tile heights
     HeatCoef hc{};
     HeatTune tune{};
+    // heat of several blocks, or on a torus: the domain as one block, which
+    // runs of many steps go to (null: no room, or already one)
+    b2r_handle* joined = nullptr;
     // elastic wave: fields and material
     float* fld[kMaxFields] = {};
     int nfld = 0;
@@ -174,6 +177,7 @@ void fill_layout(BlockLayout& L, const int n[3], const int B[3], const int nb[3]
                  int periodic, int fixed_edge);
 size_t field_bytes(const b2r_handle* h);
 size_t domain_cells(const b2r_handle* h);
+b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined);   // joined: a handle's one-block form
 b2r_status ensure_kappa(b2r_handle* h);
 b2r_status ensure_staging(b2r_handle* h, size_t bytes);
 b2r_status build_heat_maps(b2r_handle* h);

@@ -235,7 +235,7 @@ b2r_status b2r_autotune(b2r_handle* h, int trial_steps, int best[3], double* bes
     CK(h, cudaMemcpyAsync(save, h->buf[h->cur], fb, cudaMemcpyDeviceToDevice, h->stream));
     const int save_cur = h->cur;
     const long long save_ts = h->ts;
-    const bool save_fresh = h->halos_fresh;
+    const bool save_fresh = h->halos_fresh, save_lost = h->halos_lost;
     const bool save_graphs = h->graphs;
     h->graphs = false;
     static const int zchunks[] = {0, 16, 32, 64, 128, 256};
@@ -298,6 +298,7 @@ b2r_status b2r_autotune(b2r_handle* h, int trial_steps, int best[3], double* bes
     h->cur = save_cur;
     h->ts = save_ts;
     h->halos_fresh = save_fresh;
+    h->halos_lost = save_lost;
     h->graphs = save_graphs;
     // restore the field even after a failed trial; report the first failure
     cudaError_t rerr = cudaMemcpyAsync(h->buf[h->cur], save, fb, cudaMemcpyDeviceToDevice, h->stream);

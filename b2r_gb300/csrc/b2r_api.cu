@@ -448,6 +448,63 @@ b2r_status advance(b2r_handle* h, int n)
     return B2R_OK;
 }
 
+// The one-block form of a heat domain of several blocks or on a torus.  A
+// shelled domain then needs no exchange at all; a torus keeps one, every three
+// steps (a deeper halo computes more cells than the exchanges it saves cost;
+// radius 3 and 4, whose steps are longer than an exchange is, every four).
+// 48 steps with 3 / 4 / 6 / 8 steps between exchanges: 250x186x132, radius 2,
+// 725 / 863 / 833 / 965 us, 256^3, radius 1, 887 / 1000 / 1020 / 1068; 64x66x70,
+// radius 3, 311 / 271 / 293 / 294.  Made where its two buffers take at most an
+// eighth of the free memory.
+void make_joined(b2r_handle* h)
+{
+    size_t room = 0, all = 0;
+    b2r_config c = h->cfg;
+    for (int a = 0; a < 3; ++a) c.blocks[a] = 1;
+    const int least = std::min(c.env[0], std::min(c.env[1], c.env[2]));
+    c.R = h->L.periodic ? std::max(1, std::min(c.D <= 2 ? 3 : 4, least / 2 / c.D)) : 1;
+    if (h->L.nblk == 1 && c.R <= h->cfg.R) return;
+    const double cells = (double)(c.env[0] + 2 * c.R * c.D + 64) * (c.env[1] + 2 * c.R * c.D) * (c.env[2] + 2 * c.R * c.D);
+    if (cudaMemGetInfo(&room, &all) != cudaSuccess || 8.0 * cells > (double)(room / 8)) {
+        cudaGetLastError();
+        return;
+    }
+    if (create_handle(&c, &h->joined, true) != B2R_OK) {
+        h->joined = nullptr;
+        return;
+    }
+    cudaFree(h->joined->d_status);
+    h->joined->d_status = h->d_status;
+}
+
+// Joining and splitting cost about as much as eight exchanges and ragged block
+// sweeps: us for 8 and 48 steps in blocks and joined, 48x40x32 in 2x2x1 51, 236
+// and 40, 146; 512^3 in 2x2x2, R = 2, 1030, 6305 and 1125, 4279; the torus above
+// 212, 1242 and 162, 725; a torus of radius 4, 100^3 in 1x2x1, 76, 388 and 85, 366.
+bool heat_joins(const b2r_handle* h, int n)
+{
+    return h->joined && h->tune.own && n >= (h->L.periodic && h->cfg.D >= 3 ? 20 : 10);
+}
+
+b2r_status step_joined(b2r_handle* h, int n)
+{
+    b2r_handle* j = h->joined;
+    float* const blocks = static_cast<float*>(h->buf[h->cur]);
+    CK(h, launch_join(blocks, h->L, static_cast<float*>(j->buf[j->cur]), static_cast<float*>(j->buf[1 - j->cur]), j->L,
+                      h->shell, h->stream));
+    j->stream = h->stream;
+    j->graphs = h->graphs;
+    j->ts = 0;
+    j->halos_fresh = false;
+    if (b2r_status st = b2r_step(j, n); st != B2R_OK) return fail(h, st, "%s", j->err.c_str());
+    CK(h, launch_split(static_cast<const float*>(j->buf[j->cur]), j->L, blocks, h->L, h->stream));
+    h->ts += n;
+    h->upmask = 0;
+    h->halos_fresh = false;
+    h->halos_lost = true;   // the interiors are current, the halos are not
+    return B2R_OK;
+}
+
 // Game of Life over several generations runs on the domain's bit grid unless
 // a knob asks for one of the block passes.  Packing and unpacking cost about
 // one block pass, and every exchange that falls away saves a gather: with an
@@ -541,9 +598,9 @@ bool make_block_tmap(CUtensorMap* map, const void* base, const BlockLayout& L, i
 
 }  // namespace b2r
 
-extern "C" {
+namespace b2r_api {
 
-b2r_status b2r_create(const b2r_config* cfg, b2r_handle** out)
+b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined)
 {
     if (!cfg || !out) return fail(nullptr, B2R_ERR_ARG, "null argument");
     *out = nullptr;
@@ -618,6 +675,7 @@ b2r_status b2r_create(const b2r_config* cfg, b2r_handle** out)
                 g_err = h->err;
                 return bail(st);
             }
+            if (!joined && (h->L.nblk > 1 || h->L.periodic)) make_joined(h);
         }
     } else {
         h->nfld = (c.model == B2R_MODEL_EQWP_REF) ? 10 : 9;
@@ -650,9 +708,19 @@ b2r_status b2r_create(const b2r_config* cfg, b2r_handle** out)
     return B2R_OK;
 }
 
+}  // namespace b2r_api
+
+extern "C" {
+
+b2r_status b2r_create(const b2r_config* cfg, b2r_handle** out) { return create_handle(cfg, out, false); }
+
 b2r_status b2r_destroy(b2r_handle* h)
 {
     if (!h) return B2R_OK;
+    if (h->joined) {
+        h->joined->d_status = nullptr;   // this handle's
+        b2r_destroy(h->joined);
+    }
     drop_graphs(h);
     if (h->adj_ws) cudaFree(h->adj_ws);
     for (int b = 0; b < 2; ++b)
@@ -840,6 +908,7 @@ b2r_status b2r_step(b2r_handle* h, int nsteps)
         h->halos_lost = true;   // the interiors are current, the halos between blocks are not
         return B2R_OK;
     }
+    if (heat_joins(h, nsteps)) return step_joined(h, nsteps);
     const bool use_graphs = h->graphs && h->stream != nullptr &&
                             (h->cfg.model == B2R_MODEL_HEAT || h->cfg.model == B2R_MODEL_GOL);
     int s = 0;

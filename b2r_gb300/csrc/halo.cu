@@ -237,6 +237,56 @@ gather_kernel(T* __restrict__ dom, const T* __restrict__ blocks, const BlockLayo
     }
 }
 
+// ---------------------------------------------------------------- blocks <-> one block
+// Domain cells between the blocks of layout M and one block of layout S that
+// holds the whole domain (same interior, same fixed shell or torus).  JOIN:
+// every cell, shell included, from M to S, the shell also into S's second
+// buffer; else the interior from S to M.  A warp copies one row, x-block by
+// x-block, four loads in flight per lane.
+template <bool JOIN>
+__global__ void __launch_bounds__(kRowWarps * 32)
+regrid_kernel(float* __restrict__ m, const BlockLayout M, float* __restrict__ s, float* __restrict__ s2,
+              const BlockLayout S, int shell)
+{
+    const int lane = threadIdx.x & 31, edge = JOIN ? shell : 0;
+    const int e0 = S.B[0], e1 = S.B[1], e2 = S.B[2];
+    const long long rows = (long long)(e1 + 2 * edge) * (e2 + 2 * edge);
+    for (long long r = (long long)blockIdx.x * kRowWarps + (threadIdx.x >> 5); r < rows;
+         r += (long long)gridDim.x * kRowWarps) {
+        const int g1 = (int)(r % (e1 + 2 * edge)) - edge, g2 = (int)(r / (e1 + 2 * edge)) - edge;
+        const bool out = g1 < 0 || g1 >= e1 || g2 < 0 || g2 >= e2;      // a row of the shell
+        const int b1 = owner_of(g1, M.B[1], M.nb[1]), b2 = owner_of(g2, M.B[2], M.nb[2]);
+        const long long so = (long long)(g2 + S.H) * S.plane + (long long)(g1 + S.H) * S.P + S.xoff + S.H;
+        const long long mo = (long long)(g2 - b2 * M.B[2] + M.H) * M.plane + (long long)(g1 - b1 * M.B[1] + M.H) * M.P +
+                             M.xoff + M.H;
+        const int blk_yz = M.nb[0] * (b1 + M.nb[1] * b2);
+        for (int b0 = 0; b0 < M.nb[0]; ++b0) {
+            const int lo = b0 == 0 ? -edge : b0 * M.B[0];
+            const int hi = b0 == M.nb[0] - 1 ? e0 + edge : (b0 + 1) * M.B[0];
+            const long long o = (blk_yz + b0) * M.bstride + mo - (long long)b0 * M.B[0];
+            for (int xb = lo; xb < hi; xb += 32 * kRowUnroll) {
+                float v[kRowUnroll];
+#pragma unroll
+                for (int u = 0; u < kRowUnroll; ++u) {
+                    const int x = xb + u * 32 + lane;
+                    v[u] = x < hi ? (JOIN ? m[o + x] : s[so + x]) : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < kRowUnroll; ++u) {
+                    const int x = xb + u * 32 + lane;
+                    if (x >= hi) continue;
+                    if (JOIN) {
+                        s[so + x] = v[u];
+                        if (out || x < 0 || x >= e0) s2[so + x] = v[u];
+                    } else {
+                        m[o + x] = v[u];
+                    }
+                }
+            }
+        }
+    }
+}
+
 // ---------------------------------------------------------------- one-launch exchange
 // On one GPU every block can read every other block, so each halo cell can
 // be copied straight from the block that owns it: the halo shell of a block
@@ -460,5 +510,24 @@ template cudaError_t launch_scatter<uint8_t>(const uint8_t*, uint8_t*, uint8_t*,
 template cudaError_t launch_gather<float>(float*, const float*, const BlockLayout&, int, cudaStream_t);
 template cudaError_t launch_gather<uint8_t>(uint8_t*, const uint8_t*, const BlockLayout&, int,
                                             cudaStream_t);
+
+cudaError_t launch_join(const float* blocks, const BlockLayout& M, float* s, float* s2, const BlockLayout& S, int shell,
+                        cudaStream_t st)
+{
+    const long long rows = (long long)(S.B[1] + 2 * shell) * (S.B[2] + 2 * shell);
+    regrid_kernel<true><<<grid_for(rows * 32, kRowWarps * 32), kRowWarps * 32, 0, st>>>(const_cast<float*>(blocks), M, s,
+                                                                                       s2, S, shell);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_split(const float* s, const BlockLayout& S, float* blocks, const BlockLayout& M, cudaStream_t st)
+{
+    const long long rows = (long long)S.B[1] * S.B[2];
+    regrid_kernel<false><<<grid_for(rows * 32, kRowWarps * 32), kRowWarps * 32, 0, st>>>(blocks, M, const_cast<float*>(s),
+                                                                                        nullptr, S, 0);
+    count_launches(1);
+    return cudaGetLastError();
+}
 
 }  // namespace b2r

@@ -35,4 +35,11 @@ template <typename T>
 cudaError_t launch_gather(T* dom, const T* blocks, const BlockLayout& L, int shell,
                           cudaStream_t st);
 
+// The domain's cells from the blocks of layout M into one block of layout S
+// that holds the whole domain (its shell also into the second buffer s2), and
+// the interior back.
+cudaError_t launch_join(const float* blocks, const BlockLayout& M, float* s, float* s2, const BlockLayout& S, int shell,
+                        cudaStream_t st);
+cudaError_t launch_split(const float* s, const BlockLayout& S, float* blocks, const BlockLayout& M, cudaStream_t st);
+
 }  // namespace b2r
