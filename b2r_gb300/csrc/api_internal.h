@@ -40,9 +40,10 @@ struct b2r_handle {
     CUtensorMap tmapf[2][3];    // boxes of heat_far.cu's three tile heights
     HeatCoef hc{};
     HeatTune tune{};
-    // heat of several blocks, or on a torus: the domain as one block, which
-    // runs of many steps go to (null: no room, or already one)
+    // several blocks, or heat on a torus: the domain as one block, which runs of
+    // many steps go to (null: no room, or already one); blocks_of: its owner
     b2r_handle* joined = nullptr;
+    const b2r_handle* blocks_of = nullptr;
     // elastic wave: fields and material
     float* fld[kMaxFields] = {};
     int nfld = 0;
@@ -50,6 +51,7 @@ struct b2r_handle {
     // -> v^{n+1}, s^{n+1} out of place) and tensor maps of both sets'
     // stresses; fld is always the current set
     float* fld2[kMaxFields] = {};
+    bool fld2_stale = false;   // fld2 lacks the shell (not uploaded there, or used by the one-block form)
     StressMaps smaps[2];
     bool eqwp_fused = false;   // two-pass by default: faster on this GPU so far
     bool eqwp_tma = false;     // two-pass: the stress stage with TMA-streamed inputs (eqwp_tma.cu)

@@ -260,12 +260,13 @@ b2r_status exchange_one(b2r_handle* h, int field, bool staged)
 
 EqwpStagParams stag_params(const b2r_handle* h)
 {
+    const std::vector<float>& src = h->blocks_of ? h->blocks_of->src : h->src;
     EqwpStagParams p{};
     p.dt = (float)h->cfg.dt;
     p.inv_h = (float)(1.0 / h->cfg.h);
     for (int a = 0; a < 3; ++a) p.src[a] = h->cfg.src[a];
-    p.src_host = h->src.empty() ? nullptr : h->src.data();
-    p.src_len = (int)h->src.size();
+    p.src_host = src.empty() ? nullptr : src.data();
+    p.src_len = (int)src.size();
     return p;
 }
 
@@ -292,13 +293,22 @@ b2r_status substep(b2r_handle* h, int i, bool xnext)
         h->cur = 1 - h->cur;
         return B2R_OK;
     case B2R_MODEL_EQWP_REF: {
-        EqwpRefParams p = eqwp_ref_params(h->L);
-        CK(h, launch_eqwp_ref_substep(h->fld, h->L, i, (int)(h->ts - i), p, h->stream));
+        // the body force is a patch of every block, switched off at a period's start
+        const b2r_handle* o = h->blocks_of ? h->blocks_of : h;
+        const int ts = (int)(h->ts - (h->blocks_of ? h->ts % o->cfg.R : i));
+        EqwpRefParams p = eqwp_ref_params(o->L);
+        for (int a = 0; a < 3; ++a) p.every[a] = h->blocks_of ? o->L.B[a] : 1 << 30;
+        CK(h, launch_eqwp_ref_substep(h->fld, h->L, i, ts, p, h->stream));
         return B2R_OK;
     }
     case B2R_MODEL_EQWP_STAG: {
         const EqwpStagParams p = stag_params(h);
         if (h->eqwp_fused) {
+            if (h->fld2_stale) {
+                for (int f = 0; f < h->nfld; ++f)
+                    CK(h, cudaMemcpyAsync(h->fld2[f], h->fld[f], field_bytes(h), cudaMemcpyDeviceToDevice, h->stream));
+                h->fld2_stale = false;
+            }
             CK(h, launch_eqwp_stag_fused(h->smaps[0], h->fld, h->fld2, h->fld2 + B2R_F_SXX, h->mat, h->L, i,
                                          (int)h->ts, p, h->d_status, h->stream));
             for (int f = 0; f < h->nfld; ++f) std::swap(h->fld[f], h->fld2[f]);
@@ -448,14 +458,16 @@ b2r_status advance(b2r_handle* h, int n)
     return B2R_OK;
 }
 
-// The one-block form of a heat domain of several blocks or on a torus.  A
-// shelled domain then needs no exchange at all; a torus keeps one, every three
-// steps (a deeper halo computes more cells than the exchanges it saves cost;
-// radius 3 and 4, whose steps are longer than an exchange is, every four).
-// 48 steps with 3 / 4 / 6 / 8 steps between exchanges: 250x186x132, radius 2,
-// 725 / 863 / 833 / 965 us, 256^3, radius 1, 887 / 1000 / 1020 / 1068; 64x66x70,
-// radius 3, 311 / 271 / 293 / 294.  Made where its two buffers take at most an
-// eighth of the free memory.
+// The one-block form of a domain of several blocks, or of a heat domain on a
+// torus.  A shelled domain then needs no exchange at all; a torus keeps one,
+// every three steps (a deeper halo computes more cells than the exchanges it
+// saves cost; radius 3 and 4, whose steps are longer than an exchange is, every
+// four).  48 heat steps with 3 / 4 / 6 / 8 steps between exchanges:
+// 250x186x132, radius 2, 725 / 863 / 833 / 965 us, 256^3, radius 1, 887 / 1000 /
+// 1020 / 1068; 64x66x70, radius 3, 311 / 271 / 293 / 294.  Made where what it
+// allocates takes at most an eighth of the free memory: two buffers for heat,
+// ten fields for the collocated wave, the material for the staggered one, whose
+// fields lie in the second field set.
 void make_joined(b2r_handle* h)
 {
     size_t room = 0, all = 0;
@@ -464,8 +476,10 @@ void make_joined(b2r_handle* h)
     const int least = std::min(c.env[0], std::min(c.env[1], c.env[2]));
     c.R = h->L.periodic ? std::max(1, std::min(c.D <= 2 ? 3 : 4, least / 2 / c.D)) : 1;
     if (h->L.nblk == 1 && c.R <= h->cfg.R) return;
-    const double cells = (double)(c.env[0] + 2 * c.R * c.D + 64) * (c.env[1] + 2 * c.R * c.D) * (c.env[2] + 2 * c.R * c.D);
-    if (cudaMemGetInfo(&room, &all) != cudaSuccess || 8.0 * cells > (double)(room / 8)) {
+    const int nf = c.model == B2R_MODEL_HEAT ? 2 : c.model == B2R_MODEL_EQWP_REF ? 10 : 3;
+    const int H = c.R * halo_per_step(c);
+    const double cells = (double)(c.env[0] + 2 * H + 64) * (c.env[1] + 2 * H) * (c.env[2] + 2 * H);
+    if (cudaMemGetInfo(&room, &all) != cudaSuccess || 4.0 * nf * cells > (double)(room / 8)) {
         cudaGetLastError();
         return;
     }
@@ -473,31 +487,70 @@ void make_joined(b2r_handle* h)
         h->joined = nullptr;
         return;
     }
+    if (c.model == B2R_MODEL_EQWP_STAG && field_bytes(h->joined) > field_bytes(h)) {
+        b2r_destroy(h->joined);
+        h->joined = nullptr;
+        return;
+    }
+    h->joined->blocks_of = h;
     cudaFree(h->joined->d_status);
     h->joined->d_status = h->d_status;
 }
 
-// Joining and splitting cost about as much as eight exchanges and ragged block
-// sweeps: us for 8 and 48 steps in blocks and joined, 48x40x32 in 2x2x1 51, 236
-// and 40, 146; 512^3 in 2x2x2, R = 2, 1030, 6305 and 1125, 4279; the torus above
-// 212, 1242 and 162, 725; a torus of radius 4, 100^3 in 1x2x1, 76, 388 and 85, 366.
-bool heat_joins(const b2r_handle* h, int n)
+// The collocated wave's force patch (interior coordinates of a block) acts on
+// a block's own cells only, not on a neighbour's copies of them: the one-block
+// form gives the same where no such copy is stepped, with one step per period
+// or a patch farther than the halo from every face with a neighbour.
+bool force_is_inside(const b2r_handle* h)
 {
-    return h->joined && h->tune.own && n >= (h->L.periodic && h->cfg.D >= 3 ? 20 : 10);
+    const EqwpRefParams p = eqwp_ref_params(h->L);
+    const int lo[3] = {p.fx0, p.fy, p.fz0}, hi[3] = {p.fx1 - 1, p.fy, p.fz1 - 1};
+    for (int a = 0; a < 3; ++a)
+        if (h->cfg.R > 1 && h->L.nb[a] > 1 && (lo[a] < h->L.H || hi[a] >= h->L.B[a] - h->L.H)) return false;
+    return true;
+}
+
+// Whether a run of n steps goes to the one-block form.  Joining and splitting
+// cost about as much as eight exchanges and ragged block sweeps of heat: us for
+// 8 and 48 steps in blocks and joined, 48x40x32 in 2x2x1 51, 236 and 40, 146;
+// 512^3 in 2x2x2, R = 2, 1030, 6305 and 1125, 4279; the torus above 212, 1242
+// and 162, 725; a torus of radius 4, 100^3 in 1x2x1, 76, 388 and 85, 366.
+// The elastic wave pays about 1.4 steps for it; us per step in blocks and joined:
+// 512x512x256 in 2x2x1, R = 2, 1547 and 1334 (even at 9 steps), 256^3 in 2x1x1,
+// R = 1, 485 and 355 (5), 128^3 in 2x2x2 90 and 51 (4), 64^3 in 2x1x1 18.8 and
+// 9.0 (4); split along z alone, the cheapest to sweep, 320x100x320 in two 254
+// and 239 (22); collocated, 150x180x200 in 1x2x2, 200 and 174 (12).
+bool joins(const b2r_handle* h, int n)
+{
+    if (!h->joined) return false;
+    if (h->cfg.model == B2R_MODEL_HEAT) return h->tune.own && n >= (h->L.periodic && h->cfg.D >= 3 ? 20 : 10);
+    if (n < (h->L.nb[0] * h->L.nb[1] > 1 ? 12 : 24)) return false;
+    if (h->cfg.model == B2R_MODEL_EQWP_REF) return force_is_inside(h);
+    return !h->eqwp_fused && !h->eqwp_tma && !h->eqwp_overlap;
 }
 
 b2r_status step_joined(b2r_handle* h, int n)
 {
     b2r_handle* j = h->joined;
-    float* const blocks = static_cast<float*>(h->buf[h->cur]);
-    CK(h, launch_join(blocks, h->L, static_cast<float*>(j->buf[j->cur]), static_cast<float*>(j->buf[1 - j->cur]), j->L,
-                      h->shell, h->stream));
+    const int nf = std::max(1, h->nfld);
+    RegridFields F{};
+    for (int f = 0; f < nf; ++f) {
+        F.m[f] = h->nfld ? h->fld[f] : static_cast<float*>(h->buf[h->cur]);
+        if (h->cfg.model == B2R_MODEL_EQWP_STAG) {
+            j->fld[f] = h->fld2[f];
+            h->fld2_stale = true;
+        }
+        F.s[f] = h->nfld ? j->fld[f] : static_cast<float*>(j->buf[j->cur]);
+        F.s2[f] = static_cast<float*>(j->buf[1 - j->cur]);
+    }
+    CK(h, launch_join(F, nf, h->L, j->L, h->shell, h->stream));
     j->stream = h->stream;
     j->graphs = h->graphs;
-    j->ts = 0;
+    j->ts = h->nfld ? h->ts : 0;
     j->halos_fresh = false;
     if (b2r_status st = b2r_step(j, n); st != B2R_OK) return fail(h, st, "%s", j->err.c_str());
-    CK(h, launch_split(static_cast<const float*>(j->buf[j->cur]), j->L, blocks, h->L, h->stream));
+    if (!h->nfld) F.s[0] = static_cast<float*>(j->buf[j->cur]);
+    CK(h, launch_split(F, nf, h->L, j->L, h->stream));
     h->ts += n;
     h->upmask = 0;
     h->halos_fresh = false;
@@ -679,7 +732,7 @@ b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined)
         }
     } else {
         h->nfld = (c.model == B2R_MODEL_EQWP_REF) ? 10 : 9;
-        for (int f = 0; f < h->nfld; ++f) {
+        for (int f = 0; f < h->nfld && !(joined && c.model == B2R_MODEL_EQWP_STAG); ++f) {
             if (cudaMalloc(&h->fld[f], fb) != cudaSuccess)
                 return bail(fail(nullptr, B2R_ERR_OOM, "cudaMalloc of %zu bytes failed", fb));
             cudaMemset(h->fld[f], 0, fb);
@@ -690,17 +743,18 @@ b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined)
                     return bail(fail(nullptr, B2R_ERR_OOM, "cudaMalloc of %zu bytes failed", fb));
                 cudaMemset(h->mat[m], 0, fb);
             }
-            for (int f = 0; f < h->nfld; ++f) {
+            for (int f = 0; f < h->nfld && !joined; ++f) {
                 if (cudaMalloc(&h->fld2[f], fb) != cudaSuccess)
                     return bail(fail(nullptr, B2R_ERR_OOM, "cudaMalloc of %zu bytes failed", fb));
                 cudaMemset(h->fld2[f], 0, fb);
             }
             const int box = eqwp_fused_box();
-            for (int f = 0; f < 6; ++f)
+            for (int f = 0; f < 6 && !joined; ++f)
                 if (!make_block_tmap(&h->smaps[0].m[f], h->fld[B2R_F_SXX + f], h->L, 4, box, box, 1) ||
                     !make_block_tmap(&h->smaps[1].m[f], h->fld2[B2R_F_SXX + f], h->L, 4, box, box, 1))
                     return bail(fail(nullptr, B2R_ERR_CUDA, "cuTensorMapEncodeTiled failed"));
         }
+        if (!joined && h->L.nblk > 1 && !h->L.periodic) make_joined(h);
     }
     if (cudaDeviceSynchronize() != cudaSuccess)
         return bail(fail(nullptr, B2R_ERR_CUDA, "device initialisation failed"));
@@ -719,6 +773,8 @@ b2r_status b2r_destroy(b2r_handle* h)
     if (!h) return B2R_OK;
     if (h->joined) {
         h->joined->d_status = nullptr;   // this handle's
+        if (h->cfg.model == B2R_MODEL_EQWP_STAG)
+            for (float*& f : h->joined->fld) f = nullptr;   // so are these
         b2r_destroy(h->joined);
     }
     drop_graphs(h);
@@ -822,9 +878,14 @@ b2r_status b2r_upload(b2r_handle* h, int field, const void* src, int src_is_devi
     void* dst2 = nullptr;   // written with the same cells in the same pass
     if (is_mat) {
         dst = h->mat[field - B2R_F_LAMBDA];
+        if (h->joined)
+            CK(h, launch_scatter<float>(static_cast<const float*>(dsrc), h->joined->mat[field - B2R_F_LAMBDA], nullptr,
+                                        h->joined->L, h->shell, h->stream));
     } else if (eq) {
         dst = h->fld[field];
-        dst2 = h->fld2[field];   // both staggered field sets carry the shell
+        // the one-pass step needs the shell in both field sets
+        if (h->eqwp_fused) dst2 = h->fld2[field];
+        else h->fld2_stale = true;
     } else {
         dst = h->buf[h->cur];
         dst2 = h->buf[1 - h->cur];   // so do both ping-pong buffers (heat-3D.cu:591-592)
@@ -836,7 +897,7 @@ b2r_status b2r_upload(b2r_handle* h, int field, const void* src, int src_is_devi
         CK(h, launch_scatter<float>(static_cast<const float*>(dsrc), static_cast<float*>(dst),
                                     static_cast<float*>(dst2), h->L, h->shell, h->stream));
     h->ts = 0;
-    h->halos_lost = false;   // Game of Life alone sets it, and has one field
+    h->halos_lost = false;   // a period starts, with an exchange unless every field is uploaded
     // the scatter filled this field's halos; the others are fresh only if
     // they were, or once every field has been uploaded since the last step
     if (!h->halos_fresh && !is_mat) {   // material never changes: its halos stay consistent
@@ -908,7 +969,7 @@ b2r_status b2r_step(b2r_handle* h, int nsteps)
         h->halos_lost = true;   // the interiors are current, the halos between blocks are not
         return B2R_OK;
     }
-    if (heat_joins(h, nsteps)) return step_joined(h, nsteps);
+    if (joins(h, nsteps)) return step_joined(h, nsteps);
     const bool use_graphs = h->graphs && h->stream != nullptr &&
                             (h->cfg.model == B2R_MODEL_HEAT || h->cfg.model == B2R_MODEL_GOL);
     int s = 0;

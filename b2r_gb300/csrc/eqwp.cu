@@ -132,7 +132,13 @@ eqwp_ref_velocity(FieldPtrs F, const BlockLayout L, int step_i, Tiles T, EqwpRef
         qxz.p2 = ld4(sxz + o + 3 * S); qyz.p2 = ld4(syz + o + 3 * S); qzz.p2 = ld4(szz + o + 3 * S);
     }
     const float a = p.ca, b = p.cb;
-    const bool frow = (c.y == p.fy) && (ts < p.fsteps);
+    const bool frow = (c.y - L.H) % p.every[1] == p.fy && ts < p.fsteps;
+    unsigned fx = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int x = (c.xb + j - L.H) % p.every[0];
+        if (frow && x >= p.fx0 && x < p.fx1) fx |= 1u << j;
+    }
     for (int z = w.zs; z <= w.ze; ++z) {
         const long long o = (long long)z * S;
         if (B2R_EQWP_PREFETCH > 0) {
@@ -158,7 +164,11 @@ eqwp_ref_velocity(FieldPtrs F, const BlockLayout L, int step_i, Tiles T, EqwpRef
         const float4 xym2 = ld4(sxy + o - 2 * P), xym1 = ld4(sxy + o - P), xyp1 = ld4(sxy + o + P), xyp2 = ld4(sxy + o + 2 * P);
         const float4 yym2 = ld4(syy + o - 2 * P), yym1 = ld4(syy + o - P), yyp1 = ld4(syy + o + P), yyp2 = ld4(syy + o + 2 * P);
         const float4 yzm2 = ld4(syz + o - 2 * P), yzm1 = ld4(syz + o - P), yzp1 = ld4(syz + o + P), yzp2 = ld4(syz + o + 2 * P);
-        const bool fz = frow && z >= p.fz0 && z < p.fz1;
+        unsigned f = 0;
+        if (fx) {
+            const int zl = (z - L.H) % p.every[2];
+            if (zl >= p.fz0 && zl < p.fz1) f = fx;
+        }
         float* const dst[4] = {F.p[VX] + c.base + o, F.p[VY] + c.base + o, F.p[VZ] + c.base + o,
                                F.p[DISP] + c.base + o};
         float4 old[4];
@@ -173,7 +183,7 @@ eqwp_ref_velocity(FieldPtrs F, const BlockLayout L, int step_i, Tiles T, EqwpRef
                        dc4(qyz.m2, qyz.m1, qyz.p1, qyz.p2, j, a, b);
             const float sz = dcx(rxz, j, a, b) + dc4(yzm2, yzm1, yzp1, yzp2, j, a, b) +
                              dc4(qzz.m2, qzz.m1, qzz.p1, qzz.p2, j, a, b);
-            if (fz && c.xb + j >= p.fx0 && c.xb + j < p.fx1) sy += p.fval;
+            if (f & (1u << j)) sy += p.fval;
             dvx[j] = p.dt_rho * sx;
             dvy[j] = p.dt_rho * sy;
             dvz[j] = p.dt_rho * sz;
@@ -249,14 +259,15 @@ EqwpRefParams eqwp_ref_params(const BlockLayout& L)
     p.fsteps = 50;
     // Force patch of eqwp.cu:561-566 and plane of eqwp.cu:135, as the
     // reference places them in its block of Ng = B + 4 cells (R = 1), mapped
-    // to this block (interior starts at H): plane y = B - 7 of the interior,
-    // x and z in [Ng/2 - 2, Ng/2 + Ng/10 - 2).
+    // to the interior of this block: plane y = B - 7, x and z in
+    // [Ng/2 - 2, Ng/2 + Ng/10 - 2).
     const int ngx = L.B[0] + 4, ngz = L.B[2] + 4;
-    p.fy = L.H + L.B[1] - 7;
-    p.fx0 = L.H + ngx / 2 - 2;
-    p.fx1 = L.H + ngx / 2 + ngx / 10 - 2;
-    p.fz0 = L.H + ngz / 2 - 2;
-    p.fz1 = L.H + ngz / 2 + ngz / 10 - 2;
+    p.fy = L.B[1] - 7;
+    p.fx0 = ngx / 2 - 2;
+    p.fx1 = ngx / 2 + ngx / 10 - 2;
+    p.fz0 = ngz / 2 - 2;
+    p.fz1 = ngz / 2 + ngz / 10 - 2;
+    for (int& e : p.every) e = 1 << 30;
     return p;
 }
 

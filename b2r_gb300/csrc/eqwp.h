@@ -20,7 +20,8 @@ struct EqwpRefParams {
     float dt_rho, dt2_rho;           // dt/rho, dt^2/rho
     float fval;                      // body force (y)
     int fsteps;                      // force active while ts < fsteps
-    int fy, fx0, fx1, fz0, fz1;      // force plane / patch (block coordinates)
+    int fy, fx0, fx1, fz0, fz1;      // force plane / patch (interior coordinates),
+    int every[3];                    // repeated with these periods
 };
 
 struct EqwpStagParams {

@@ -241,13 +241,15 @@ gather_kernel(T* __restrict__ dom, const T* __restrict__ blocks, const BlockLayo
 // Domain cells between the blocks of layout M and one block of layout S that
 // holds the whole domain (same interior, same fixed shell or torus).  JOIN:
 // every cell, shell included, from M to S, the shell also into S's second
-// buffer; else the interior from S to M.  A warp copies one row, x-block by
-// x-block, four loads in flight per lane.
+// buffer if it has one; else the interior from S to M.  blockIdx.y: field.  A
+// warp copies one row, x-block by x-block, four loads in flight per lane.
 template <bool JOIN>
 __global__ void __launch_bounds__(kRowWarps * 32)
-regrid_kernel(float* __restrict__ m, const BlockLayout M, float* __restrict__ s, float* __restrict__ s2,
-              const BlockLayout S, int shell)
+regrid_kernel(const RegridFields F, const BlockLayout M, const BlockLayout S, int shell)
 {
+    float* const m = F.m[blockIdx.y];
+    float* const s = F.s[blockIdx.y];
+    float* const s2 = F.s2[blockIdx.y];
     const int lane = threadIdx.x & 31, edge = JOIN ? shell : 0;
     const int e0 = S.B[0], e1 = S.B[1], e2 = S.B[2];
     const long long rows = (long long)(e1 + 2 * edge) * (e2 + 2 * edge);
@@ -277,7 +279,7 @@ regrid_kernel(float* __restrict__ m, const BlockLayout M, float* __restrict__ s,
                     if (x >= hi) continue;
                     if (JOIN) {
                         s[so + x] = v[u];
-                        if (out || x < 0 || x >= e0) s2[so + x] = v[u];
+                        if (s2 && (out || x < 0 || x >= e0)) s2[so + x] = v[u];
                     } else {
                         m[o + x] = v[u];
                     }
@@ -511,21 +513,19 @@ template cudaError_t launch_gather<float>(float*, const float*, const BlockLayou
 template cudaError_t launch_gather<uint8_t>(uint8_t*, const uint8_t*, const BlockLayout&, int,
                                             cudaStream_t);
 
-cudaError_t launch_join(const float* blocks, const BlockLayout& M, float* s, float* s2, const BlockLayout& S, int shell,
+cudaError_t launch_join(const RegridFields& F, int nf, const BlockLayout& M, const BlockLayout& S, int shell,
                         cudaStream_t st)
 {
     const long long rows = (long long)(S.B[1] + 2 * shell) * (S.B[2] + 2 * shell);
-    regrid_kernel<true><<<grid_for(rows * 32, kRowWarps * 32), kRowWarps * 32, 0, st>>>(const_cast<float*>(blocks), M, s,
-                                                                                       s2, S, shell);
+    regrid_kernel<true><<<dim3(grid_for(rows * 32, kRowWarps * 32), nf), kRowWarps * 32, 0, st>>>(F, M, S, shell);
     count_launches(1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_split(const float* s, const BlockLayout& S, float* blocks, const BlockLayout& M, cudaStream_t st)
+cudaError_t launch_split(const RegridFields& F, int nf, const BlockLayout& M, const BlockLayout& S, cudaStream_t st)
 {
     const long long rows = (long long)S.B[1] * S.B[2];
-    regrid_kernel<false><<<grid_for(rows * 32, kRowWarps * 32), kRowWarps * 32, 0, st>>>(blocks, M, const_cast<float*>(s),
-                                                                                        nullptr, S, 0);
+    regrid_kernel<false><<<dim3(grid_for(rows * 32, kRowWarps * 32), nf), kRowWarps * 32, 0, st>>>(F, M, S, 0);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -35,11 +35,16 @@ template <typename T>
 cudaError_t launch_gather(T* dom, const T* blocks, const BlockLayout& L, int shell,
                           cudaStream_t st);
 
-// The domain's cells from the blocks of layout M into one block of layout S
-// that holds the whole domain (its shell also into the second buffer s2), and
-// the interior back.
-cudaError_t launch_join(const float* blocks, const BlockLayout& M, float* s, float* s2, const BlockLayout& S, int shell,
+// nf fields of a domain between the blocks of layout M (m) and one block of
+// layout S that holds the whole domain (s): every cell into S, its shell also
+// into the second buffer s2 unless that is null, and the interior back.
+struct RegridFields {
+    float* m[kMaxFields];
+    float* s[kMaxFields];
+    float* s2[kMaxFields];
+};
+cudaError_t launch_join(const RegridFields& F, int nf, const BlockLayout& M, const BlockLayout& S, int shell,
                         cudaStream_t st);
-cudaError_t launch_split(const float* s, const BlockLayout& S, float* blocks, const BlockLayout& M, cudaStream_t st);
+cudaError_t launch_split(const RegridFields& F, int nf, const BlockLayout& M, const BlockLayout& S, cudaStream_t st);
 
 }  // namespace b2r
