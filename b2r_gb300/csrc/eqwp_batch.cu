@@ -8,12 +8,19 @@
 // of the queue: the velocity stage, then the stress stage, each over the
 // tiles x z chunks of the stage kernels' grid (eqwp_stag.cuh, the same
 // bodies as the stage launches, so results are bit-identical to stepping
-// each handle on its own).  The stages update their fields in place; a round
-// starts only after every unit of the instance's previous round has
-// finished, which orders both the reads of the neighbours' new values and
-// the in-place writes after the previous stage's reads.  The fields are
-// read through coherent loads (other CTAs update them between rounds); the
-// material through the read-only path.
+// each handle on its own).  The stages update their fields in place, and
+// reach two planes: a unit starts when every unit of the previous round in its
+// own z chunk and the chunks within two planes of it has finished (one counter
+// per chunk), which orders both the reads of the neighbours' new values and
+// the in-place writes after the previous stage's reads.  Against one counter
+// per instance the next round starts while the last units of a round still
+// run, so units can be longer: two instances of 144^3 41.5 GLUPS in units of
+// 12 planes, 37.4 with one counter (40.8 and 40.5 in units of 8).  DRAM moves
+// 0.70 of the copy rate on 16 instances of 32-128 cells per edge (39.8 GLUPS);
+// working through them in sets that fit L2, or with the rounds of all spread
+// evenly over the queue, was slower (30 to 34: too few units in flight; 39.3).
+// The fields are read through coherent loads (other CTAs update them between
+// rounds); the material through the read-only path.
 #include <algorithm>
 #include <cstdio>
 #include <new>
@@ -37,13 +44,16 @@ struct EInst {
     const float* amp;          // source increment of each step of the run (device)
     int gx, gy, bx, by;        // tiles per row / column of the stage grid, CTA shape
     int nsteps, rounds, units;
+    int tiles;                 // units of a z chunk and round
+    int chunk0;                // the instance's first chunk counter
+    int reach;                 // chunks that two planes reach
 };
 
 struct EArgs {
     const EInst* inst;                   // sorted by rounds, descending
     const unsigned long long* items;     // the queue: work items in claim order
     unsigned long long* head;
-    unsigned* done;
+    unsigned* done;                      // units finished per z chunk, all rounds
     int* status;
     long long total;
 };
@@ -63,8 +73,15 @@ __global__ void __launch_bounds__(kEThreads, B2R_EQWP_MINB) eqwp_batch_kernel(co
             if (item < a.total) {
                 int t, k, u;
                 wq::unpack_item(a.items[item], t, k, u);
-                // wait for round t-1 of this instance (bounded)
-                s_ok = t == 0 || wq::wait_done(&a.done[k], (unsigned)t * (unsigned)a.inst[k].units);
+                // wait for round t-1 of the chunks that the unit reads (bounded)
+                s_ok = 1;
+                if (t > 0) {
+                    const EInst& in = a.inst[k];
+                    const unsigned need = (unsigned)t * (unsigned)in.tiles;
+                    const int zc = u / in.tiles, last = min(zc + in.reach, in.T.nzc - 1);
+                    for (int c = max(zc - in.reach, 0); c <= last && s_ok; ++c)
+                        s_ok = wq::wait_done(&a.done[in.chunk0 + c], need);
+                }
                 s_t = t;
                 s_k = k;
                 s_u = u;
@@ -95,7 +112,7 @@ __global__ void __launch_bounds__(kEThreads, B2R_EQWP_MINB) eqwp_batch_kernel(co
                 stag_velocity_unit<false, false>(in.F, in.F, in.M, in.L, 0, in.T, in.p, AccPtrs{}, 0, zc, q);
         }
         __syncthreads();                     // every store of this unit is issued
-        if (threadIdx.x == 0) wq::release_done(&a.done[k]);
+        if (threadIdx.x == 0) wq::release_done(&a.done[in.chunk0 + zc]);
     }
 }
 
@@ -114,7 +131,8 @@ struct b2r_eqwp_batch {
     unsigned long long* d_items = nullptr;   // the queue (capacity items_cap)
     long long items_cap = 0;
     unsigned long long* d_head = nullptr;
-    unsigned* d_done = nullptr;
+    unsigned* d_done = nullptr;      // the z chunks' counters (capacity chunks_cap)
+    int chunks = 0, chunks_cap = 0;
     int* d_status = nullptr;
     long long total = 0;
     int lz_policy = -1;              // z chunk cap per unit; -1: by the batch's size (auto_lz)
@@ -147,23 +165,43 @@ b2r_status efail(b2r_status s, const char* msg, cudaError_t e = cudaSuccess)
         }                                                                                    \
     } while (0)
 
-// z chunk of the units when the caller set none: short units keep more of a
-// round in flight, which small instances need (16 instances of 32-128 cells
-// per edge: 36.9 GLUPS at 8 planes, 26.1 at 32), while large ones have work
-// enough in 32-plane units and re-read fewer z-skirt planes with them -- 8
-// planes when units of 32 would give fewer than 8 per resident CTA in a
-// round, else 32.
+static int planes_of(const EInst& in)
+{
+    int lo, hi;
+    stage_region(in.L, edge_bits(in.L, 0), 2, 2, lo, hi);
+    return std::max(1, hi - lo + 1);
+}
+
+// z chunk of the units when the caller set none: the one with the shortest
+// run if a unit takes 4 us and 2.05 us per plane (eqwp_tile.cuh) and a
+// round lasts one unit at least, or as many units one after the other as each
+// resident CTA gets; at most 12 planes, beyond which neighbouring tiles lose
+// their L2 hits.  GLUPS by planes 3, 4, 6, 8, 12, 16, 32: 16 instances of
+// 32-128 cells per edge 31.7, 34.2, 37.5, 38.8, 39.7, 39.8, 31.6; 8 of 64^3
+// 34.9, 37.5, 40.0, 32.8, 25.8, 18.8, 10.1; 12 of 36^3 23.4, 18.5, 13.4, 10.6,
+// 7.4, 7.4, 5.3; 6 of 200^3 32.4, 35.7, 38.9, 40.4, 40.1, 38.3, 34.5.
 static int auto_lz(const b2r_eqwp_batch* b)
 {
-    long long units = 0;
-    for (int k = 0; k < b->n; ++k) {
-        const EInst& in = b->host[k];
-        int lo, hi;
-        stage_region(in.L, edge_bits(in.L, 0), 2, 2, lo, hi);
-        const int nz = std::max(1, hi - lo + 1);
-        units += (long long)in.gx * in.gy * ((nz + 31) / 32);
+    std::vector<int> by(b->n);
+    for (int k = 0; k < b->n; ++k) by[k] = k;
+    std::sort(by.begin(), by.end(), [&](int x, int y) { return b->nsteps[x] > b->nsteps[y]; });
+    int best = 2;
+    double least = 1e300;
+    for (int lz = 2; lz <= 12; ++lz) {
+        double us = 0;
+        long long units = 0;   // of a round in which the first j + 1 instances still step
+        for (int j = 0; j < b->n; ++j) {
+            const EInst& in = b->host[by[j]];
+            units += (long long)in.gx * in.gy * ((planes_of(in) + lz - 1) / lz);
+            const int rounds = 2 * (b->nsteps[by[j]] - (j + 1 < b->n ? b->nsteps[by[j + 1]] : 0));
+            us += rounds * std::max(1.0, (double)units / b->grid) * (4 + 2.05 * lz);
+        }
+        if (us < least) {
+            least = us;
+            best = lz;
+        }
     }
-    return units < 8LL * b->grid ? 8 : 32;
+    return best;
 }
 
 // tiles, z chunks and the queue for the current z-chunk policy
@@ -181,13 +219,13 @@ b2r_status build(b2r_eqwp_batch* b)
     const int policy = b->lz_policy >= 0 ? b->lz_policy : auto_lz(b);
     for (int k = 0; k < b->n; ++k) {
         EInst& in = b->host[k];
-        int lo, hi;
-        stage_region(in.L, edge_bits(in.L, 0), 2, 2, lo, hi);
-        const int nz = std::max(1, hi - lo + 1);
+        const int nz = planes_of(in);
         const int lz = policy > 0 ? std::min(policy, nz) : nz;
         in.T.nzc = (nz + lz - 1) / lz;
         in.units = in.gx * in.gy * in.T.nzc;
         in.rounds = 2 * in.nsteps;
+        in.tiles = in.gx * in.gy;
+        in.reach = lz >= 2 ? 1 : 2;
     }
     b->sched.resize(b->n);
     for (int k = 0; k < b->n; ++k) b->sched[k] = k;
@@ -197,6 +235,7 @@ b2r_status build(b2r_eqwp_batch* b)
     std::vector<int> rounds(b->n), units(b->n);
     for (int j = 0; j < b->n; ++j) {
         dev[j] = b->host[b->sched[j]];
+        dev[j].chunk0 = j ? dev[j - 1].chunk0 + dev[j - 1].T.nzc : 0;
         rounds[j] = dev[j].rounds;
         units[j] = dev[j].units;
     }
@@ -214,6 +253,15 @@ b2r_status build(b2r_eqwp_batch* b)
         ECK(cudaMalloc(&b->d_items, sizeof(unsigned long long) * std::max<long long>(1, b->total)), "queue allocation");
         b->items_cap = b->total;
     }
+    const int chunks = dev[b->n - 1].chunk0 + dev[b->n - 1].T.nzc;
+    if (chunks > b->chunks_cap) {
+        cudaFree(b->d_done);
+        b->d_done = nullptr;
+        b->chunks_cap = 0;
+        ECK(cudaMalloc(&b->d_done, sizeof(unsigned) * chunks), "counter allocation");
+        b->chunks_cap = chunks;
+    }
+    b->chunks = chunks;
     ECK(cudaMemcpy(b->d_inst, dev.data(), sizeof(EInst) * b->n, cudaMemcpyHostToDevice), "copy descriptors");
     if (b->total > 0)
         ECK(cudaMemcpy(b->d_items, items.data(), sizeof(unsigned long long) * b->total, cudaMemcpyHostToDevice),
@@ -228,7 +276,7 @@ b2r_status build(b2r_eqwp_batch* b)
 b2r_status enqueue(b2r_eqwp_batch* b, cudaStream_t st)
 {
     ECK(cudaMemsetAsync(b->d_head, 0, sizeof(unsigned long long), st), "reset queue");
-    ECK(cudaMemsetAsync(b->d_done, 0, sizeof(unsigned) * b->n, st), "reset counters");
+    ECK(cudaMemsetAsync(b->d_done, 0, sizeof(unsigned) * b->chunks, st), "reset counters");
     EArgs a;
     a.inst = b->d_inst;
     a.items = b->d_items;
@@ -291,7 +339,6 @@ b2r_status b2r_eqwp_batch_create(b2r_handle* const* hs, const int* nsteps, int n
     if (cudaMalloc(&b->d_inst, sizeof(EInst) * n) != cudaSuccess ||
         cudaMalloc(&b->d_amp, sizeof(float) * namp) != cudaSuccess ||
         cudaMalloc(&b->d_head, sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc(&b->d_done, sizeof(unsigned) * n) != cudaSuccess ||
         cudaMalloc(&b->d_status, sizeof(int)) != cudaSuccess)
         return bail(efail(B2R_ERR_OOM, "batch table allocation failed"));
     cudaMemset(b->d_status, 0, sizeof(int));

@@ -4,13 +4,14 @@
 // Work items (round t, instance k, unit u) are listed round-major by the
 // host; instances are sorted by round count (descending), so the instances
 // still active at round t are a prefix of the list.  A CTA claims the next
-// item with one atomicAdd on a head counter.  Before reading round t of instance
-// k it waits until done[k] >= t * units[k] (every unit of round t-1 of that
-// instance has finished), runs the unit and bumps done[k] with a release
-// reduction.  (The heat batch's default kernel counts warps per z chunk
-// instead and waits for the chunks that a unit reads.)  Items are claimed in increasing order and an item only waits
-// on smaller items, which are held by running CTAs, so the queue cannot
-// deadlock; every wait is bounded (2 s) and reports B2R_ERR_TIMEOUT.
+// item with one atomicAdd on a head counter.  Before reading round t it waits
+// for a counter: either done[k] >= t * units[k] (every unit of round t-1 of
+// instance k has finished; the two-step heat units), or the counters of the z
+// chunks that the unit reads (one-step heat, elastic wave).  Then it runs the
+// unit and bumps its counter with a release reduction.  Items are claimed in
+// increasing order and an item only waits on smaller items, which are held by
+// running CTAs, so the queue cannot deadlock; every wait is bounded (2 s) and
+// reports B2R_ERR_TIMEOUT.
 #pragma once
 #include <vector>
 

@@ -410,8 +410,8 @@ b2r_status b2r_batch_autotune(b2r_batch* b, void* cuda_stream, int* best_zchunk,
 /* Many staggered elastic-wave handles (B2R_MODEL_EQWP_STAG, one block each,
  * fixed shell) of uneven sizes advanced in one persistent launch driven by a
  * device work queue of (stage round, instance, tile chunk) items: a time step
- * of an instance is its velocity stage then its stress stage, each waiting
- * for the instance's previous stage to finish everywhere.  Each run advances
+ * of an instance is its velocity stage then its stress stage, a unit waiting
+ * for the previous stage of the planes it reads.  Each run advances
  * handle i by nsteps[i] steps from its current time step, in place, with its
  * own material and source; results are identical to b2r_step on each handle
  * with the two-pass step.  The batch keeps pointers to the handles: they must
@@ -432,9 +432,8 @@ b2r_status b2r_eqwp_batch_run(b2r_eqwp_batch* b, void* cuda_stream, int use_grap
 b2r_status b2r_eqwp_batch_synchronize(b2r_eqwp_batch* b, void* cuda_stream);
 /* Lattice-site updates of one run (sum of interior cells x steps). */
 int64_t b2r_eqwp_batch_lups(const b2r_eqwp_batch* b);
-/* Planes per work unit along z (0 = whole column).  Default: 8 when units
- * of 32 planes would give fewer than 8 per resident CTA in a round (small
- * instances), else 32. */
+/* Planes per work unit along z (0 = whole column).  Default: of 2 to 12 those
+ * with the shortest run, estimated from the sizes and step counts. */
 b2r_status b2r_eqwp_batch_set_zchunk(b2r_eqwp_batch* b, int zchunk);
 
 /* ---- diagnostics (no reference counterpart) ------------------------------- *
