@@ -106,7 +106,20 @@ struct AdjS {
     float* g_lam;          // FP32 partial sums
     float* g_mu;
     float k;
+    // the residuals of step n-1, added to vb_y at the receivers (rec: element
+    // offsets) by the first CTA: the stress adjoint does not touch vb, and a
+    // launch of its own took 2.5 us of a 150 us reverse step at 128^3
+    float* vby;
+    const long long* rec;
+    const float* res;
+    int nrec;
 };
+__device__ __forceinline__ void inject(const AdjS& A)
+{
+    if (blockIdx.x || blockIdx.y || blockIdx.z) return;
+    for (int r = threadIdx.y * blockDim.x + threadIdx.x; r < A.nrec; r += blockDim.x * blockDim.y)
+        atomicAdd(&A.vby[A.rec[r]], A.res[r]);
+}
 
 // Adjoint of the stress stage of step n followed by the velocity-stage
 // weighting:  vb -= k * D q  (D^T E = -D: the transpose of the strain
@@ -190,6 +203,7 @@ __global__ void __launch_bounds__(kBX * kBY, B2R_EQWP_MINB)
 adj_stress_kernel(AdjS A, const BlockLayout L, Tiles T)
 {
     pdl_begin();
+    inject(A);
     const int nzc = T.nzc;
     const int blk = blockIdx.z / nzc, zc = blockIdx.z % nzc;
     const Win w = window(L, blk, zc, nzc, 4);
@@ -302,6 +316,7 @@ __global__ void __launch_bounds__(kBX * kBY, B2R_ADJ_FUSED_MINB)
 adj_stress_lm_kernel(AdjS A, const BlockLayout L, Tiles T)
 {
     pdl_begin();
+    inject(A);
     const int nzc = T.nzc;
     const int blk = blockIdx.z / nzc, zc = blockIdx.z % nzc;
     const Win w = window(L, blk, zc, nzc, 4);
@@ -376,11 +391,11 @@ adj_stress_lm_kernel(AdjS A, const BlockLayout L, Tiles T)
     }
 }
 
-__global__ void rec_sample_kernel(const float* vy, const long long* idx, int nrec, float* out)
+__global__ void rec_sample_kernel(const float* vy, long long stride, const long long* idx, int nrec, float* out)
 {
     pdl_begin();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < nrec) out[r] = vy[idx[r]];
+    if (r < nrec) out[(long long)blockIdx.y * nrec + r] = vy[blockIdx.y * stride + idx[r]];
 }
 
 __global__ void rec_inject_kernel(float* vby, const long long* idx, int nrec, const float* res)
@@ -422,9 +437,14 @@ inline int grid_for(long long work)
 
 // ---------------------------------------------------------------- driver
 
-cudaError_t adjoint_sample(const float* vy, const long long* d_idx, int nrec, float* out, cudaStream_t st)
+cudaError_t adjoint_sample(const float* vy, const long long* d_idx, int nrec, float* out, cudaStream_t st, int steps,
+                           long long stride)
 {
-    return launch_pdl(rec_sample_kernel, (nrec + 127) / 128, 128, 0, st, vy, d_idx, nrec, out);
+    for (int n = 0; n < steps; n += 65535)
+        if (cudaError_t e = launch_pdl(rec_sample_kernel, dim3((nrec + 127) / 128, std::min(steps - n, 65535)), 128, 0,
+                                       st, vy + n * stride, stride, d_idx, nrec, out + (long long)n * nrec))
+            return e;
+    return cudaSuccess;
 }
 
 cudaError_t adjoint_inject(float* vby, const long long* d_idx, int nrec, const float* res, cudaStream_t st)
@@ -434,11 +454,13 @@ cudaError_t adjoint_inject(float* vby, const long long* d_idx, int nrec, const f
 
 // Reverse step n: q (from the later step) -> vb, w, g_b; then, unless n is
 // the first step, w -> sb, q for step n-1, g_lambda, g_mu (one sweep when
-// fused, else the stress kernel and the gradient kernel).  tmp = vb[3],
-// sb[6], q[6], w[3]; v_n = forward v^n, acc_n = forward D s^n.
+// fused, else the stress kernel and the gradient kernel), and the residuals
+// res_prev of step n-1 into vb.  tmp = vb[3], sb[6], q[6], w[3]; v_n = forward
+// v^n, acc_n = forward D s^n.
 cudaError_t adjoint_step(float* const* tmp, const float* const* v_n, const float* const* acc_n,
                          const float* const* mat, float* const* g, const BlockLayout& L, float dt_h,
-                         bool last, bool fused, cudaStream_t st)
+                         bool last, bool fused, const long long* rec, int nrec, const float* res_prev,
+                         cudaStream_t st)
 {
     AdjV V;
     AdjS T;
@@ -462,6 +484,10 @@ cudaError_t adjoint_step(float* const* tmp, const float* const* v_n, const float
     T.g_lam = g[0];
     T.g_mu = g[1];
     T.k = dt_h;
+    T.vby = tmp[1];
+    T.rec = rec;
+    T.res = res_prev;
+    T.nrec = nrec;
     // the fused sweep's CTAs are one per SM, the others B2R_EQWP_MINB
     const Grid ga = stage_grid(L, 2), gb = stage_grid(L, 4, fused ? B2R_ADJ_FUSED_MINB : B2R_EQWP_MINB);
     if (cudaError_t e = launch_pdl(adj_velocity_kernel, ga.g, ga.b, 0, st, V, L, ga.t)) return e;

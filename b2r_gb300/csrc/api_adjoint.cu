@@ -75,18 +75,21 @@ b2r_status b2r_eqwp_misfit_gradient(b2r_handle* h, int nsteps, int nrec, const i
     const size_t fb = field_bytes(h);
     const size_t nseg = (size_t)(nsteps + K - 1) / K;
     // workspace, carved from one allocation kept on the handle: checkpoints
-    // (9 fields each), the replayed velocities v^{n0+k} (k = 1..K; k = 0 is
-    // the checkpoint) and stencil sums of a segment, the replay's stresses,
-    // the adjoint fields and the FP64 gradients
-    // Two replay buffers when the workspace fits: segment s-1 is replayed
-    // on a second stream while segment s runs its reverse steps.
+    // (9 fields each), the velocities v^{n0+k} (k = 1..K; k = 0 is the
+    // checkpoint) and stencil sums of a segment, the replay's stresses, the
+    // adjoint fields, the FP64 gradients as stored and as returned, receivers.
+    // Two segment buffers when the workspace fits: segment s-1 is replayed on a
+    // second stream while segment s runs its reverse steps.
+    const auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t gbytes = (size_t)h->L.bstride * sizeof(double);
-    const size_t nf_ckpt = nseg * 9, nf_v = (size_t)(K + 1) * 3, nf_a = (size_t)K * 3;
-    const size_t fba = (fb + 255) & ~(size_t)255, gba = (gbytes + 255) & ~(size_t)255;
+    const size_t ncell = (size_t)h->cfg.env[0] * h->cfg.env[1] * h->cfg.env[2];
+    const size_t nf_ckpt = nseg * 9, nf_v = (size_t)K * 3, nf_a = (size_t)K * 3;
+    const size_t fba = up(fb), gba = up(gbytes);
+    const size_t rb = up(sizeof(float) * (size_t)nrec * nsteps), ib = up(sizeof(long long) * nrec);
     int nbuf = nseg > 1 ? 2 : 1;
     for (;; --nbuf) {
-        const size_t nfields = nf_ckpt + nbuf * (nf_v + nf_a + 6) + 18 + 3;
-        const size_t need = nfields * fba + 3 * gba;
+        const size_t nfields = nf_ckpt + nbuf * (nf_v + nf_a) + 6 + 18 + 3;
+        const size_t need = nfields * fba + 3 * gba + up(ncell * sizeof(double)) + 2 * rb + ib;
         if (h->adj_ws_bytes >= need) break;
         if (h->adj_ws) cudaFree(h->adj_ws);
         h->adj_ws = nullptr;
@@ -100,50 +103,107 @@ b2r_status b2r_eqwp_misfit_gradient(b2r_handle* h, int nsteps, int nrec, const i
         if (nbuf == 1) return fail(h, B2R_ERR_OOM, "misfit gradient needs %zu bytes of workspace", need);
     }
     char* ws = static_cast<char*>(h->adj_ws);
+    auto take = [&](size_t bytes) {
+        char* p = ws;
+        ws += bytes;
+        return p;
+    };
     auto carve = [&](size_t n, std::vector<float*>& out) {
         out.resize(n);
-        for (size_t i = 0; i < n; ++i, ws += fba) out[i] = reinterpret_cast<float*>(ws);
+        for (float*& p : out) p = reinterpret_cast<float*>(take(fba));
     };
     std::vector<float*> ckpt, vrep, arep, srep, tmp;
     carve(nf_ckpt, ckpt);
     carve(nf_v * nbuf, vrep);   // buffer b: entries [b * nf_v, (b + 1) * nf_v)
     carve(nf_a * nbuf, arep);
-    carve(6 * (size_t)nbuf, srep);
+    carve(6, srep);
     carve(18, tmp);
     std::vector<float*> g32;            // FP32 partial gradient sums, folded into gp
     carve(3, g32);
     double* gp[3];
-    for (int m = 0; m < 3; ++m, ws += gba) {
-        gp[m] = reinterpret_cast<double*>(ws);
-        CK(h, cudaMemsetAsync(gp[m], 0, gbytes, h->stream));
-    }
-    for (float* b : g32) CK(h, cudaMemsetAsync(b, 0, fb, h->stream));
-    DevBuf d_idx, d_rec, d_res;
-    // cells outside the update window never change: every replay slot starts
-    // as a copy of the initial state there
-    for (size_t k = 0; k < vrep.size(); ++k)
-        CK(h, cudaMemcpyAsync(vrep[k], h->fld[B2R_F_VX + k % 3], fb, cudaMemcpyDeviceToDevice, h->stream));
-    for (float* b : arep) CK(h, cudaMemsetAsync(b, 0, fb, h->stream));
-    for (float* b : tmp) CK(h, cudaMemsetAsync(b, 0, fb, h->stream));
-    CK(h, cudaMalloc(&d_idx.p, sizeof(long long) * nrec));
-    CK(h, cudaMalloc(&d_rec.p, sizeof(float) * (size_t)nrec * nsteps));
-    CK(h, cudaMalloc(&d_res.p, sizeof(float) * (size_t)nrec * nsteps));
-    CK(h, cudaMemcpyAsync(d_idx.p, idx.data(), sizeof(long long) * nrec, cudaMemcpyHostToDevice, h->stream));
-    const long long* didx = (const long long*)d_idx.p;
+    for (double*& g : gp) g = reinterpret_cast<double*>(take(gba));
+    double* const d_out = reinterpret_cast<double*>(take(up(ncell * sizeof(double))));
+    float* const d_rec = reinterpret_cast<float*>(take(rb));
+    float* const d_res = reinterpret_cast<float*>(take(rb));
+    long long* const didx = reinterpret_cast<long long*>(take(ib));
+    CK(h, cudaMemsetAsync(tmp[0], 0, 21 * fba + 3 * gba, h->stream));   // tmp, g32 and gp
+    // shell cells never change: every velocity of a segment has the initial
+    // ones (the sums are read where they are written)
+    const long long vstride = (long long)(3 * fba / sizeof(float));
+    for (int f = 0; f < 3; ++f)
+        CK(h, launch_heat_shell(h->fld[B2R_F_VX + f], vrep[f], vstride, K * nbuf, h->L, h->shell, h->stream));
+    CK(h, cudaMemcpyAsync(didx, idx.data(), sizeof(long long) * nrec, cudaMemcpyHostToDevice, h->stream));
 
-    // forward with checkpoints every K steps and receiver samples
+    const EqwpStagParams sp = stag_params(h);
+    // v^{n0+k} of segment sgi: the checkpoint's velocities for k = 0, slot k of
+    // the segment's buffer after
+    auto vslot = [&](long long sgi, int k, int f) -> float* {
+        return k == 0 ? ckpt[sgi * 9 + B2R_F_VX + f] : vrep[(size_t)(sgi % nbuf) * nf_v + (size_t)(k - 1) * 3 + f];
+    };
+    auto aslot = [&](long long sgi, int k) -> float* const* {
+        return &arep[(size_t)(sgi % nbuf) * nf_a + (size_t)k * 3];
+    };
+    // every step of a segment with its velocities and stencil sums kept; s6: the
+    // checkpoint's stresses, updated in place
+    auto replay = [&](long long sgi, float* const* s6, cudaStream_t st) -> b2r_status {
+        const int n0 = (int)sgi * K, n1 = std::min(nsteps, n0 + K);
+        for (int n = n0; n < n1; ++n) {
+            const int k = n - n0;
+            const float* vin[3] = {vslot(sgi, k, 0), vslot(sgi, k, 1), vslot(sgi, k, 2)};
+            float* vout[3] = {vslot(sgi, k + 1, 0), vslot(sgi, k + 1, 1), vslot(sgi, k + 1, 2)};
+            CK(h, launch_eqwp_stag_step_replay(vin, s6, vout, aslot(sgi, k), h->mat, h->L, n, sp, st));
+        }
+        return B2R_OK;
+    };
+    auto replay_again = [&](long long sgi, cudaStream_t st) -> b2r_status {
+        for (int f = 0; f < 6; ++f)
+            CK(h, cudaMemcpyAsync(srep[f], ckpt[sgi * 9 + B2R_F_SXX + f], fb, cudaMemcpyDeviceToDevice, st));
+        return replay(sgi, srep.data(), st);
+    };
+
+    // forward with checkpoints every K steps and receiver samples; the last
+    // nbuf segments are kept as they are stepped, so they need no replay
+    const long long slast = (long long)nseg - 1, kept = (long long)nseg - nbuf;
     h->ts = 0;
-    for (int n = 0; n < nsteps; ++n) {
-        if (n % K == 0)
-            for (int f = 0; f < 9; ++f)
-                CK(h, cudaMemcpyAsync(ckpt[(n / K) * 9 + f], h->fld[f], fb, cudaMemcpyDeviceToDevice, h->stream));
-        if ((st = substep(h, 0)) != B2R_OK) return st;
-        h->ts++;
-        CK(h, adjoint_sample(h->fld[B2R_F_VY], didx, nrec, (float*)d_rec.p + (size_t)n * nrec, h->stream));
+    for (long long sgi = 0; sgi <= slast; ++sgi) {
+        const int n0 = (int)sgi * K, n1 = std::min(nsteps, n0 + K);
+        for (int f = 0; f < 9; ++f)
+            CK(h, cudaMemcpyAsync(ckpt[sgi * 9 + f], h->fld[f], fb, cudaMemcpyDeviceToDevice, h->stream));
+        for (int n = n0; n < n1 && sgi < kept; ++n) {
+            if ((st = substep(h, 0)) != B2R_OK) return st;
+            h->ts++;
+            CK(h, adjoint_sample(h->fld[B2R_F_VY], didx, nrec, d_rec + (size_t)n * nrec, h->stream));
+        }
+        if (sgi < kept) continue;
+        if ((st = replay(sgi, h->fld + B2R_F_SXX, h->stream)) != B2R_OK) return st;
+        CK(h, adjoint_sample(vslot(sgi, 1, 1), didx, nrec, d_rec + (size_t)n0 * nrec, h->stream, n1 - n0, vstride));
+        for (int f = 0; f < 3; ++f)
+            CK(h, cudaMemcpyAsync(h->fld[B2R_F_VX + f], vslot(sgi, n1 - n0, f), fb, cudaMemcpyDeviceToDevice,
+                                  h->stream));
+    }
+
+    // reverse sweep, segment by segment, those not kept replayed forward from
+    // their checkpoint into segment buffer sgi % nbuf first.  With two buffers
+    // the replay of the segment below runs on a second stream while this
+    // segment's reverse steps run; the results are the same bits.
+    struct AuxStream {
+        cudaStream_t s = nullptr;
+        cudaEvent_t rep[2] = {}, rev[2] = {};
+        ~AuxStream()
+        {
+            for (cudaEvent_t e : {rep[0], rep[1], rev[0], rev[1]})
+                if (e) cudaEventDestroy(e);
+            if (s) cudaStreamDestroy(s);
+        }
+    } ax;
+    if (nbuf == 2) {
+        CK(h, cudaStreamCreateWithFlags(&ax.s, cudaStreamNonBlocking));
+        for (cudaEvent_t* e : {&ax.rep[0], &ax.rep[1], &ax.rev[0], &ax.rev[1]})
+            CK(h, cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
     // misfit and residual (host, FP64)
     std::vector<float> syn((size_t)nrec * nsteps), res((size_t)nrec * nsteps);
-    CK(h, cudaMemcpyAsync(syn.data(), d_rec.p, sizeof(float) * syn.size(), cudaMemcpyDeviceToHost, h->stream));
+    CK(h, cudaMemcpyAsync(syn.data(), d_rec, sizeof(float) * syn.size(), cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
     double J = 0.0;
     for (size_t i = 0; i < syn.size(); ++i) {
@@ -153,95 +213,43 @@ b2r_status b2r_eqwp_misfit_gradient(b2r_handle* h, int nsteps, int nrec, const i
     }
     if (misfit) *misfit = J;
     if (d_syn) std::copy(syn.begin(), syn.end(), d_syn);
-    CK(h, cudaMemcpyAsync(d_res.p, res.data(), sizeof(float) * res.size(), cudaMemcpyHostToDevice, h->stream));
+    CK(h, cudaMemcpyAsync(d_res, res.data(), sizeof(float) * res.size(), cudaMemcpyHostToDevice, h->stream));
 
-    // reverse sweep, segment by segment: each segment is replayed forward
-    // from its checkpoint into replay buffer sgi % nbuf (velocities and
-    // stencil sums of every step kept), then its reverse steps run.  With two
-    // buffers the replay of the segment below runs on a second stream while
-    // this segment's reverse steps run; the results are the same bits.
     float* const* tp = tmp.data();
     const float* mat[3] = {h->mat[0], h->mat[1], h->mat[2]};
     const float dt_h = (float)(h->cfg.dt / h->cfg.h);
-    const EqwpStagParams sp = stag_params(h);
-    struct AuxStream {
-        cudaStream_t s = nullptr;
-        cudaEvent_t start = nullptr, rep[2] = {}, rev[2] = {};
-        ~AuxStream()
-        {
-            for (cudaEvent_t e : {start, rep[0], rep[1], rev[0], rev[1]})
-                if (e) cudaEventDestroy(e);
-            if (s) cudaStreamDestroy(s);
-        }
-    } ax;
-    cudaStream_t aux = h->stream;
-    if (nbuf == 2) {
-        CK(h, cudaStreamCreateWithFlags(&ax.s, cudaStreamNonBlocking));
-        for (cudaEvent_t* e : {&ax.start, &ax.rep[0], &ax.rep[1], &ax.rev[0], &ax.rev[1]})
-            CK(h, cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-        aux = ax.s;
-        CK(h, cudaEventRecord(ax.start, h->stream));   // the forward and the residual are in place
-        CK(h, cudaStreamWaitEvent(aux, ax.start, 0));
-    }
-    // v^{n0+k} of segment sgi: the checkpoint's velocities for k = 0, replay
-    // slot k of the segment's buffer after
-    auto vslot = [&](long long sgi, int k, int f) -> float* {
-        return k == 0 ? ckpt[sgi * 9 + B2R_F_VX + f] : vrep[(size_t)(sgi % nbuf) * nf_v + (size_t)k * 3 + f];
-    };
-    auto aslot = [&](long long sgi, int k) -> float* const* {
-        return &arep[(size_t)(sgi % nbuf) * nf_a + (size_t)k * 3];
-    };
-    auto replay = [&](long long sgi, cudaStream_t st) -> b2r_status {
-        const int n0 = (int)sgi * K, n1 = std::min(nsteps, n0 + K);
-        float* const* s6 = srep.data() + 6 * (sgi % nbuf);
-        for (int f = 0; f < 6; ++f)
-            CK(h, cudaMemcpyAsync(s6[f], ckpt[sgi * 9 + B2R_F_SXX + f], fb, cudaMemcpyDeviceToDevice, st));
-        for (int n = n0; n < n1; ++n) {
-            const int k = n - n0;
-            const float* vin[3] = {vslot(sgi, k, 0), vslot(sgi, k, 1), vslot(sgi, k, 2)};
-            float* vout[3] = {vslot(sgi, k + 1, 0), vslot(sgi, k + 1, 1), vslot(sgi, k + 1, 2)};
-            CK(h, launch_eqwp_stag_step_replay(vin, s6, vout, aslot(sgi, k), h->mat, h->L, n, sp, st));
-        }
-        return B2R_OK;
-    };
-    if ((st = replay((long long)nseg - 1, aux)) != B2R_OK) return st;
-    if (nbuf == 2) CK(h, cudaEventRecord(ax.rep[(nseg - 1) % 2], aux));
-    for (long long sgi = (long long)nseg - 1; sgi >= 0; --sgi) {
+    CK(h, adjoint_inject(tp[1], didx, nrec, d_res + (size_t)(nsteps - 1) * nrec, h->stream));
+    for (long long sgi = slast; sgi >= 0; --sgi) {
         const int n0 = (int)sgi * K;
         const int n1 = std::min(nsteps, n0 + K);
-        if (nbuf == 2) {
-            CK(h, cudaStreamWaitEvent(h->stream, ax.rep[sgi % 2], 0));
-            if (sgi >= 1) {
-                const int b1 = (int)((sgi - 1) % 2);
-                // that buffer last served segment sgi + 1, whose reverse steps are queued
-                if (sgi + 1 < (long long)nseg) CK(h, cudaStreamWaitEvent(aux, ax.rev[b1], 0));
-                if ((st = replay(sgi - 1, aux)) != B2R_OK) return st;
-                CK(h, cudaEventRecord(ax.rep[b1], aux));
-            }
+        if (nbuf == 1 && sgi < kept && (st = replay_again(sgi, h->stream)) != B2R_OK) return st;
+        if (nbuf == 2 && sgi < kept) CK(h, cudaStreamWaitEvent(h->stream, ax.rep[sgi % 2], 0));
+        if (nbuf == 2 && sgi >= 1 && sgi <= kept) {
+            const int b1 = (int)((sgi - 1) % 2);
+            // that buffer last served segment sgi + 1, whose reverse steps are queued
+            CK(h, cudaStreamWaitEvent(ax.s, ax.rev[b1], 0));
+            if ((st = replay_again(sgi - 1, ax.s)) != B2R_OK) return st;
+            CK(h, cudaEventRecord(ax.rep[b1], ax.s));
         }
         for (int n = n1 - 1; n >= n0; --n) {
             const int k = n - n0;
-            CK(h, adjoint_inject(tp[1], didx, nrec, (const float*)d_res.p + (size_t)n * nrec, h->stream));
             const float* vn[3] = {vslot(sgi, k, 0), vslot(sgi, k, 1), vslot(sgi, k, 2)};
             float* const* a = aslot(sgi, k);
             const float* an[3] = {a[0], a[1], a[2]};
-            CK(h, adjoint_step(tp, vn, an, mat, g32.data(), h->L, dt_h, n == 0, h->adj_fused, h->stream));
+            CK(h, adjoint_step(tp, vn, an, mat, g32.data(), h->L, dt_h, n == 0, h->adj_fused, didx, nrec,
+                               n > 0 ? d_res + (size_t)(n - 1) * nrec : nullptr, h->stream));
             // the partial sums into FP64 on a fixed schedule of step numbers
             // (step 0 is the last reverse step, so nothing is left behind)
             if (n % adjoint_fold_steps() == 0) CK(h, adjoint_fold(g32.data(), gp, h->L, h->stream));
         }
         if (nbuf == 2) CK(h, cudaEventRecord(ax.rev[sgi % 2], h->stream));
-        else if (sgi >= 1 && (st = replay(sgi - 1, h->stream)) != B2R_OK) return st;
     }
     // gradients out (interior cells, x fastest), g_rho = -g_b / rho^2
     double* outs[3] = {grad_lambda, grad_mu, grad_rho};
-    const size_t ncell = (size_t)h->cfg.env[0] * h->cfg.env[1] * h->cfg.env[2];
-    DevBuf d_out;
-    CK(h, cudaMalloc(&d_out.p, ncell * sizeof(double)));
     for (int m = 0; m < 3; ++m) {
         if (!outs[m]) continue;
-        CK(h, adjoint_grad_out(gp[m], h->mat[2], m == 2, h->L, (double*)d_out.p, h->stream));
-        CK(h, cudaMemcpyAsync(outs[m], d_out.p, ncell * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        CK(h, adjoint_grad_out(gp[m], h->mat[2], m == 2, h->L, d_out, h->stream));
+        CK(h, cudaMemcpyAsync(outs[m], d_out, ncell * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     }
     CK(h, cudaStreamSynchronize(h->stream));
     h->ts = nsteps;

@@ -84,12 +84,16 @@ cudaError_t launch_eqwp_stag_fused(const StressMaps& maps, const float* const* v
 // adjoint.cu: receiver sampling / injection and one reverse step of the
 // staggered scheme (tmp = vb[3], sb[6], q[6], w[3]; stress order xx, xy, xz,
 // yy, yz, zz; v_n = forward v^n, acc_n = forward stencil sums of step n;
-// last = step 0, whose stress-side half has no earlier step to feed).
-cudaError_t adjoint_sample(const float* vy, const long long* d_idx, int nrec, float* out, cudaStream_t st);
+// last = step 0, whose stress-side half has no earlier step to feed; res_prev =
+// the residuals of step n-1, injected at the receivers rec after step n).
+// adjoint_sample: `steps` fields, `stride` elements apart, nrec samples each.
+cudaError_t adjoint_sample(const float* vy, const long long* d_idx, int nrec, float* out, cudaStream_t st,
+                           int steps = 1, long long stride = 0);
 cudaError_t adjoint_inject(float* vby, const long long* d_idx, int nrec, const float* res, cudaStream_t st);
 cudaError_t adjoint_step(float* const* tmp, const float* const* v_n, const float* const* acc_n,
                          const float* const* mat, float* const* g, const BlockLayout& L, float dt_h,
-                         bool last, bool fused, cudaStream_t st);
+                         bool last, bool fused, const long long* rec, int nrec, const float* res_prev,
+                         cudaStream_t st);
 // g holds FP32 partial sums of the lambda, mu and b gradients; every
 // adjoint_fold_steps() reverse steps (at step numbers that are multiples of
 // it, and at step 0) adjoint_fold adds them into the FP64 gradients g64 and
