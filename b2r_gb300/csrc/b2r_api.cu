@@ -124,12 +124,11 @@ b2r_status build_heat_maps(b2r_handle* h)
 
 // Steps per HBM pass of radius 1 unless a knob says otherwise: three on four
 // rows per thread (heat_rows.cu, whose tiles are 120 x 44 cells), or two in
-// two-row tiles where the blocks are too small to fill those (128^3: 5.2 us
-// per step against 7.0; 64^3: 4.4 against 2.8; four blocks of 24x20x32 cells
-// 6.5 against 4.9).
+// two-row tiles (heat2.cu) where too few of those fill the GPU, by the
+// estimates of a pass of either.
 int heat_own_steps(const b2r_handle* h)
 {
-    if (h->L.B[0] < 96 || h->L.B[1] < 40 || (long long)h->L.B[0] * h->L.B[1] * h->L.B[2] < 1000000) return 2;
+    if (heat2_us(h->L) / 2 <= heat_rows_us(h->L) / 3) return 2;
     // a period of four steps between exchanges is one pass of four, not three
     // and one (512^3 torus in 2x2x2 blocks: 136 us per step, 157 as 3 + 1)
     return (h->L.nblk > 1 || h->L.periodic) && h->cfg.R == 4 ? 4 : 3;

@@ -66,6 +66,9 @@ cudaError_t launch_heat_substep(const CUtensorMap* tin, float* out, const BlockL
 // tensor map must have the box heat2_box_w() x heat2_box_h().
 int heat2_box_w();
 int heat2_box_h();
+// Estimates of one pass: two steps (heat2.cu), three steps (heat_rows.cu).
+double heat2_us(const BlockLayout& L);
+double heat_rows_us(const BlockLayout& L);
 cudaError_t launch_heat_substep2(const CUtensorMap* tin, float* out, const BlockLayout& L, int step_i,
                                  const HeatCoef& c, int* status, cudaStream_t st, int zchunk);
 

@@ -1,5 +1,7 @@
 // heat2.cu -- two heat time steps per HBM pass (temporal blocking), radius 1:
 // the launch of heat2_unit.cuh's units over every tile of every block.
+#include <algorithm>
+
 #include "heat2_unit.cuh"
 
 namespace b2r {
@@ -18,6 +20,7 @@ struct H2Sched {
     long long U;
 };
 
+template <bool ROW>
 __global__ void __launch_bounds__(kT2, 2)
 heat2_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ out, const BlockLayout L,
              const int step_i, const HeatCoef C, const H2Sched sch, int* __restrict__ status)
@@ -56,7 +59,7 @@ heat2_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ out, c
         r /= sch.nty;
         const int zc = (int)(r % sch.nzc);
         const int blk = (int)(r / sch.nzc);
-        if (!h2_unit<kS2, kPlane>(c, &tin, out, L, step_i, blk, tx, ty, zc * sch.Lz, sch.Lz, false)) break;
+        if (!h2_unit<kS2, kPlane, ROW>(c, &tin, out, L, step_i, blk, tx, ty, zc * sch.Lz, sch.Lz, false)) break;
     }
     if (c.aborted && c.tid == 0) {
         report(status, DEV_TIMEOUT);
@@ -65,32 +68,58 @@ heat2_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ out, c
     }
 }
 
+bool h2_whole_rows(const BlockLayout& L)
+{
+    return L.nb[0] == 1 && !L.periodic && L.fixed_edge < 0 && L.B[0] > kOutW && L.B[0] <= kBoxW;
+}
+
+// The launch's tiles, and output planes per unit.  A CTA takes about 1 us to
+// start and 0.52 us per plane (whole rows 0.61), of which it reads four beyond
+// its chunk; two on an SM 0.71 us per plane of both (0.8).  The chunk with the
+// least busy busiest SM, at most 32 planes: us per step at 48x40x32 1.86 in
+// chunks of 1, 2.63 of 4; 64^3 2.37 of 3, 2.63 of 4, 2.51 of 2; 94x200x300 8.0
+// of 15, 9.7 of 8, 11.4 of 24.
+struct H2Plan {
+    int ntx, nty, Lz;
+    double us;
+};
+H2Plan h2_plan(const BlockLayout& L)
+{
+    const bool row = h2_whole_rows(L);
+    const int NZ = L.n[2] - 2, sms = 152;
+    H2Plan p{row ? 1 : h2_ntx(L), h2_nty(L), 1, 1e300};
+    const long long tiles = (long long)p.ntx * p.nty * L.nblk;
+    for (int lz = 1; lz <= 32 && lz <= NZ; ++lz) {
+        const long long q = (tiles * ((NZ + lz - 1) / lz) + sms - 1) / sms;
+        const double us = (q / 2) * (1.0 + (row ? 0.80 : 0.71) * (lz + 4)) + (q % 2) * (0.9 + (row ? 0.61 : 0.52) * (lz + 4));
+        if (us < p.us) {
+            p.us = us;
+            p.Lz = lz;
+        }
+    }
+    return p;
+}
+
 }  // namespace
 
 int heat2_box_w() { return kBoxW; }
 int heat2_box_h() { return kBoxH; }
+double heat2_us(const BlockLayout& L) { return h2_plan(L).us; }
 
 cudaError_t launch_heat_substep2(const CUtensorMap* tin, float* out, const BlockLayout& L, int step_i,
                                  const HeatCoef& c, int* status, cudaStream_t st, int zchunk)
 {
-    static KernelSetup setup;
-    int resident = 0;                          // CTAs resident on the whole GPU
-    if (cudaError_t e = kernel_setup(setup, heat2_kernel, kT2, kSmem2, nullptr, &resident)) return e;
+    static KernelSetup setup[2];
+    const bool row = h2_whole_rows(L);
+    if (cudaError_t e = kernel_setup(setup[row], row ? heat2_kernel<true> : heat2_kernel<false>, kT2, kSmem2, nullptr, nullptr)) return e;
     H2Sched sch;
-    sch.ntx = h2_ntx(L);
-    sch.nty = h2_nty(L);
+    const H2Plan plan = h2_plan(L);
+    sch.ntx = plan.ntx;
+    sch.nty = plan.nty;
     sch.NZ = L.n[2] - 2;
-    const long long tiles = (long long)sch.ntx * sch.nty * L.nblk;
-    int Lz = zchunk > 0 ? zchunk : 16;
-    if (zchunk <= 0 && tiles * ((sch.NZ + 15) / 16) < 2LL * resident) {
-        long long nzc = (2LL * resident + tiles - 1) / tiles;
-        if (nzc > sch.NZ / 4) nzc = sch.NZ / 4 > 0 ? sch.NZ / 4 : 1;
-        Lz = (int)((sch.NZ + nzc - 1) / nzc);
-    }
-    if (Lz > sch.NZ) Lz = sch.NZ;
-    sch.Lz = Lz;
-    sch.nzc = (sch.NZ + Lz - 1) / Lz;
-    sch.U = tiles * sch.nzc;
+    sch.Lz = std::min(zchunk > 0 ? zchunk : plan.Lz, sch.NZ);
+    sch.nzc = (sch.NZ + sch.Lz - 1) / sch.Lz;
+    sch.U = (long long)sch.ntx * sch.nty * L.nblk * sch.nzc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(sch.U < 1 ? 1 : sch.U));
     cfg.blockDim = dim3(kT2);
@@ -101,7 +130,7 @@ cudaError_t launch_heat_substep2(const CUtensorMap* tin, float* out, const Block
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, heat2_kernel, *tin, out, L, step_i, c, sch, status);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, row ? heat2_kernel<true> : heat2_kernel<false>, *tin, out, L, step_i, c, sch, status);
     count_launches(1);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();

@@ -278,10 +278,10 @@ heat_rows_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ ou
 // Output planes per unit: the count of z chunks that leaves the busiest SM
 // the fewest planes, a unit reading T planes beyond its chunk on each side
 // and costing about two more to start.
-int r_chunk(long long tiles, int NZ, int T, int sms)
+int r_chunk(long long tiles, int NZ, int T, int sms, long long& least)
 {
     int best = NZ;
-    long long least = 1ll << 62;
+    least = 1ll << 62;
     for (int n = 1; n <= NZ; ++n) {
         const int lz = (NZ + n - 1) / n;
         if (n > 1 && lz < 4) break;
@@ -295,6 +295,18 @@ int r_chunk(long long tiles, int NZ, int T, int sms)
 }
 
 template <int T, int NW>
+RSched r_sched(const BlockLayout& L, int sms, long long& cost)
+{
+    RSched sch;
+    const int out0 = (L.xoff + 1) & ~3, NZ = L.n[2] - 2;
+    sch.ntx = (L.xoff + L.n[0] - 1 - out0 + kOutW - 1) / kOutW;
+    sch.nty = (L.n[1] - 2 + RCfg<T, NW>::OH - 1) / RCfg<T, NW>::OH;
+    sch.Lz = r_chunk((long long)sch.ntx * sch.nty * L.nblk, NZ, T, sms, cost);
+    sch.nzc = (NZ + sch.Lz - 1) / sch.Lz;
+    return sch;
+}
+
+template <int T, int NW>
 cudaError_t launch_r(const CUtensorMap* tin, float* out, const BlockLayout& L, int step_i, const HeatCoef& c,
                      int* status, cudaStream_t st)
 {
@@ -302,15 +314,9 @@ cudaError_t launch_r(const CUtensorMap* tin, float* out, const BlockLayout& L, i
     static KernelSetup setup;
     int total = 0;      // one CTA per SM
     if (cudaError_t e = kernel_setup(setup, heat_rows_kernel<T, NW>, 32 * NW, Cfg::SMEM, nullptr, &total)) return e;
-    RSched sch;
-    const int out0 = (L.xoff + 1) & ~3;
-    sch.ntx = (L.xoff + L.n[0] - 1 - out0 + kOutW - 1) / kOutW;
-    sch.nty = (L.n[1] - 2 + Cfg::OH - 1) / Cfg::OH;
-    const int NZ = L.n[2] - 2;
-    const long long tiles = (long long)sch.ntx * sch.nty * L.nblk;
-    sch.Lz = r_chunk(tiles, NZ, T, total);
-    sch.nzc = (NZ + sch.Lz - 1) / sch.Lz;
-    return launch_pdl(heat_rows_kernel<T, NW>, (unsigned)(tiles * sch.nzc), 32 * NW, Cfg::SMEM, st, *tin, out, L, step_i,
+    long long cost;
+    const RSched sch = r_sched<T, NW>(L, total, cost);
+    return launch_pdl(heat_rows_kernel<T, NW>, (unsigned)((long long)sch.ntx * sch.nty * L.nblk * sch.nzc), 32 * NW, Cfg::SMEM, st, *tin, out, L, step_i,
                       c, sch, status);
 }
 
@@ -319,6 +325,13 @@ constexpr int kNW2 = 12, kNW3 = 12, kNW4 = 8;   // warps by steps per pass
 }  // namespace
 
 int heat_rows_box_w() { return kBoxW; }
+// three steps per pass: a plane takes a CTA 1.05 to 1.2 us
+double heat_rows_us(const BlockLayout& L)
+{
+    long long cost;
+    r_sched<3, kNW3>(L, 152, cost);
+    return 1.12 * (double)cost;
+}
 int heat_rows_box_h(int T) { return kRY * (T == 2 ? kNW2 : T == 3 ? kNW3 : kNW4) + 2; }
 
 cudaError_t launch_heat_rows(int T, const CUtensorMap* tin, float* out, const BlockLayout& L, int step_i,

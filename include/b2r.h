@@ -141,8 +141,8 @@ enum {
                                   (bit-sliced cells, tblock >= 2) up to four generations per L2
                                   pass, never across a halo exchange; byte cells need >= 4;
                                   1 = one step per pass */
-    B2R_TUNE_ZCHUNK2 = 5,      /* planes per work unit of the several-step heat sweeps (0 = 16
-                                  for two steps, 64 for three or four) */
+    B2R_TUNE_ZCHUNK2 = 5,      /* planes per work unit of the several-step heat sweeps (0 = by the
+                                  size for two steps, 64 for three or four) */
     B2R_TUNE_EQWP_FUSED = 6,   /* staggered elastic wave: 1 = one-pass step, 0 = the velocity
                                   and stress stages as two passes (default); bit-identical */
     B2R_TUNE_GOL_BYTES = 7,    /* Game of Life one-generation kernel: 0 = bit-sliced cells

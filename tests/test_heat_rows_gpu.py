@@ -7,13 +7,15 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-# blocks at the smallest size that takes this path; rows of one tile, one cell
-# more, and ragged float4s at the high face; periods of 2 (two steps per
+# blocks on both sides of the line to two rows per thread; rows of one tile, one
+# cell more, and ragged float4s at the high face; periods of 2 (two steps per
 # pass), 3, 4 (four) and 5 (three and two); tori
 @pytest.mark.parametrize("env,blocks,R,periodic", [
     ((120, 88, 100), (1, 1, 1), 1, False), ((121, 89, 97), (1, 1, 1), 1, False), ((126, 40, 199), (1, 1, 1), 4, False),
     ((246, 91, 93), (2, 1, 1), 2, False), ((97, 268, 202), (1, 2, 2), 3, False), ((242, 104, 167), (2, 1, 1), 4, True),
-    ((122, 133, 64), (1, 1, 1), 5, True)])
+    ((122, 133, 64), (1, 1, 1), 5, True), ((240, 132, 150), (1, 1, 1), 1, False), ((245, 177, 198), (1, 1, 1), 4, False),
+    ((482, 132, 190), (2, 1, 1), 2, False), ((241, 268, 302), (1, 2, 2), 3, False),
+    ((480, 176, 167), (2, 1, 1), 4, True), ((242, 133, 264), (1, 1, 1), 5, True)])
 def test_rows_equal_one_step_per_pass(b2r, env, blocks, R, periodic):
     rng = np.random.default_rng(51)
     shape = env[::-1] if periodic else tuple(e + 2 for e in env[::-1])
