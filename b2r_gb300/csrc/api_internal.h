@@ -40,6 +40,10 @@ struct b2r_handle {
     CUtensorMap tmapf[2][3];    // boxes of heat_far.cu's three tile heights
     HeatCoef hc{};
     HeatTune tune{};
+    // heat: the cluster of heat_small.cu that holds the domain and steps it faster
+    // (0: none), and the us per step that it saves
+    int small_ctas = 0;
+    double small_gain = 0;
     // several blocks, or heat on a torus: the domain as one block, which runs of
     // many steps go to (null: no room, or already one); blocks_of: its owner
     b2r_handle* joined = nullptr;

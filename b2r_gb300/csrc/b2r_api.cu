@@ -457,6 +457,30 @@ b2r_status advance(b2r_handle* h, int n)
     return B2R_OK;
 }
 
+// Whether a cluster's shared memory holds the heat domain and steps it faster
+// than launches do: by the estimate of a pass of two (radius 1), of a launch per
+// step (radius 2: 3.1 us at least), on a torus with an exchange every third.
+void make_small(b2r_handle* h)
+{
+    const b2r_config& c = h->cfg;
+    const int ctas = heat_small_ctas(c.env, c.D);
+    if (!ctas) return;
+    BlockLayout one;
+    const int H = (h->L.periodic ? 3 : 1) * c.D, nb[3] = {1, 1, 1};
+    const int n[3] = {c.env[0] + 2 * H, c.env[1] + 2 * H, c.env[2] + 2 * H};
+    fill_layout(one, n, c.env, nb, H, 4, h->L.periodic, -1);
+    const double other = (c.D == 1 ? heat2_us(one) / 2 : 3.1) + (h->L.periodic ? 1.2 : 0.0);
+    h->small_gain = other - heat_small_us(c.env, c.D, ctas);
+    if (h->small_gain > 0) h->small_ctas = ctas;
+}
+
+// Reading the domain and writing it back takes about 8 us, less than the
+// exchanges and ragged sweeps of several blocks or a torus save.
+bool small_runs(const b2r_handle* h, int n)
+{
+    return h->small_ctas && h->tune.own && n >= 4 && (h->L.nblk > 1 || h->L.periodic || n * h->small_gain > 8.0);
+}
+
 // The one-block form of a domain of several blocks, or of a heat domain on a
 // torus.  A shelled domain then needs no exchange at all; a torus keeps one,
 // every three steps (a deeper halo computes more cells than the exchanges it
@@ -727,7 +751,8 @@ b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined)
                 g_err = h->err;
                 return bail(st);
             }
-            if (!joined && (h->L.nblk > 1 || h->L.periodic)) make_joined(h);
+            if (!joined) make_small(h);
+            if (!joined && !h->small_ctas && (h->L.nblk > 1 || h->L.periodic)) make_joined(h);
         }
     } else {
         h->nfld = (c.model == B2R_MODEL_EQWP_REF) ? 10 : 9;
@@ -966,6 +991,15 @@ b2r_status b2r_step(b2r_handle* h, int nsteps)
         h->upmask = 0;
         h->halos_fresh = false;
         h->halos_lost = true;   // the interiors are current, the halos between blocks are not
+        return B2R_OK;
+    }
+    if (small_runs(h, nsteps)) {
+        CK(h, launch_heat_small(static_cast<float*>(h->buf[h->cur]), h->L, h->cfg.env, h->cfg.D, h->small_ctas, h->hc,
+                                nsteps, h->d_status, h->stream));
+        h->ts += nsteps;
+        h->upmask = 0;
+        h->halos_fresh = false;
+        h->halos_lost = h->L.nblk > 1 || h->L.periodic;   // the interiors are current, the halos are not
         return B2R_OK;
     }
     if (joins(h, nsteps)) return step_joined(h, nsteps);

@@ -66,6 +66,13 @@ cudaError_t launch_heat_substep(const CUtensorMap* tin, float* out, const BlockL
 // tensor map must have the box heat2_box_w() x heat2_box_h().
 int heat2_box_w();
 int heat2_box_h();
+// heat_small.cu: CTAs of the cluster whose shared memory holds the domain of e
+// cells, 0 if none does; nsteps steps of the interiors of buf's blocks (the
+// halos between blocks are left behind).
+int heat_small_ctas(const int e[3], int D);
+double heat_small_us(const int e[3], int D, int ctas);   // a step's estimate
+cudaError_t launch_heat_small(float* buf, const BlockLayout& M, const int e[3], int D, int ctas, const HeatCoef& c,
+                              int nsteps, int* status, cudaStream_t st);
 // Estimates of one pass: two steps (heat2.cu), three steps (heat_rows.cu).
 double heat2_us(const BlockLayout& L);
 double heat_rows_us(const BlockLayout& L);

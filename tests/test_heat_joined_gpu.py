@@ -12,7 +12,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("env,blocks,R,D,periodic", [
     ((48, 40, 32), (2, 2, 1), 2, 1, False), ((39, 34, 27), (3, 1, 3), 1, 2, False), ((66, 30, 46), (2, 3, 1), 1, 4, False),
     ((37, 31, 29), (1, 1, 1), 1, 1, True), ((50, 22, 26), (2, 1, 1), 2, 2, True), ((35, 16, 17), (1, 1, 1), 1, 4, True),
-    ((33, 8, 90), (1, 1, 2), 1, 3, True), ((244, 104, 168), (2, 2, 2), 4, 1, False)])
+    ((33, 8, 90), (1, 1, 2), 1, 3, True), ((244, 104, 168), (2, 2, 2), 4, 1, False),
+    ((130, 63, 70), (2, 3, 1), 1, 1, False), ((100, 62, 81), (1, 2, 3), 2, 2, False), ((90, 75, 64), (2, 1, 1), 2, 1, True),
+    ((77, 83, 65), (1, 1, 1), 1, 2, True)])
 def test_joined_equals_blocks(b2r, env, blocks, R, D, periodic):
     import torch
     rng = np.random.default_rng(71)
