@@ -308,7 +308,6 @@ __device__ __noinline__ uint4 run_two_step(const BatchArgs& a, int k, int t, int
     c.ring = ring;
     c.s1 = s1;
     c.bar = reinterpret_cast<uint64_t*>(ring + kS * kSlot);
-    c.abort_flag = reinterpret_cast<int*>(c.bar + kS);
     c.tid = threadIdx.x;
     c.lane = threadIdx.x & 31;
     c.warp = threadIdx.x >> 5;

@@ -31,7 +31,6 @@ heat2_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ out, c
     c.ring = ring;
     c.s1 = ring + kS2 * kPlane;                          // 2 stage-1 planes
     c.bar = reinterpret_cast<uint64_t*>(c.s1 + 2 * kP1);
-    c.abort_flag = reinterpret_cast<int*>(c.bar + kS2);
     c.tid = threadIdx.x;
     c.lane = c.tid & 31;
     c.warp = c.tid >> 5;
@@ -40,7 +39,6 @@ heat2_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ out, c
     c.plane = L.plane;
     c.P = L.P;
     if (c.tid == 0) {
-        *c.abort_flag = 0;
         for (int s = 0; s < kS2; ++s) mbar_init(&c.bar[s], 1);
         fence_mbar_init();
     }
@@ -77,8 +75,10 @@ bool h2_whole_rows(const BlockLayout& L)
 // start and 0.52 us per plane (whole rows 0.61), of which it reads four beyond
 // its chunk; two on an SM 0.71 us per plane of both (0.8).  The chunk with the
 // least busy busiest SM, at most 32 planes: us per step at 48x40x32 1.86 in
-// chunks of 1, 2.63 of 4; 64^3 2.37 of 3, 2.63 of 4, 2.51 of 2; 94x200x300 8.0
-// of 15, 9.7 of 8, 11.4 of 24.
+// chunks of 1, 2.63 of 4; 64^3 2.32 of 3, 2.57 of 4, 2.45 of 2; 94x200x300 7.9
+// of 16, 9.4 of 8.  The 0.52 us are neither the ring's depth (eight slots
+// instead of four: the same) nor too few warps (16 of one row each: the same
+// alone, slower two on an SM) nor the refill (a producer warp: 0.59).
 struct H2Plan {
     int ntx, nty, Lz;
     double us;

@@ -25,8 +25,8 @@
 // so one tile column does instead of two of which the second is nearly empty:
 // lane 0's left and lane 31's right neighbour are shell cells, the same in both
 // stages, which these lanes read from the field (in the output buffer, whose
-// shell holds the same and is not written).  128^3: 4.1 us per step against
-// 5.1; a plane costs 0.61 us instead of 0.52.
+// shell holds the same and is not written).  128^3: 3.85 us per step against
+// 4.95; a plane costs 0.6 us instead of 0.52.
 // A unit in single-step mode stores the stage-1 values of its output tile
 // and skips stage 2 (the last step of a run with an odd step count).
 #pragma once
@@ -61,11 +61,11 @@ struct H2Ctx {
     const float* ring;
     float* s1;
     uint64_t* bar;
-    int* abort_flag;
-    float* outb;                 // out + block + lane's storage x
+    float* dst;                  // the thread's first cell in plane p-2 of the output
     const CUtensorMap* tmap;
     HeatCoef C;
-    long long plane, P;
+    long long plane;
+    int P;
     unsigned gp;
     int np, first, zs, ze, xs0, y0, blk, ya, warp, lane, tid;
     int lo1z, hi1z, lo2z, hi2z, nz;
@@ -98,7 +98,7 @@ __device__ __forceinline__ void h2_iter(H2Ctx& c, int pr)
 {
     constexpr int CZ = (PH + 2) % 3, MZ = (PH + 1) % 3, NZ = PH;
     const unsigned g = c.gp + pr;
-    if (!mbar_wait_bounded(&c.bar[g % S], (g / S) & 1)) *c.abort_flag = 1;
+    const bool bad = !mbar_wait_bounded(&c.bar[g % S], (g / S) & 1);
     const float* pl = c.ring + (g % S) * SLOT;
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr)
@@ -142,7 +142,7 @@ __device__ __forceinline__ void h2_iter(H2Ctx& c, int pr)
                 res = ce;
             }
             if (st1 && c.in1y[rr])
-                h2_store(c.outb + (long long)z1 * c.plane + (long long)(c.ya + rr) * c.P, res, c.st1_all, c.in1x);
+                h2_store(c.dst + c.plane + rr * c.P, res, c.st1_all, c.in1x);
             *reinterpret_cast<float4*>(s1p + (2 * c.warp + rr) * kBoxW + 4 * c.lane) = res;
             c.q1[rr][NZ] = res;
         }
@@ -168,11 +168,11 @@ __device__ __forceinline__ void h2_iter(H2Ctx& c, int pr)
             const float4 yp = rr == 0 ? c.q1[1][CZ] : dn;
             const float4 v = heat_upd4(c.C, ce, l, rt, ym, yp, c.q1[rr][MZ], c.q1[rr][NZ]);
             if (zin && c.in2y[rr] && c.st_any)
-                h2_store(c.outb + (long long)z2 * c.plane + (long long)(c.ya + rr) * c.P, v, c.st_all, c.in2x);
+                h2_store(c.dst + rr * c.P, v, c.st_all, c.in2x);
         }
     }
-    __syncthreads();
-    if (*c.abort_flag) {
+    c.dst += c.plane;
+    if (__syncthreads_or(bad)) {
         c.aborted = true;
         c.stop = g;
         return;
@@ -203,7 +203,7 @@ __host__ __device__ inline int h2_nty(const BlockLayout& L) { return (L.n[1] - 2
 
 // One unit: tile (tx, ty) of block blk, output planes [1 + zi0, zi0 + Lz]
 // clipped to the window, sub-steps step_i and step_i + 1 (single: step_i
-// only).  c.ring/s1/bar/abort_flag/tid/lane/warp/C/plane/P and the ring
+// only).  c.ring/s1/bar/tid/lane/warp/C/plane/P and the ring
 // position must be set.  Returns false if a bounded wait gave up (c.stop
 // holds where).
 template <int S, int SLOT, bool ROW = false>
@@ -274,7 +274,8 @@ __device__ __forceinline__ bool h2_unit(H2Ctx& c, const CUtensorMap* tmap, float
     c.st_any = c.in2x[0] || c.in2x[1] || c.in2x[2] || c.in2x[3];
     c.st1_all = c.in1x[0] && c.in1x[1] && c.in1x[2] && c.in1x[3];
     c.st1_any = c.in1x[0] || c.in1x[1] || c.in1x[2] || c.in1x[3];
-    c.outb = out + (long long)blk * L.bstride + c.xs0 + 4 * c.lane;
+    c.dst = out + (long long)blk * L.bstride + (long long)(c.first - 2) * L.plane + (long long)c.ya * L.P + c.xs0 +
+            4 * c.lane;
 
     if (ROW) {
         c.nz = L.n[2];
@@ -282,7 +283,7 @@ __device__ __forceinline__ bool h2_unit(H2Ctx& c, const CUtensorMap* tmap, float
         for (int rr = 0; rr < 2; ++rr) {
             const int y = c.ya + rr;
             const bool has = (c.lane == 0 || c.lane == 31) && y >= 0 && y < L.n[1];
-            c.ep[rr] = has ? c.outb + (long long)c.first * c.plane + (long long)y * c.P + (c.lane == 0 ? -1 : 4) : nullptr;
+            c.ep[rr] = has ? c.dst + 2 * c.plane + rr * c.P + (c.lane == 0 ? -1 : 4) : nullptr;
         }
     }
     for (int pr = 0; pr < c.np;) {
