@@ -132,7 +132,11 @@ __device__ __forceinline__ bool f_iter(FCtx<D, S, SLOT, BWC>& c, const Coef& C, 
         }
         c.dst += c.plane;
     }
-    if (pr >= D) {              // plane pr - D is read: its slot may be refilled
+    if (pr >= D) {
+        // plane pr - D is read: its slot may be refilled.  What the stores above were
+        // made of has been loaded; while nothing is stored yet, a load that has only
+        // been issued could still be under way when the barrier counts the arrival.
+        if (pr < 2 * D) __threadfence_block();
         __syncwarp();
         if (c.lane0) mbar_arrive(&c.empty[cslot]);
     }
