@@ -68,6 +68,7 @@ struct b2r_handle {
     bool xdone = false;        // the last sub-step issued the next period's exchange
     cudaStream_t xs = nullptr;
     cudaEvent_t xev[2] = {};   // [band tiles done, exchange done]
+    std::map<std::pair<bool, int>, EqwpRefMaps> rmaps;   // collocated model: by stage and tile width
     std::map<int, EqwpStressMaps> emaps;   // its tensor maps per tile width (threads per row), built
     const void* emaps_of[11] = {};         // for the field pointers in emaps_of
     bool gol_bytes = false;    // Game of Life: byte-SWAR kernel instead of bit-sliced cells

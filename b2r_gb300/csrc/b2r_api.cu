@@ -269,6 +269,42 @@ EqwpStagParams stag_params(const b2r_handle* h)
     return p;
 }
 
+// The collocated model's stages stream their inputs through TMA rings from a
+// size on: us per step plain and streamed, 64^3 10.1 and 19.2, 100x70x64 17.9 and
+// 20.9, 96^3 21.0 and 21.0, 128x128x64 26.6 and 21.4, 110^3 45.9 and 29.7, 256^3
+// 410 and 334, 512x256x512 1474 and 1256.
+bool streams_ref(const b2r_handle* h)
+{
+    return (long long)h->L.B[0] * h->L.B[1] * h->L.B[2] * h->L.nblk >= 900000;
+}
+
+// The collocated model's tensor maps of one stage and tile width, built on first
+// use (its fields stay where they are).
+b2r_status ref_maps(b2r_handle* h, int i, bool velocity, const EqwpRefMaps*& got)
+{
+    int tx = 0, ty = 0;
+    eqwp_ref_tma_shape(h->L, i, velocity, &tx, &ty);
+    auto it = h->rmaps.find({velocity, tx});
+    if (it == h->rmaps.end()) {
+        static const int kV[2][3] = {{B2R_F_VX, B2R_F_VY, B2R_F_VZ}, {B2R_F_SXZ, B2R_F_SYZ, B2R_F_SZZ}};
+        static const int kH[3] = {B2R_F_SXX, B2R_F_SXY, B2R_F_SYY};
+        static const int kO[2][6] = {{B2R_F_SXX, B2R_F_SYY, B2R_F_SZZ, B2R_F_SXY, B2R_F_SXZ, B2R_F_SYZ},
+                                     {B2R_F_VX, B2R_F_VY, B2R_F_VZ, B2R_F_DISP, -1, -1}};
+        EqwpRefMaps m{};
+        bool ok = true;
+        auto make = [&](CUtensorMap& t, int f, bool wide) {
+            if (f >= 0) ok = ok && make_block_tmap(&t, h->fld[f], h->L, 4, wide ? 4 * tx + 8 : 4 * tx, wide ? ty + 4 : ty, 1);
+        };
+        for (int k = 0; k < 3; ++k) make(m.v[k], kV[velocity][k], true);
+        for (int k = 0; k < 3 && velocity; ++k) make(m.h[k], kH[k], true);
+        for (int k = 0; k < 6; ++k) make(m.o[k], kO[velocity][k], false);
+        if (!ok) return fail(h, B2R_ERR_CUDA, "cuTensorMapEncodeTiled failed for the elastic-wave fields");
+        it = h->rmaps.emplace(std::make_pair(velocity, tx), m).first;
+    }
+    got = &it->second;
+    return B2R_OK;
+}
+
 b2r_status substep(b2r_handle* h, int i, bool xnext)
 {
     h->upmask = 0;
@@ -297,6 +333,14 @@ b2r_status substep(b2r_handle* h, int i, bool xnext)
         const int ts = (int)(h->ts - (h->blocks_of ? h->ts % o->cfg.R : i));
         EqwpRefParams p = eqwp_ref_params(o->L);
         for (int a = 0; a < 3; ++a) p.every[a] = h->blocks_of ? o->L.B[a] : 1 << 30;
+        if (streams_ref(h)) {
+            for (int vel = 0; vel < 2; ++vel) {
+                const EqwpRefMaps* m = nullptr;
+                if (b2r_status st = ref_maps(h, i, vel != 0, m); st != B2R_OK) return st;
+                CK(h, launch_eqwp_ref_tma(*m, vel != 0, h->fld, h->L, i, ts, p, h->d_status, h->stream));
+            }
+            return B2R_OK;
+        }
         CK(h, launch_eqwp_ref_substep(h->fld, h->L, i, ts, p, h->stream));
         return B2R_OK;
     }

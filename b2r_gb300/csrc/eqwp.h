@@ -43,6 +43,17 @@ cudaError_t launch_eqwp_stag_step_replay(const float* const* v_in, float* const*
                                          float* const* acc, float* const* mat, const BlockLayout& L,
                                          int ts, const EqwpStagParams& p, cudaStream_t st);
 
+// eqwp_ref_tma.cu: the collocated model's stages on TMA rings; maps.v and maps.h
+// have boxes of (4 tx + 8) x (ty + 4) cells, maps.o of 4 tx x ty, tx and ty by
+// eqwp_ref_tma_shape.  Stress stage: v = vx, vy, vz; o = sxx, syy, szz, sxy, sxz,
+// syz.  Velocity stage: v = sxz, syz, szz; h = sxx, sxy, syy; o = vx, vy, vz, disp.
+struct EqwpRefMaps {
+    CUtensorMap v[3], h[3], o[6];
+};
+void eqwp_ref_tma_shape(const BlockLayout& L, int step_i, bool velocity, int* tx, int* ty);
+cudaError_t launch_eqwp_ref_tma(const EqwpRefMaps& maps, bool velocity, float* const* fld, const BlockLayout& L,
+                                int step_i, int ts, const EqwpRefParams& p, int* status, cudaStream_t st);
+
 // eqwp_tma.cu: the staggered stress stage with its inputs streamed through
 // TMA rings, on the plain stage launch's tiles: eqwp_stress_tma_shape gives
 // the CTA shape tx x ty of sub-step step_i; maps.v: vx, vy, vz with boxes of
