@@ -560,7 +560,6 @@ void make_joined(b2r_handle* h)
         return;
     }
     h->joined->blocks_of = h;
-    cudaFree(h->joined->d_status);
     h->joined->d_status = h->d_status;
 }
 
@@ -769,9 +768,11 @@ b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined)
         cudaGetLastError();   // a failed allocation must not surface in the caller's next launch check
         return s;
     };
-    if (cudaMalloc(&h->d_status, sizeof(int)) != cudaSuccess)
-        return bail(fail(nullptr, B2R_ERR_CUDA, "cudaMalloc(status) failed"));
-    cudaMemset(h->d_status, 0, sizeof(int));
+    if (!joined) {                       // a one-block form reports to its owner's
+        if (cudaMalloc(&h->d_status, sizeof(int)) != cudaSuccess)
+            return bail(fail(nullptr, B2R_ERR_CUDA, "cudaMalloc(status) failed"));
+        cudaMemset(h->d_status, 0, sizeof(int));
+    }
     const size_t fb = field_bytes(h);
     if (c.model == B2R_MODEL_HEAT || c.model == B2R_MODEL_GOL) {
         for (int b = 0; b < 2; ++b) {
@@ -824,7 +825,7 @@ b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined)
         }
         if (!joined && h->L.nblk > 1 && !h->L.periodic) make_joined(h);
     }
-    if (cudaDeviceSynchronize() != cudaSuccess)
+    if (!joined && cudaDeviceSynchronize() != cudaSuccess)
         return bail(fail(nullptr, B2R_ERR_CUDA, "device initialisation failed"));
     *out = h;
     return B2R_OK;
