@@ -194,6 +194,7 @@ int gol_pass_gens(const b2r_handle* h, int i, int left);
 b2r_status check_status(b2r_handle* h);
 b2r_status exchange_all(b2r_handle* h, bool staged, cudaStream_t xst = nullptr);   // xst: another stream than the handle's
 b2r_status exchange_one(b2r_handle* h, int field, bool staged);
+b2r_status ensure_halos(b2r_handle* h);
 EqwpStagParams stag_params(const b2r_handle* h);
 // One sub-step i of a period.  xnext: the caller starts the next period
 // without an exchange if h->xdone is set afterwards (the sub-step may then

@@ -257,6 +257,17 @@ b2r_status exchange_one(b2r_handle* h, int field, bool staged)
     return B2R_OK;
 }
 
+// The blocks' halos from their owners, where a run that needs none left them
+// behind: before anything but a step looks at whole blocks.
+b2r_status ensure_halos(b2r_handle* h)
+{
+    if (!h->halos_lost) return B2R_OK;
+    if (b2r_status st = exchange_all(h, false); st != B2R_OK) return st;
+    h->halos_lost = false;
+    h->halos_fresh = h->ts % h->cfg.R == 0;
+    return B2R_OK;
+}
+
 EqwpStagParams stag_params(const b2r_handle* h)
 {
     const std::vector<float>& src = h->blocks_of ? h->blocks_of->src : h->src;
@@ -1011,6 +1022,7 @@ b2r_status b2r_download_blocks(b2r_handle* h, int field, void* dst, int dst_is_d
     const bool is_mat = eq && field >= B2R_F_LAMBDA && field <= B2R_F_BUOY && h->mat[0];
     if (!is_mat && (field < 0 || field >= (eq ? h->nfld : 1)))
         return fail(h, B2R_ERR_ARG, "invalid field id %d", field);
+    if (b2r_status st = ensure_halos(h); st != B2R_OK) return st;
     const char* srcb = static_cast<const char*>(
         is_mat ? (const void*)h->mat[field - B2R_F_LAMBDA]
                : (eq ? (const void*)h->fld[field] : h->buf[h->cur]));
@@ -1401,6 +1413,7 @@ b2r_status b2r_write_block_data(b2r_handle* h, int field, int block, int time_st
         src = h->mat[field - B2R_F_LAMBDA];
     }
     if (!src) return fail(h, B2R_ERR_ARG, "field %d has no data on this handle", field);
+    if (b2r_status st = ensure_halos(h); st != B2R_OK) return st;
     const BlockLayout& L = h->L;
     std::string path = dir && dir[0] ? std::string(dir) + "/" : std::string();
     path += name;
@@ -1438,6 +1451,7 @@ b2r_status b2r_eqwp_gpu_main(b2r_handle* h, int ts, int R, double* gpu_seconds)
     if (h->cfg.model != B2R_MODEL_EQWP_REF)
         return fail(h, B2R_ERR_ARG, "eqwp_gpu_main needs a B2R_MODEL_EQWP_REF handle");
     if (R < 1 || R > h->cfg.R) return fail(h, B2R_ERR_ARG, "R must be in 1..%d", h->cfg.R);
+    if (b2r_status st = ensure_halos(h); st != B2R_OK) return st;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);

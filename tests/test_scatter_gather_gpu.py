@@ -46,3 +46,31 @@ def test_every_cell(b2r, env, blocks, R, periodic, gol):
             d.download(out[start:start + dom.size].view(shape))
             assert np.array_equal(out[start:start + dom.size].view(shape).cpu().numpy(), dom)
             assert (out[:start] == 7).all() and (out[start + dom.size:] == 7).all()
+
+
+@pytest.mark.parametrize("model,env,blocks,R,periodic", [
+    ("HEAT", (40, 33, 32), (2, 1, 2), 2, True), ("HEAT", (130, 63, 70), (2, 3, 1), 1, False),
+    ("GOL", (36, 30, 24), (2, 2, 2), 3, True), ("EQWP_STAG", (48, 40, 32), (2, 1, 2), 2, False)])
+def test_whole_blocks_after_long_runs(b2r, model, env, blocks, R, periodic):
+    """Runs that leave the halos between blocks behind: blocks read whole afterwards
+    hold their neighbours' current cells, and the next steps are none the worse."""
+    rng = np.random.default_rng(9)
+    wave = model == "EQWP_STAG"
+    H, shell = R * (4 if wave else 1), 0 if periodic else (2 if wave else 1)
+    shape = tuple(e + 2 * shell for e in env[::-1])
+    dom = rng.integers(0, 2, shape).astype(np.uint8) if model == "GOL" else rng.random(shape, dtype=np.float32)
+    bc = b2r.BC_PERIODIC if periodic else b2r.BC_SHELL
+    ends = []
+    for look in (True, False):
+        with b2r.Domain(getattr(b2r, "MODEL_" + model), env, blocks=blocks, R=R, D=2 if wave else 1, boundary=bc,
+                        **(dict(dt=2e-4, h=1.0, src=(3, 4, 5)) if wave else {})) as d:
+            for f in (*range(9), "lambda", "mu", "buoy") if wave else (0,):
+                d.upload(dom, field=f)
+            d.step(25)
+            if look:
+                want = padded(d.download(), env, blocks, H, shell, periodic)
+                for key, got in d.download_blocks().items():
+                    assert np.array_equal(got, want[key]), key
+            d.step(3)
+            ends.append(d.download())
+    assert np.array_equal(*ends)
