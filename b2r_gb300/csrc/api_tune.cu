@@ -154,7 +154,9 @@ static b2r_status autotune_knobs(b2r_handle* h, int trial_steps, int best[3], do
     // trials run as the stepping will (graph replay included, each
     // candidate's graphs captured in its warm run) and over whole periods:
     // a single period would not show what a choice costs at period ends
-    const int trial = h->cfg.model == B2R_MODEL_GOL ? std::max(trial_steps, 16 * h->cfg.R) : trial_steps;
+    // or, where long runs go to the one-block form, one long enough for that
+    const int trial = h->cfg.model == B2R_MODEL_GOL ? std::max(trial_steps, 16 * h->cfg.R)
+                                                    : std::max(trial_steps, h->joined ? 24 : 1);
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -265,6 +267,8 @@ b2r_status b2r_autotune(b2r_handle* h, int trial_steps, int best[3], double* bes
         for (int z2 : {0, 32, 64, 96, 128}) cands.push_back({2, z2, 0, 0, 1, 0, 0, 1});
         trial_steps = (trial_steps + 1) / 2 * 2;
     }
+    // the library's own rule takes long runs elsewhere than into the blocks
+    if (h->joined || h->small_ctas) trial_steps = std::max(trial_steps, 24);
     for (int pdl = 0; pdl < 2; ++pdl)
         for (int zc : zchunks)
             for (int cp : persist)
@@ -280,7 +284,7 @@ b2r_status b2r_autotune(b2r_handle* h, int trial_steps, int best[3], double* bes
         h->tune.zchunk = cd.zc;
         h->tune.ctas_per_sm = cd.cp;
         h->tune.pdl = cd.pdl;
-        if ((st = b2r_step(h, 1)) != B2R_OK) break;       // warm
+        if ((st = b2r_step(h, cd.tb == 0 ? trial_steps : 1)) != B2R_OK) break;   // warm
         cudaEventRecord(e0, h->stream);
         if ((st = b2r_step(h, trial_steps)) != B2R_OK) break;
         cudaEventRecord(e1, h->stream);

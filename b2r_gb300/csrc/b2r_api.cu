@@ -589,9 +589,9 @@ bool force_is_inside(const b2r_handle* h)
 
 // Whether a run of n steps goes to the one-block form.  Joining and splitting
 // cost about as much as eight exchanges and ragged block sweeps of heat: us for
-// 8 and 48 steps in blocks and joined, 48x40x32 in 2x2x1 51, 236 and 40, 146;
-// 512^3 in 2x2x2, R = 2, 1030, 6305 and 1125, 4279; the torus above 212, 1242
-// and 162, 725; a torus of radius 4, 100^3 in 1x2x1, 76, 388 and 85, 366.
+// 8 and 48 steps in blocks and joined, 512^3 in 2x2x2, R = 2, 1030, 6305 and
+// 1125, 4279; the torus above 212, 1242 and 162, 725; a torus of radius 4, 100^3
+// in 1x2x1, 76, 388 and 85, 366.
 // The elastic wave pays about 1.4 steps for it; us per step in blocks and joined:
 // 512x512x256 in 2x2x1, R = 2, 1547 and 1334 (even at 9 steps), 256^3 in 2x1x1,
 // R = 1, 485 and 355 (5), 128^3 in 2x2x2 90 and 51 (4), 64^3 in 2x1x1 18.8 and
