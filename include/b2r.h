@@ -116,7 +116,8 @@ b2r_status b2r_download(b2r_handle* h, int field, void* dst, int dst_is_device);
 
 /* Copy every padded block of a field, halos included, into a dense array of
  * blocks*Ngz*Ngy*Ngx cells (block index slowest, x fastest) -- the per-rank
- * blocks of the reference (B2R_BLOCK_SIZE_*, b2r.h:81-85) side by side. */
+ * blocks of the reference (B2R_BLOCK_SIZE_*, b2r.h:81-85) side by side.  After
+ * a run that went through no halos (see TBLOCK) they are brought up to date first. */
 b2r_status b2r_download_blocks(b2r_handle* h, int field, void* dst, int dst_is_device);
 
 /* ---- time stepping ------------------------------------------------------ */
@@ -136,11 +137,14 @@ enum {
     B2R_TUNE_CTAS_PER_SM = 2,  /* 0 = one CTA per unit, k = persistent k CTAs per SM */
     B2R_TUNE_PDL = 3,          /* programmatic dependent launch on / off */
     B2R_TUNE_TBLOCK = 4,       /* time steps per pass: heat of radius 1 takes up to tblock (2, 3
-                                  or 4; default 2, or three on large blocks until this or another
-                                  knob of the several-step sweeps is set) steps per HBM pass and Game of Life
-                                  (bit-sliced cells, tblock >= 2) up to four generations per L2
-                                  pass, never across a halo exchange; byte cells need >= 4;
-                                  1 = one step per pass */
+                                  or 4; default 2) steps per HBM pass.  Until a heat knob is set
+                                  the library chooses: two or three steps by the block size, long
+                                  runs on several blocks as one block, small domains in one
+                                  cluster's shared memory.  Game of Life (bit-sliced cells, tblock
+                                  >= 2): several generations per pass, on the whole domain's bit
+                                  grid unless GOL_PUSH or GOL_ROWS is set (then up to four, never
+                                  across a halo exchange); byte cells need >= 4; 1 = one step per
+                                  pass */
     B2R_TUNE_ZCHUNK2 = 5,      /* planes per work unit of the several-step heat sweeps (0 = by the
                                   size for two steps, 64 for three or four) */
     B2R_TUNE_EQWP_FUSED = 6,   /* staggered elastic wave: 1 = one-pass step, 0 = the velocity
