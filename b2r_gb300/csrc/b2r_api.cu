@@ -538,11 +538,11 @@ bool small_runs(const b2r_handle* h, int n)
 
 // The one-block form of a domain of several blocks, or of a heat domain on a
 // torus.  A shelled domain then needs no exchange at all; a torus keeps one,
-// every three steps (a deeper halo computes more cells than the exchanges it
-// saves cost; radius 3 and 4, whose steps are longer than an exchange is, every
-// four).  48 heat steps with 3 / 4 / 6 / 8 steps between exchanges:
-// 250x186x132, radius 2, 725 / 863 / 833 / 965 us, 256^3, radius 1, 887 / 1000 /
-// 1020 / 1068; 64x66x70, radius 3, 311 / 271 / 293 / 294.  Made where what it
+// every three steps, with radius 3 and 4 every two (a deeper halo computes more
+// cells than the exchanges it saves cost).  48 heat steps with 1 / 2 / 3 / 4 steps
+// between exchanges: 250x186x132, radius 2, 819 / 671 / 670 / 702 us, 128^3 495 /
+// 434 / 422 / 439; radius 1, 256^3 1661 / 1065 / 885 / 1003; radius 3, 128^3 536 /
+// 503 / 529 / 525; radius 4, 250x100x100 650 / 587 / 639 / 660.  Made where what it
 // allocates takes at most an eighth of the free memory: two buffers for heat,
 // ten fields for the collocated wave, the material for the staggered one, whose
 // fields lie in the second field set.
@@ -552,7 +552,7 @@ void make_joined(b2r_handle* h)
     b2r_config c = h->cfg;
     for (int a = 0; a < 3; ++a) c.blocks[a] = 1;
     const int least = std::min(c.env[0], std::min(c.env[1], c.env[2]));
-    c.R = h->L.periodic ? std::max(1, std::min(c.D <= 2 ? 3 : 4, least / 2 / c.D)) : 1;
+    c.R = h->L.periodic ? std::max(1, std::min(c.D <= 2 ? 3 : 2, least / 2 / c.D)) : 1;
     if (h->L.nblk == 1 && c.R <= h->cfg.R) return;
     const int nf = c.model == B2R_MODEL_HEAT ? 2 : c.model == B2R_MODEL_EQWP_REF ? 10 : 3;
     const int H = c.R * halo_per_step(c);
