@@ -23,6 +23,7 @@
 // p-s-1, p-s, p-s+1, which the thread holds in registers (the newest made in
 // this iteration); the edge rows of plane p-s were exchanged one iteration
 // earlier, so one barrier per plane orders everything.
+#include <algorithm>
 #include <climits>
 
 #include "b2r_common.cuh"
@@ -49,6 +50,7 @@ struct RCfg {
 
 struct RSched {
     int ntx, nty, nzc, Lz;
+    int x0, y0, z0;     // storage x, row and plane of the first stored cells: the windows' first
 };
 
 __device__ __forceinline__ float4 rld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -206,10 +208,10 @@ heat_rows_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ ou
     int lo[3], hi[3];                               // window of the last stage: the stored cells
 #pragma unroll
     for (int a = 0; a < 3; ++a) stage_region(L, edge, a, step_i + T, lo[a], hi[a]);
-    c.X0 = ((L.xoff + 1) & ~3) - 4 + tx * kOutW;    // storage x of the first computed cell
-    c.Y0 = 1 + ty * Cfg::OH - (T - 1);              // block y of computed row 0
-    c.zs = max(1 + zc * sch.Lz, lo[2]);
-    c.ze = min((zc + 1) * sch.Lz, hi[2]);           // output planes [zs, ze]
+    c.X0 = sch.x0 - 4 + tx * kOutW;                 // storage x of the first computed cell
+    c.Y0 = sch.y0 + ty * Cfg::OH - (T - 1);         // block y of computed row 0
+    c.zs = max(sch.z0 + zc * sch.Lz, lo[2]);
+    c.ze = min(sch.z0 + (zc + 1) * sch.Lz - 1, hi[2]);   // output planes [zs, ze]
     if (c.zs > c.ze) return;
     const int ox0 = c.X0 + 4 - L.xoff, oy0 = c.Y0 + T - 1;   // first stored cell (block x, y)
     if (ox0 > hi[0] || ox0 + kOutW - 1 < lo[0] || oy0 > hi[1] || oy0 + Cfg::OH - 1 < lo[1]) return;
@@ -295,12 +297,24 @@ int r_chunk(long long tiles, int NZ, int T, int sms, long long& least)
 }
 
 template <int T, int NW>
-RSched r_sched(const BlockLayout& L, int sms, long long& cost)
+RSched r_sched(const BlockLayout& L, int step_i, int sms, long long& cost)
 {
+    // tiles over the union of the blocks' windows after the pass
+    int lo[3] = {1 << 30, 1 << 30, 1 << 30}, hi[3] = {-1, -1, -1};
+    for (int b = 0; b < L.nblk; ++b)
+        for (int a = 0; a < 3; ++a) {
+            int l, h;
+            stage_region(L, edge_bits(L, b), a, step_i + T, l, h);
+            lo[a] = std::min(lo[a], l);
+            hi[a] = std::max(hi[a], h);
+        }
     RSched sch;
-    const int out0 = (L.xoff + 1) & ~3, NZ = L.n[2] - 2;
-    sch.ntx = (L.xoff + L.n[0] - 1 - out0 + kOutW - 1) / kOutW;
-    sch.nty = (L.n[1] - 2 + RCfg<T, NW>::OH - 1) / RCfg<T, NW>::OH;
+    sch.x0 = (L.xoff + lo[0]) & ~3;
+    sch.y0 = lo[1];
+    sch.z0 = lo[2];
+    const int NZ = std::max(1, hi[2] - lo[2] + 1);
+    sch.ntx = std::max(0, L.xoff + hi[0] - sch.x0) / kOutW + 1;
+    sch.nty = (std::max(1, hi[1] - lo[1] + 1) + RCfg<T, NW>::OH - 1) / RCfg<T, NW>::OH;
     sch.Lz = r_chunk((long long)sch.ntx * sch.nty * L.nblk, NZ, T, sms, cost);
     sch.nzc = (NZ + sch.Lz - 1) / sch.Lz;
     return sch;
@@ -315,7 +329,7 @@ cudaError_t launch_r(const CUtensorMap* tin, float* out, const BlockLayout& L, i
     int total = 0;      // one CTA per SM
     if (cudaError_t e = kernel_setup(setup, heat_rows_kernel<T, NW>, 32 * NW, Cfg::SMEM, nullptr, &total)) return e;
     long long cost;
-    const RSched sch = r_sched<T, NW>(L, total, cost);
+    const RSched sch = r_sched<T, NW>(L, step_i, total, cost);
     return launch_pdl(heat_rows_kernel<T, NW>, (unsigned)((long long)sch.ntx * sch.nty * L.nblk * sch.nzc), 32 * NW, Cfg::SMEM, st, *tin, out, L, step_i,
                       c, sch, status);
 }
@@ -329,7 +343,7 @@ int heat_rows_box_w() { return kBoxW; }
 double heat_rows_us(const BlockLayout& L)
 {
     long long cost;
-    r_sched<3, kNW3>(L, 152, cost);
+    r_sched<3, kNW3>(L, 0, 152, cost);
     return 1.12 * (double)cost;
 }
 int heat_rows_box_h(int T) { return kRY * (T == 2 ? kNW2 : T == 3 ? kNW3 : kNW4) + 2; }
