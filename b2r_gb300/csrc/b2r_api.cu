@@ -512,6 +512,16 @@ b2r_status advance(b2r_handle* h, int n)
     return B2R_OK;
 }
 
+// The heat domain as one block, on a torus with three steps between exchanges.
+BlockLayout one_block(const b2r_handle* h)
+{
+    const int* e = h->cfg.env;
+    const int H = (h->L.periodic ? 3 : 1) * h->cfg.D, nb[3] = {1, 1, 1}, n[3] = {e[0] + 2 * H, e[1] + 2 * H, e[2] + 2 * H};
+    BlockLayout one;
+    fill_layout(one, n, e, nb, H, 4, h->L.periodic, -1);
+    return one;
+}
+
 // Whether a cluster's shared memory holds the heat domain and steps it faster
 // than launches do: by the estimate of a pass of two (radius 1), of a launch per
 // step (radius 2: 3.1 us at least), on a torus with an exchange every third.
@@ -520,10 +530,7 @@ void make_small(b2r_handle* h)
     const b2r_config& c = h->cfg;
     const int ctas = heat_small_ctas(c.env, c.D);
     if (!ctas) return;
-    BlockLayout one;
-    const int H = (h->L.periodic ? 3 : 1) * c.D, nb[3] = {1, 1, 1};
-    const int n[3] = {c.env[0] + 2 * H, c.env[1] + 2 * H, c.env[2] + 2 * H};
-    fill_layout(one, n, c.env, nb, H, 4, h->L.periodic, -1);
+    const BlockLayout one = one_block(h);
     const double other = (c.D == 1 ? heat2_us(one) / 2 : 3.1) + (h->L.periodic ? 1.2 : 0.0);
     h->small_gain = other - heat_small_us(c.env, c.D, ctas);
     if (h->small_gain > 0) h->small_ctas = ctas;
@@ -538,10 +545,12 @@ bool small_runs(const b2r_handle* h, int n)
 
 // The one-block form of a domain of several blocks, or of a heat domain on a
 // torus.  A shelled domain then needs no exchange at all; a torus keeps one,
-// every three steps, with radius 3 and 4 every two (a deeper halo computes more
-// cells than the exchanges it saves cost).  48 heat steps with 1 / 2 / 3 / 4 steps
+// every three steps, with radius 3 and 4 every two, with radius 1 every four where
+// a pass takes two (a deeper halo computes more cells than the exchanges it saves
+// cost).  48 heat steps with 1 / 2 / 3 / 4 steps
 // between exchanges: 250x186x132, radius 2, 819 / 671 / 670 / 702 us, 128^3 495 /
-// 434 / 422 / 439; radius 1, 256^3 1661 / 1065 / 885 / 1003; radius 3, 128^3 536 /
+// 434 / 422 / 439; radius 1, 256^3 1661 / 1065 / 885 / 1003, 120^3 436 / 345 / 328 /
+// 299; radius 3, 128^3 536 /
 // 503 / 529 / 525; radius 4, 250x100x100 650 / 587 / 639 / 660.  Made where what it
 // allocates takes at most an eighth of the free memory: two buffers for heat,
 // ten fields for the collocated wave, the material for the staggered one, whose
@@ -552,7 +561,12 @@ void make_joined(b2r_handle* h)
     b2r_config c = h->cfg;
     for (int a = 0; a < 3; ++a) c.blocks[a] = 1;
     const int least = std::min(c.env[0], std::min(c.env[1], c.env[2]));
-    c.R = h->L.periodic ? std::max(1, std::min(c.D <= 2 ? 3 : 2, least / 2 / c.D)) : 1;
+    c.R = 1;
+    if (h->L.periodic) {
+        const BlockLayout one = one_block(h);
+        const int period = c.D >= 3 ? 2 : c.D == 1 && heat2_us(one) / 2 <= heat_rows_us(one) / 3 ? 4 : 3;
+        c.R = std::max(1, std::min(period, least / 2 / c.D));
+    }
     if (h->L.nblk == 1 && c.R <= h->cfg.R) return;
     const int nf = c.model == B2R_MODEL_HEAT ? 2 : c.model == B2R_MODEL_EQWP_REF ? 10 : 3;
     const int H = c.R * halo_per_step(c);
