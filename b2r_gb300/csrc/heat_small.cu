@@ -145,23 +145,25 @@ heat_small_kernel(float* __restrict__ buf, const BlockLayout M, const SGeo s, co
     const bool k1 = left > 1, k2 = left > 2, k3 = left > 3;
     const int store = (int)threadIdx.x < items ? nzr : 0;   // planes stored
     // where the neighbours' copies of this CTA's outer planes lie (shared
-    // addresses of cell (0, 0, plane 0 of this CTA), 0: no neighbour)
+    // addresses of cell (0, 0, plane 0 of this CTA) as the neighbour counts, which
+    // may lie before its memory, at 0 even)
     const uint32_t here = smem_u32(sm) + 4u * (uint32_t)origin;
     uint32_t below = 0, above = 0, bar_below = 0, bar_above = 0;
-    if (rank > 0 || M.periodic) {
+    const bool has_below = rank > 0 || M.periodic, has_above = rank < s.ctas - 1 || M.periodic;
+    if (has_below) {
         const int q = rank > 0 ? rank - 1 : s.ctas - 1;
         bar_below = peer(smem_u32(bar), q);
         below = peer(here, q) + 4u * (uint32_t)((s.base + (q < s.rem)) * plane);
     }
-    if (rank < s.ctas - 1 || M.periodic) {
+    if (has_above) {
         const int q = rank < s.ctas - 1 ? rank + 1 : 0;
         bar_above = peer(smem_u32(bar), q);
         above = peer(here, q) - 4u * (uint32_t)(nzl * plane);
     }
-    const uint32_t bytes = 16u * (uint32_t)(D * cols) * ((below ? 1 : 0) + (above ? 1 : 0));   // received per step
-    const bool waits = (below && zr < D) || (above && zr + nzr > nzl - D);
+    const uint32_t bytes = 16u * (uint32_t)(D * cols) * ((has_below ? 1 : 0) + (has_above ? 1 : 0));   // received per step
+    const bool waits = (has_below && zr < D) || (has_above && zr + nzr > nzl - D);
     // planes stored there: the first `down`, and from `up` on
-    const int down = below ? min(store, D - zr) : 0, up = above ? max(0, nzl - D - zr) : ZR;
+    const int down = has_below ? min(store, D - zr) : 0, up = has_above ? max(0, nzl - D - zr) : ZR;
     const float2 a0 = make_float2(C.a0, C.a0);
     cluster_sync();
 

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
     ((48, 40, 32), (2, 2, 1), 2, 1, False), ((33, 17, 2), (1, 1, 1), 1, 1, False), ((6, 5, 37), (1, 1, 1), 1, 1, False),
     ((129, 8, 31), (1, 1, 1), 1, 1, False), ((30, 45, 51), (3, 1, 3), 2, 1, False), ((47, 40, 32), (1, 1, 1), 1, 2, False),
     ((16, 20, 18), (2, 2, 1), 1, 2, False), ((40, 33, 32), (2, 1, 1), 1, 1, True), ((35, 2, 2), (1, 1, 1), 1, 1, True),
-    ((4, 4, 18), (1, 1, 1), 1, 2, True), ((37, 13, 21), (1, 1, 1), 1, 2, True), ((18, 12, 48), (1, 2, 3), 1, 2, True)])
+    ((4, 4, 18), (1, 1, 1), 1, 2, True), ((2, 21, 41), (1, 3, 1), 1, 1, True), ((37, 13, 21), (1, 1, 1), 1, 2, True), ((18, 12, 48), (1, 2, 3), 1, 2, True)])
 def test_small_equals_blocks(b2r, env, blocks, R, D, periodic):
     import torch
     rng = np.random.default_rng(29)
