@@ -327,9 +327,7 @@ __device__ __noinline__ uint4 run_two_step(const BatchArgs& a, int k, int t, int
 #ifndef B2R_BATCH_MINB
 #define B2R_BATCH_MINB 2   // resident CTAs per SM the register budget is fitted to (no spills)
 #endif
-// TWO: some instance runs on two-step units (a separate instantiation, so
-// that runs without them keep the one-step units' register allocation)
-template <bool TWO>
+// Batches of which some instance runs on two-step units.
 __global__ void __launch_bounds__(kThreads, B2R_BATCH_MINB) batch_kernel(const BatchArgs a)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -370,7 +368,7 @@ __global__ void __launch_bounds__(kThreads, B2R_BATCH_MINB) batch_kernel(const B
         const int t = s_t, k = s_k, u = s_u;
         const InstDev& in = a.inst[k];
         bool ok;
-        if (TWO && in.tb == 2) {
+        if (in.tb == 2) {
             const uint4 r = run_two_step(a, k, t, u, rg.gp, rg.issued_hi, rg.stop, s1, rg.smem);
             rg.gp = r.x;
             rg.issued_hi = r.y;
@@ -629,7 +627,7 @@ b2r_status enqueue_run(b2r_batch* b, cudaStream_t st)
         a.done = b->d_done;
         a.status = b->d_status;
         a.total = u.total;
-        if (b->two) batch_kernel<true><<<b->grid[4], kThreads, b->smem, s>>>(a);
+        if (b->two) batch_kernel<<<b->grid[4], kThreads, b->smem, s>>>(a);
         else
             switch (u.D) {
             case 1: batch_far_kernel<1><<<b->grid[0], kQThreads, kQSmem, s>>>(a); break;
@@ -733,7 +731,7 @@ b2r_status b2r_batch_create(const b2r_batch_item* items, int n, b2r_batch** out)
         static SmemLimit limit[5];
         const void* fns[5] = {(const void*)batch_far_kernel<1>, (const void*)batch_far_kernel<2>,
                               (const void*)batch_far_kernel<3>, (const void*)batch_far_kernel<4>,
-                              (const void*)batch_kernel<true>};
+                              (const void*)batch_kernel};
         for (int v = 0; v < 5; ++v) {
             int occ = 0;
             const size_t smem = v < 4 ? kQSmem : b->smem;
