@@ -415,7 +415,7 @@ struct b2r_batch {
     size_t staging_bytes = 0;
     int maxrounds = 0;               // rounds of the current schedule's longest instance
     long long total = 0;
-    int lz_policy = 16;              // z chunk cap per unit (autotuned)
+    int lz_policy = -1;              // z chunk cap per unit; -1: by the batch's sizes (auto_planes)
     int grid[5] = {};                // persistent grid (every resident slot): radius 1..4, with two-step units
     bool two = false;                // some instance runs on two-step units
     // launches of a run: one per radius (instances sched[first .. first + n), queue d_items + at),
@@ -532,6 +532,46 @@ b2r_status apply_shapes(b2r_batch* b, const std::vector<int>& sh)
 
 b2r_status apply_shape(b2r_batch* b, int s) { return apply_shapes(b, std::vector<int>(b->n, s)); }
 
+// Planes per unit when the caller set none: the count with the shortest run if a
+// unit takes 3 us and 0.55 us per plane it reads, a round of a radius (a launch
+// of its own) lasts one unit at least, or as many one after the other as each
+// resident CTA gets, and the radii follow one another.  The units of a small
+// batch have to be short for every CTA to get one: 18 instances of 24..75 cells a
+// side took 4.98 ms at 16 planes and take 2.77 ms at the 2 or 3 this picks, 14 of
+// 32..80 5.31 and 3.01, 39 of 32..140 17.1 and 14.7 (12.9 at 6); 64 of 32..192
+// stay at 16 (46.8 ms, at 8 planes 52.4).
+static int auto_planes(const b2r_batch* b)
+{
+    if (b->two) return 16;
+    std::vector<int> by(b->sched);
+    std::sort(by.begin(), by.end(), [&](int x, int y) { return b->host[x].rounds > b->host[y].rounds; });
+    int best = 16;
+    double least = 1e300;
+    for (int lz : {16, 12, 8, 6, 4, 3, 2}) {
+        double us = 0;
+        for (int D = 1; D <= 4; ++D) {
+            double units = 0, planes = 0, one = 0;   // of a round of the instances so far, which all step longer
+            int left = 0;
+            for (int k : by) {
+                const InstDev& in = b->host[k];
+                if (in.D != D) continue;
+                us += (left - in.rounds) * one;
+                const double n = (double)in.ntx * in.nty * ((in.NZ + lz - 1) / lz);
+                units += n;
+                planes += n * (std::min(lz, in.NZ) + 2 * D);
+                one = std::max(1.0, units / 304.0) * (3.0 + 0.55 * planes / units);
+                left = in.rounds;
+            }
+            us += left * one;
+        }
+        if (us < least) {
+            least = us;
+            best = lz;
+        }
+    }
+    return best;
+}
+
 // The queue for the current shapes and Lz policy: work items (round,
 // instance, unit) written out in claim order, round-major.  A round is one
 // step of a one-step instance or two of a two-step one; the instances are
@@ -550,9 +590,10 @@ b2r_status build_schedule(b2r_batch* b)
     std::vector<CUtensorMap> maps(2 * b->n);
     b->maxrounds = 0;
     int ndone = 0;
+    const int policy = b->lz_policy >= 0 ? b->lz_policy : auto_planes(b);
     for (int j = 0; j < b->n; ++j) {
         InstDev& in = b->host[b->sched[j]];
-        in.Lz = std::min(in.NZ, b->lz_policy > 0 ? b->lz_policy : in.NZ);
+        in.Lz = std::min(in.NZ, policy > 0 ? policy : in.NZ);
         in.nzc = (in.NZ + in.Lz - 1) / in.Lz;
         in.units = in.ntx * in.nty * in.nzc;
         in.done0 = ndone;
