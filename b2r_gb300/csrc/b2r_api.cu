@@ -1477,6 +1477,8 @@ b2r_status b2r_eqwp_gpu_main(b2r_handle* h, int ts, int R, double* gpu_seconds)
         st = substep(h, i);
     }
     h->ts = save;
+    h->halos_fresh = false;   // whoever filled the halos, the interiors have moved on
+    h->xmask = 0;
     cudaEventRecord(e1, h->stream);
     cudaEventSynchronize(e1);
     float ms = 0.f;

@@ -297,7 +297,9 @@ b2r_status b2r_heat_3D_gpu_main_noalloc(const float* d_in, float* d_out, int R, 
                                         void* cuda_stream);
 /* eqwp_gpu_main (eqwp.cu:661): R steps of the reference elastic-wave model on
  * the handle's fields (model B2R_MODEL_EQWP_REF), ts = the outer time step
- * (selects the body force, eqwp.cu:135).  Does not exchange halos. */
+ * (selects the body force, eqwp.cu:135).  Does not exchange halos, except
+ * after a run that went through none (see TBLOCK), whose halos are brought
+ * up to date first; the next b2r_step starts with an exchange. */
 b2r_status b2r_eqwp_gpu_main(b2r_handle* h, int ts, int R, double* gpu_seconds);
 /* write_block_data_bin / write_block_data (eqwp.cu:616-651): one padded
  * block of a float field (halos included, Ngx*Ngy*Ngz cells, x fastest) to
