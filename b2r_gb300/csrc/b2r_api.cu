@@ -991,13 +991,13 @@ b2r_status b2r_upload(b2r_handle* h, int field, const void* src, int src_is_devi
         CK(h, launch_scatter<float>(static_cast<const float*>(dsrc), static_cast<float*>(dst),
                                     static_cast<float*>(dst2), h->L, h->shell, h->stream));
     h->ts = 0;
-    h->halos_lost = false;   // a period starts, with an exchange unless every field is uploaded
     // the scatter filled this field's halos; the others are fresh only if
     // they were, or once every field has been uploaded since the last step
     if (!h->halos_fresh && !is_mat) {   // material never changes: its halos stay consistent
         const int nf = eq ? h->nfld : 1;
         h->upmask |= 1u << (eq ? field : 0);
         h->halos_fresh = h->upmask == (nf >= 32 ? ~0u : (1u << nf) - 1u);
+        if (h->halos_fresh) h->halos_lost = false;
     }
     return B2R_OK;
 }
@@ -1219,7 +1219,10 @@ static b2r_status note_exchange(b2r_handle* h, int field, b2r_status st)
     }
     h->xmask |= 1u << field;
     const int nf = (h->cfg.model == B2R_MODEL_EQWP_REF || h->cfg.model == B2R_MODEL_EQWP_STAG) ? h->nfld : 1;
-    if (h->xmask == (nf >= 32 ? ~0u : (1u << nf) - 1u)) h->halos_fresh = true;
+    if (h->xmask == (nf >= 32 ? ~0u : (1u << nf) - 1u)) {
+        h->halos_fresh = true;
+        h->halos_lost = false;
+    }
     return st;
 }
 
