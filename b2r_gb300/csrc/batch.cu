@@ -495,7 +495,7 @@ b2r_status build_schedule(b2r_batch* b);
 
 // tile counts, steps per unit and tensor-map boxes of every instance for
 // its shape sh[k] (two-step units for radius 1 only)
-b2r_status apply_shapes(b2r_batch* b, const std::vector<int>& sh)
+b2r_status set_shapes(b2r_batch* b, const std::vector<int>& sh)
 {
     b->two = false;
     for (int k = 0; k < b->n; ++k) b->two = b->two || (sh[k] == kTwoStep && b->host[k].D == 1);
@@ -530,6 +530,21 @@ b2r_status apply_shapes(b2r_batch* b, const std::vector<int>& sh)
     return build_schedule(b);
 }
 
+// ... and where that fails (a queue too long), the shapes and the queue of before
+b2r_status apply_shapes(b2r_batch* b, const std::vector<int>& sh)
+{
+    const std::vector<InstDev> host = b->host;
+    const std::vector<CUtensorMap> maps = b->maps;
+    const bool two = b->two;
+    const b2r_status st = set_shapes(b, sh);
+    if (st != B2R_OK) {
+        b->host = host;
+        b->maps = maps;
+        b->two = two;
+    }
+    return st;
+}
+
 b2r_status apply_shape(b2r_batch* b, int s) { return apply_shapes(b, std::vector<int>(b->n, s)); }
 
 // Planes per unit when the caller set none: the count with the shortest run if a
@@ -543,7 +558,8 @@ b2r_status apply_shape(b2r_batch* b, int s) { return apply_shapes(b, std::vector
 static int auto_planes(const b2r_batch* b)
 {
     if (b->two) return 16;
-    std::vector<int> by(b->sched);
+    std::vector<int> by(b->n);
+    for (int k = 0; k < b->n; ++k) by[k] = k;
     std::sort(by.begin(), by.end(), [&](int x, int y) { return b->host[x].rounds > b->host[y].rounds; });
     int best = 16;
     double least = 1e300;
@@ -580,45 +596,35 @@ static int auto_planes(const b2r_batch* b)
 // instance, which the queue holds earlier, so the queue cannot deadlock.
 b2r_status build_schedule(b2r_batch* b)
 {
-    b->sched.resize(b->n);
-    for (int k = 0; k < b->n; ++k) b->sched[k] = k;
-    std::stable_sort(b->sched.begin(), b->sched.end(), [&](int x, int y) {
+    // everything that a run uses changes at the end, together: a queue that is
+    // refused leaves the one before it, with its descriptors, in place
+    std::vector<int> sched(b->n);
+    for (int k = 0; k < b->n; ++k) sched[k] = k;
+    std::stable_sort(sched.begin(), sched.end(), [&](int x, int y) {
         const InstDev &p = b->host[x], &q = b->host[y];
         return !b->two && p.D != q.D ? p.D > q.D : p.rounds > q.rounds;
     });
-    std::vector<InstDev> dev(b->n);
+    std::vector<InstDev> host = b->host, dev(b->n);
     std::vector<CUtensorMap> maps(2 * b->n);
-    b->maxrounds = 0;
-    int ndone = 0;
+    std::vector<int> rounds(b->n), units(b->n);
+    int maxrounds = 0, ndone = 0;
     const int policy = b->lz_policy >= 0 ? b->lz_policy : auto_planes(b);
     for (int j = 0; j < b->n; ++j) {
-        InstDev& in = b->host[b->sched[j]];
+        InstDev& in = host[sched[j]];
         in.Lz = std::min(in.NZ, policy > 0 ? policy : in.NZ);
         in.nzc = (in.NZ + in.Lz - 1) / in.Lz;
         in.units = in.ntx * in.nty * in.nzc;
         in.done0 = ndone;
         ndone += b->two ? 1 : in.nzc;
         dev[j] = in;
-        maps[2 * j] = b->maps[2 * b->sched[j]];
-        maps[2 * j + 1] = b->maps[2 * b->sched[j] + 1];
-        b->maxrounds = std::max(b->maxrounds, in.rounds);
-    }
-    // no run of this batch may still read the queue or the descriptors
-    BCK(cudaDeviceSynchronize(), "waiting for the batch's runs");
-    if (ndone > b->ndone) {
-        cudaFree(b->d_done);
-        b->d_done = nullptr;
-        b->ndone = 0;
-        BCK(cudaMalloc(&b->d_done, sizeof(unsigned) * ndone), "counter allocation");
-        b->ndone = ndone;
-    }
-    std::vector<int> rounds(b->n), units(b->n);
-    for (int j = 0; j < b->n; ++j) {
-        rounds[j] = dev[j].rounds;
-        units[j] = dev[j].units;
+        rounds[j] = in.rounds;
+        units[j] = in.units;
+        maps[2 * j] = b->maps[2 * sched[j]];
+        maps[2 * j + 1] = b->maps[2 * sched[j] + 1];
+        maxrounds = std::max(maxrounds, in.rounds);
     }
     std::vector<unsigned long long> items, part;
-    b->runs.clear();
+    std::vector<b2r_batch::Launch> runs;
     for (int first = 0; first < b->n;) {
         int n = 1;
         while (first + n < b->n && (b->two || dev[first + n].D == dev[first].D)) ++n;
@@ -626,33 +632,37 @@ b2r_status build_schedule(b2r_batch* b)
             items.size() + part.size() > (size_t)1 << 28)
             return bfail(B2R_ERR_ARG, "the batch queue is too long (an instance with more than 2^24 units or "
                                       "rounds, or more than 2^28 work items): split the batch");
-        b->runs.push_back({dev[first].D, first, n, (long long)items.size(), (long long)part.size()});
+        runs.push_back({dev[first].D, first, n, (long long)items.size(), (long long)part.size()});
         items.insert(items.end(), part.begin(), part.end());
         first += n;
     }
-    b->total = (long long)items.size();
-    if (b->total > b->items_cap) {
-        cudaFree(b->d_items);
-        b->d_items = nullptr;
-        b->items_cap = 0;
-        BCK(cudaMalloc(&b->d_items, sizeof(unsigned long long) * std::max<long long>(1, b->total)), "queue allocation");
-        b->items_cap = b->total;
-    }
+    const long long total = (long long)items.size();
+    // no run of this batch may still read the queue or the descriptors
+    BCK(cudaDeviceSynchronize(), "waiting for the batch's runs");
+    auto no_graph = [&] {
+        if (b->gexec) cudaGraphExecDestroy(b->gexec);
+        b->gexec = nullptr;
+    };
+    BCK(wq::grow(b->d_done, b->ndone, ndone, no_graph), "counter allocation");
+    BCK(wq::grow(b->d_items, b->items_cap, std::max<long long>(1, total), no_graph), "queue allocation");
+    no_graph();
     BCK(cudaMemcpy(b->d_inst, dev.data(), sizeof(InstDev) * b->n, cudaMemcpyHostToDevice), "copy descriptors");
     BCK(cudaMemcpy(b->d_maps, maps.data(), sizeof(CUtensorMap) * 2 * b->n, cudaMemcpyHostToDevice),
         "copy tensor maps");
-    if (b->total > 0)
-        BCK(cudaMemcpy(b->d_items, items.data(), sizeof(unsigned long long) * b->total, cudaMemcpyHostToDevice),
+    if (total > 0)
+        BCK(cudaMemcpy(b->d_items, items.data(), sizeof(unsigned long long) * total, cudaMemcpyHostToDevice),
             "copy the queue");
-    if (b->gexec) {
-        cudaGraphExecDestroy(b->gexec);
-        b->gexec = nullptr;
-    }
+    b->host = host;
+    b->sched = sched;
+    b->runs = runs;
+    b->total = total;
+    b->maxrounds = maxrounds;
     return B2R_OK;
 }
 
 b2r_status enqueue_run(b2r_batch* b, cudaStream_t st)
 {
+    if (!b->d_items || !b->d_done) return bfail(B2R_ERR_STATE, "no memory was left for the batch's queue");
     BCK(cudaMemsetAsync(b->d_head, 0, 4 * sizeof(unsigned long long), st), "reset queue");
     BCK(cudaMemsetAsync(b->d_done, 0, sizeof(unsigned) * b->ndone, st), "reset counters");
     if (b->runs.size() > 1) BCK(cudaEventRecord(b->fork, st), "batch launch");
@@ -897,8 +907,11 @@ int64_t b2r_batch_lups(const b2r_batch* b)
 b2r_status b2r_batch_set_zchunk(b2r_batch* b, int zchunk)
 {
     if (!b || zchunk < 0) return bfail(B2R_ERR_ARG, "invalid argument");
+    const int before = b->lz_policy;
     b->lz_policy = zchunk;
-    return build_schedule(b);
+    const b2r_status st = build_schedule(b);
+    if (st != B2R_OK) b->lz_policy = before;
+    return st;
 }
 
 

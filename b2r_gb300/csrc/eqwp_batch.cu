@@ -227,54 +227,47 @@ b2r_status build(b2r_eqwp_batch* b)
         in.tiles = in.gx * in.gy;
         in.reach = lz >= 2 ? 1 : 2;
     }
-    b->sched.resize(b->n);
-    for (int k = 0; k < b->n; ++k) b->sched[k] = k;
-    std::stable_sort(b->sched.begin(), b->sched.end(),
+    std::vector<int> sched(b->n);
+    for (int k = 0; k < b->n; ++k) sched[k] = k;
+    std::stable_sort(sched.begin(), sched.end(),
                      [&](int x, int y) { return b->host[x].rounds > b->host[y].rounds; });
     std::vector<EInst> dev(b->n);
     std::vector<int> rounds(b->n), units(b->n);
     for (int j = 0; j < b->n; ++j) {
-        dev[j] = b->host[b->sched[j]];
+        dev[j] = b->host[sched[j]];
         dev[j].chunk0 = j ? dev[j - 1].chunk0 + dev[j - 1].T.nzc : 0;
         rounds[j] = dev[j].rounds;
         units[j] = dev[j].units;
     }
-    // no run of this batch may still read the queue or the descriptors
-    ECK(cudaDeviceSynchronize(), "waiting for the batch's runs");
+    const int chunks = dev[b->n - 1].chunk0 + dev[b->n - 1].T.nzc;
+    // a queue that is refused leaves the one before it in place
     std::vector<unsigned long long> items;
     if (!wq::round_major_items(rounds.data(), units.data(), b->n, items))
         return efail(B2R_ERR_ARG, "the batch queue is too long (an instance with more than 2^24 units or "
                                   "rounds, or more than 2^28 work items): split the batch");
-    b->total = (long long)items.size();
-    if (b->total > b->items_cap) {
-        cudaFree(b->d_items);
-        b->d_items = nullptr;
-        b->items_cap = 0;
-        ECK(cudaMalloc(&b->d_items, sizeof(unsigned long long) * std::max<long long>(1, b->total)), "queue allocation");
-        b->items_cap = b->total;
-    }
-    const int chunks = dev[b->n - 1].chunk0 + dev[b->n - 1].T.nzc;
-    if (chunks > b->chunks_cap) {
-        cudaFree(b->d_done);
-        b->d_done = nullptr;
-        b->chunks_cap = 0;
-        ECK(cudaMalloc(&b->d_done, sizeof(unsigned) * chunks), "counter allocation");
-        b->chunks_cap = chunks;
-    }
-    b->chunks = chunks;
-    ECK(cudaMemcpy(b->d_inst, dev.data(), sizeof(EInst) * b->n, cudaMemcpyHostToDevice), "copy descriptors");
-    if (b->total > 0)
-        ECK(cudaMemcpy(b->d_items, items.data(), sizeof(unsigned long long) * b->total, cudaMemcpyHostToDevice),
-            "copy the queue");
-    if (b->gexec) {
-        cudaGraphExecDestroy(b->gexec);
+    const long long total = (long long)items.size();
+    // no run of this batch may still read the queue or the descriptors
+    ECK(cudaDeviceSynchronize(), "waiting for the batch's runs");
+    auto no_graph = [&] {
+        if (b->gexec) cudaGraphExecDestroy(b->gexec);
         b->gexec = nullptr;
-    }
+    };
+    ECK(wq::grow(b->d_items, b->items_cap, std::max<long long>(1, total), no_graph), "queue allocation");
+    ECK(wq::grow(b->d_done, b->chunks_cap, chunks, no_graph), "counter allocation");
+    no_graph();
+    ECK(cudaMemcpy(b->d_inst, dev.data(), sizeof(EInst) * b->n, cudaMemcpyHostToDevice), "copy descriptors");
+    if (total > 0)
+        ECK(cudaMemcpy(b->d_items, items.data(), sizeof(unsigned long long) * total, cudaMemcpyHostToDevice),
+            "copy the queue");
+    b->sched = sched;
+    b->chunks = chunks;
+    b->total = total;
     return B2R_OK;
 }
 
 b2r_status enqueue(b2r_eqwp_batch* b, cudaStream_t st)
 {
+    if (!b->d_items || !b->d_done) return efail(B2R_ERR_STATE, "no memory was left for the batch's queue");
     ECK(cudaMemsetAsync(b->d_head, 0, sizeof(unsigned long long), st), "reset queue");
     ECK(cudaMemsetAsync(b->d_done, 0, sizeof(unsigned) * b->chunks, st), "reset counters");
     EArgs a;
@@ -474,8 +467,11 @@ int64_t b2r_eqwp_batch_lups(const b2r_eqwp_batch* b)
 b2r_status b2r_eqwp_batch_set_zchunk(b2r_eqwp_batch* b, int zchunk)
 {
     if (!b || zchunk < 0) return efail(B2R_ERR_ARG, "invalid argument");
+    const int before = b->lz_policy;
     b->lz_policy = zchunk;
-    return build(b);
+    const b2r_status st = build(b);
+    if (st != B2R_OK) b->lz_policy = before;
+    return st;
 }
 
 }  // extern "C"

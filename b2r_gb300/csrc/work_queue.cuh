@@ -67,6 +67,29 @@ inline bool round_major_items(const int* rounds, const int* units, int n, std::v
     return true;
 }
 
+// Room for `need` elements in the device array p that now holds `cap`.  Where
+// both fit, the old array is given up only for the new one, so that a failure
+// leaves it as it was; `give_up` (destroy what still refers to it) comes first.
+template <class T, class N, class F>
+inline cudaError_t grow(T*& p, N& cap, N need, F give_up)
+{
+    if (need <= cap) return cudaSuccess;
+    T* more = nullptr;
+    cudaError_t e = cudaMalloc(&more, sizeof(T) * (size_t)need);
+    if (e != cudaSuccess) cudaGetLastError();
+    if (e == cudaSuccess || p) {
+        give_up();
+        cudaFree(p);
+        p = nullptr;
+        cap = 0;
+        if (e != cudaSuccess) e = cudaMalloc(&more, sizeof(T) * (size_t)need);
+    }
+    if (e != cudaSuccess) return e;
+    p = more;
+    cap = need;
+    return cudaSuccess;
+}
+
 // Bounded wait (2 s) until *done >= need; false if it gave up.  Afterwards
 // the data that other CTAs stored with generic stores may be read through
 // TMA as well.
