@@ -19,6 +19,7 @@
 #include <new>
 #include <vector>
 
+#include "batch_planes.h"
 #include "heat2_unit.cuh"
 #include "heat_far.cuh"
 #include "heat_unit.cuh"
@@ -547,45 +548,13 @@ b2r_status apply_shapes(b2r_batch* b, const std::vector<int>& sh)
 
 b2r_status apply_shape(b2r_batch* b, int s) { return apply_shapes(b, std::vector<int>(b->n, s)); }
 
-// Planes per unit when the caller set none: the count with the shortest run if a
-// unit takes 3 us and 0.55 us per plane it reads, a round of a radius (a launch
-// of its own) lasts one unit at least, or as many one after the other as each
-// resident CTA gets, and the radii follow one another.  The units of a small
-// batch have to be short for every CTA to get one: 18 instances of 24..75 cells a
-// side took 4.98 ms at 16 planes and take 2.77 ms at the 2 or 3 this picks, 14 of
-// 32..80 5.31 and 3.01, 39 of 32..140 17.1 and 14.7 (12.9 at 6); 64 of 32..192
-// stay at 16 (46.8 ms, at 8 planes 52.4).
+// Planes per unit when the caller set none (batch_planes.h).
 static int auto_planes(const b2r_batch* b)
 {
     if (b->two) return 16;
-    std::vector<int> by(b->n);
-    for (int k = 0; k < b->n; ++k) by[k] = k;
-    std::sort(by.begin(), by.end(), [&](int x, int y) { return b->host[x].rounds > b->host[y].rounds; });
-    int best = 16;
-    double least = 1e300;
-    for (int lz : {16, 12, 8, 6, 4, 3, 2}) {
-        double us = 0;
-        for (int D = 1; D <= 4; ++D) {
-            double units = 0, planes = 0, one = 0;   // of a round of the instances so far, which all step longer
-            int left = 0;
-            for (int k : by) {
-                const InstDev& in = b->host[k];
-                if (in.D != D) continue;
-                us += (left - in.rounds) * one;
-                const double n = (double)in.ntx * in.nty * ((in.NZ + lz - 1) / lz);
-                units += n;
-                planes += n * (std::min(lz, in.NZ) + 2 * D);
-                one = std::max(1.0, units / 304.0) * (3.0 + 0.55 * planes / units);
-                left = in.rounds;
-            }
-            us += left * one;
-        }
-        if (us < least) {
-            least = us;
-            best = lz;
-        }
-    }
-    return best;
+    std::vector<wq::Column> in;
+    for (const InstDev& i : b->host) in.push_back({i.D, i.ntx * i.nty, i.NZ, i.rounds});
+    return wq::heat_planes(in);
 }
 
 // The queue for the current shapes and Lz policy: work items (round,
@@ -629,7 +598,7 @@ b2r_status build_schedule(b2r_batch* b)
         int n = 1;
         while (first + n < b->n && (b->two || dev[first + n].D == dev[first].D)) ++n;
         if (!wq::round_major_items(rounds.data() + first, units.data() + first, n, part) ||
-            items.size() + part.size() > (size_t)1 << 28)
+            (long long)(items.size() + part.size()) > wq::kMaxItems)
             return bfail(B2R_ERR_ARG, "the batch queue is too long (an instance with more than 2^24 units or "
                                       "rounds, or more than 2^28 work items): split the batch");
         runs.push_back({dev[first].D, first, n, (long long)items.size(), (long long)part.size()});

@@ -172,36 +172,13 @@ static int planes_of(const EInst& in)
     return std::max(1, hi - lo + 1);
 }
 
-// z chunk of the units when the caller set none: the one with the shortest
-// run if a unit takes 4 us and 2.05 us per plane (eqwp_tile.cuh) and a
-// round lasts one unit at least, or as many units one after the other as each
-// resident CTA gets; at most 12 planes, beyond which neighbouring tiles lose
-// their L2 hits.  GLUPS by planes 3, 4, 6, 8, 12, 16, 32: 16 instances of
-// 32-128 cells per edge 31.7, 34.2, 37.5, 38.8, 39.7, 39.8, 31.6; 8 of 64^3
-// 34.9, 37.5, 40.0, 32.8, 25.8, 18.8, 10.1; 12 of 36^3 23.4, 18.5, 13.4, 10.6,
-// 7.4, 7.4, 5.3; 6 of 200^3 32.4, 35.7, 38.9, 40.4, 40.1, 38.3, 34.5.
+// Planes per unit when the caller set none (batch_planes.h).
 static int auto_lz(const b2r_eqwp_batch* b)
 {
-    std::vector<int> by(b->n);
-    for (int k = 0; k < b->n; ++k) by[k] = k;
-    std::sort(by.begin(), by.end(), [&](int x, int y) { return b->nsteps[x] > b->nsteps[y]; });
-    int best = 2;
-    double least = 1e300;
-    for (int lz = 2; lz <= 12; ++lz) {
-        double us = 0;
-        long long units = 0;   // of a round in which the first j + 1 instances still step
-        for (int j = 0; j < b->n; ++j) {
-            const EInst& in = b->host[by[j]];
-            units += (long long)in.gx * in.gy * ((planes_of(in) + lz - 1) / lz);
-            const int rounds = 2 * (b->nsteps[by[j]] - (j + 1 < b->n ? b->nsteps[by[j + 1]] : 0));
-            us += rounds * std::max(1.0, (double)units / b->grid) * (4 + 2.05 * lz);
-        }
-        if (us < least) {
-            least = us;
-            best = lz;
-        }
-    }
-    return best;
+    std::vector<wq::Column> in;
+    for (int k = 0; k < b->n; ++k)
+        in.push_back({2, b->host[k].gx * b->host[k].gy, planes_of(b->host[k]), 2 * b->nsteps[k]});
+    return wq::wave_planes(in, b->grid);
 }
 
 // tiles, z chunks and the queue for the current z-chunk policy

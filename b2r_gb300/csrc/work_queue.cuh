@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "b2r_common.cuh"
+#include "batch_planes.h"
 
 namespace b2r {
 namespace wq {
@@ -58,7 +59,7 @@ inline bool round_major_items(const int* rounds, const int* units, int n, std::v
         total += (long long)units[j] * rounds[j];
         maxr = rounds[j] > maxr ? rounds[j] : maxr;
     }
-    if (total > (1ll << 28)) return false;
+    if (total > kMaxItems) return false;
     items.clear();
     items.reserve((size_t)total);
     for (int t = 0; t < maxr; ++t)
