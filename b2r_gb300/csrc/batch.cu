@@ -456,27 +456,28 @@ b2r_status bfail(b2r_status s, const char* msg, cudaError_t e = cudaSuccess)
 
 inline int roundup(int v, int m) { return (v + m - 1) / m * m; }
 
-// cells one plane of an instance computes with tile shape s
-long long plane_cells(const b2r_batch* b, int k, int s)
+// cells one plane of an instance computes with tile shape s; two: in a batch
+// with two-step units
+long long plane_cells(const b2r_batch* b, int k, int s, bool two)
 {
     const InstDev& in = b->host[k];
     const BlockLayout& L = in.L;
     const int D = in.D;
     const int X = L.xoff + L.n[0] - D - ((L.xoff + D) & ~3), Y = L.n[1] - 2 * D;
-    const int tw = 4 * kLpr[s], th = b->two ? kTileY[D][s] : kQTileY[s];
+    const int tw = 4 * kLpr[s], th = two ? kTileY[D][s] : kQTileY[s];
     return (long long)((X + tw - 1) / tw) * tw * ((Y + th - 1) / th) * th;
 }
 
 // The tile shape of instance k: the fewest cells computed per plane, narrow
 // tiles paying a little for their wider skirt (their boxes re-read a larger
 // share of the neighbouring tiles).
-int default_shape(const b2r_batch* b, int k)
+int default_shape(const b2r_batch* b, int k, bool two)
 {
     static const double penalty[3] = {1.0, 1.03, 1.08};
     int best = 0;
     double bc = 1e300;
     for (int s = 0; s < 3; ++s) {
-        const double c = (double)plane_cells(b, k, s) * penalty[s];
+        const double c = (double)plane_cells(b, k, s, two) * penalty[s];
         if (c < bc - 1e-9) {
             bc = c;
             best = s;
@@ -485,10 +486,10 @@ int default_shape(const b2r_batch* b, int k)
     return best;
 }
 
-std::vector<int> default_shapes(const b2r_batch* b)
+std::vector<int> default_shapes(const b2r_batch* b, bool two)
 {
     std::vector<int> sh(b->n);
-    for (int k = 0; k < b->n; ++k) sh[k] = default_shape(b, k);
+    for (int k = 0; k < b->n; ++k) sh[k] = default_shape(b, k, two);
     return sh;
 }
 
@@ -504,7 +505,7 @@ b2r_status set_shapes(b2r_batch* b, const std::vector<int>& sh)
         InstDev& in = b->host[k];
         const BlockLayout& L = in.L;
         const int D = in.D;
-        const int s = (sh[k] == kTwoStep && D != 1) ? default_shape(b, k) : sh[k];
+        const int s = (sh[k] == kTwoStep && D != 1) ? default_shape(b, k, b->two) : sh[k];
         in.shape = s;
         in.lpr = kLpr[s];
         int bw, bh;
@@ -761,7 +762,7 @@ b2r_status b2r_batch_create(const b2r_batch_item* items, int n, b2r_batch** out)
             b->grid[v] = std::max(1, occ) * std::max(1, sms);
         }
     }
-    b2r_status st = apply_shapes(b, default_shapes(b));
+    b2r_status st = apply_shapes(b, default_shapes(b, false));
     if (st != B2R_OK) return bail(st);
     if (cudaDeviceSynchronize() != cudaSuccess) return bail(bfail(B2R_ERR_CUDA, "batch set-up failed"));
     *out = b;
@@ -873,17 +874,20 @@ int64_t b2r_batch_lups(const b2r_batch* b)
     return s;
 }
 
-b2r_status b2r_batch_set_zchunk(b2r_batch* b, int zchunk)
+static b2r_status set_policy(b2r_batch* b, int policy)
 {
-    if (!b || zchunk < 0) return bfail(B2R_ERR_ARG, "invalid argument");
     const int before = b->lz_policy;
-    b->lz_policy = zchunk;
+    b->lz_policy = policy;
     const b2r_status st = build_schedule(b);
     if (st != B2R_OK) b->lz_policy = before;
     return st;
 }
 
-
+b2r_status b2r_batch_set_zchunk(b2r_batch* b, int zchunk)
+{
+    if (!b || zchunk < 0) return bfail(B2R_ERR_ARG, "invalid argument");
+    return set_policy(b, zchunk);
+}
 
 b2r_status b2r_batch_autotune(b2r_batch* b, void* stream, int* best_zchunk, double* best_ms)
 {
@@ -922,58 +926,75 @@ b2r_status b2r_batch_autotune(b2r_batch* b, void* stream, int* best_zchunk, doub
         cudaEventElapsedTime(&ms, e0, e1);
         return B2R_OK;
     };
-    static const int cands[] = {8, 16, 32, 64, 0};
-    float best = 1e30f;
-    int bestz = b->lz_policy;
-    // the z-chunk cap for the current shapes (a change must gain 0.5 %)
-    auto tune_zchunk = [&]() -> b2r_status {
-        for (int c = 0; c < 5; ++c) {
-            float ms = 0.f;
-            b2r_status r = b2r_batch_set_zchunk(b, cands[c]);
-            if (r == B2R_OK) r = trial(ms);
-            if (r != B2R_OK) return r;
-            if (ms < best * (cands[c] == bestz ? 1.f : 0.995f)) {
-                best = ms;
-                bestz = cands[c];
-            }
-        }
-        return b2r_batch_set_zchunk(b, bestz);
-    };
-    // 1. the z-chunk cap with every instance on its fewest-cells shape
-    std::vector<int> sh = default_shapes(b);
-    b2r_status s = apply_shapes(b, sh);
-    if (s == B2R_OK) s = tune_zchunk();
-    // 2. tile shapes per (stencil order, size class): the instances of one
-    // class try each other shape while the rest keep theirs (radius 1 also
-    // the two-step units); the size class is the interior width (the extent
-    // a tile width divides)
+    // the size class is the interior width (the extent a tile width divides)
     auto cls = [&](int k) {
         const int w = b->items[b->order[k]].env[0];
         return (b->host[k].D - 1) * 3 + (w <= 64 ? 0 : (w <= 128 ? 1 : 2));
     };
-    bool changed = false;
-    for (int c = 0; c < 12 && s == B2R_OK; ++c)
-        for (int t = 0; t < kShapes && s == B2R_OK; ++t) {
-            if (t == kTwoStep && c >= 3) continue;      // two-step units: radius 1 only
-            std::vector<int> cand = sh;
-            bool differs = false;
-            for (int k = 0; k < b->n; ++k)
-                if (cls(k) == c && cand[k] != t) {
-                    cand[k] = t;
-                    differs = true;
+    struct Found {
+        float ms = 1e30f;
+        int z = 0;
+        std::vector<int> sh;
+    };
+    // the best schedule found from one set of z chunks (-1: by the sizes)
+    auto search = [&](const std::vector<int>& zs, Found& f) -> b2r_status {
+        // the z chunk for the current shapes (a change must gain 0.5 %)
+        auto tune_zchunk = [&]() -> b2r_status {
+            for (int z : zs) {
+                float ms = 0.f;
+                b2r_status r = set_policy(b, z);
+                if (r == B2R_OK) r = trial(ms);
+                if (r != B2R_OK) return r;
+                if (ms < f.ms * (z == f.z ? 1.f : 0.995f)) {
+                    f.ms = ms;
+                    f.z = z;
                 }
-            if (!differs) continue;
-            float ms = 0.f;
-            if ((s = apply_shapes(b, cand)) != B2R_OK || (s = trial(ms)) != B2R_OK) break;
-            if (ms < best * 0.995f) {
-                best = ms;
-                sh = cand;
-                changed = true;
             }
-        }
-    // 3. the z-chunk cap again for the shapes picked
-    if (s == B2R_OK) s = apply_shapes(b, sh);
-    if (s == B2R_OK && changed) s = tune_zchunk();
+            return set_policy(b, f.z);
+        };
+        // 1. the z chunk with every instance on its fewest-cells shape
+        f.sh = default_shapes(b, false);
+        b2r_status s = apply_shapes(b, f.sh);
+        if (s == B2R_OK) s = tune_zchunk();
+        // 2. tile shapes per (stencil order, size class): the instances of one
+        // class try each other shape while the rest keep theirs (radius 1 also
+        // the two-step units)
+        bool changed = false;
+        for (int c = 0; c < 12 && s == B2R_OK; ++c)
+            for (int t = 0; t < kShapes && s == B2R_OK; ++t) {
+                if (t == kTwoStep && c >= 3) continue;      // two-step units: radius 1 only
+                std::vector<int> cand = f.sh;
+                bool differs = false;
+                for (int k = 0; k < b->n; ++k)
+                    if (cls(k) == c && cand[k] != t) {
+                        cand[k] = t;
+                        differs = true;
+                    }
+                if (!differs) continue;
+                float ms = 0.f;
+                if ((s = apply_shapes(b, cand)) != B2R_OK || (s = trial(ms)) != B2R_OK) break;
+                if (ms < f.ms * 0.995f) {
+                    f.ms = ms;
+                    f.sh = cand;
+                    changed = true;
+                }
+            }
+        // 3. the z chunk again for the shapes picked
+        if (s == B2R_OK) s = apply_shapes(b, f.sh);
+        if (s == B2R_OK && changed && zs.size() > 1) s = tune_zchunk();
+        return s;
+    };
+    // once with the units that the sizes give, as at creation, and once with
+    // fixed z chunks, which two-step units may want (ms of 18 instances of 24..75
+    // cells a side, of 12 of 24..39 with radius 4: 4.73, 1.30 with the former,
+    // 4.43, 1.98 with the latter)
+    Found own, fixed;
+    b2r_status s = search({-1}, own);
+    if (s == B2R_OK) s = search({8, 16, 32, 64, 0}, fixed);
+    const Found& best = fixed.ms < own.ms * 0.995f ? fixed : own;
+    const int bestz = best.z;
+    if (s == B2R_OK) s = set_policy(b, bestz);
+    if (s == B2R_OK) s = apply_shapes(b, best.sh);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     // restore every instance even after a failed trial; report the first failure
@@ -988,8 +1009,8 @@ b2r_status b2r_batch_autotune(b2r_batch* b, void* stream, int* best_zchunk, doub
     if (rerr == cudaSuccess) rerr = se;
     if (s != B2R_OK) return s;
     BCK(rerr, "restoring the instances after the trials");
-    if (best_zchunk) *best_zchunk = bestz;
-    if (best_ms) *best_ms = best;
+    if (best_zchunk) *best_zchunk = bestz >= 0 ? bestz : auto_planes(b) <= 8 ? 8 : 16;
+    if (best_ms) *best_ms = best.ms;
     return B2R_OK;
 }
 
@@ -997,7 +1018,7 @@ b2r_status b2r_batch_set_tile(b2r_batch* b, int width)
 {
     if (!b) return bfail(B2R_ERR_ARG, "null batch");
     switch (width) {
-    case 0: return apply_shapes(b, default_shapes(b));
+    case 0: return apply_shapes(b, default_shapes(b, false));
     case 128: return apply_shape(b, 0);
     case 64: return apply_shape(b, 1);
     case 32: return apply_shape(b, 2);
@@ -1024,7 +1045,7 @@ b2r_status b2r_batch_set_pass_steps(b2r_batch* b, int steps)
     if (steps != 1 && steps != 2) return bfail(B2R_ERR_ARG, "steps per pass must be 1 or 2");
     std::vector<int> sh(b->n);
     for (int k = 0; k < b->n; ++k)
-        sh[k] = b->host[k].D == 1 ? (steps == 2 ? kTwoStep : default_shape(b, k)) : b->host[k].shape;
+        sh[k] = b->host[k].D == 1 ? (steps == 2 ? kTwoStep : default_shape(b, k, false)) : b->host[k].shape;
     return apply_shapes(b, sh);
 }
 

@@ -383,7 +383,8 @@ b2r_status b2r_batch_run(b2r_batch* b, void* cuda_stream, int use_graph);
 b2r_status b2r_batch_synchronize(b2r_batch* b, void* cuda_stream);
 /* Total lattice-site updates of one run (sum of cells x steps). */
 int64_t b2r_batch_lups(const b2r_batch* b);
-/* Planes per work unit along z (0 = whole column). */
+/* Planes per work unit along z (0 = whole column).  Default: of 2 to 16 those
+ * with the shortest run, estimated from the sizes and step counts. */
 b2r_status b2r_batch_set_zchunk(b2r_batch* b, int zchunk);
 /* Tile shape of the instances: 128 x 14, 64 x 28 or 32 x 56 cells (x by y;
  * with two-step units in the batch 16, 32 or 64 rows, half as many for D >= 3),
@@ -405,11 +406,13 @@ int b2r_batch_instance_tile(const b2r_batch* b, int i);
 b2r_status b2r_batch_set_pass_steps(b2r_batch* b, int steps);
 int b2r_batch_instance_pass_steps(const b2r_batch* b, int i);
 /* Autotune on the uploaded inputs (restored afterwards), timing whole runs:
- * the z-chunk cap (8, 16, 32, 64, whole column), then the tile shape and
- * steps per pass per (stencil order, size class) -- the instances of one
- * class (order D, interior width <= 64, <= 128 or wider) try each tile shape
- * and, at radius 1, the two-step units, while the others keep theirs --
- * then the z-chunk cap again. */
+ * the z-chunk cap (by the sizes as at creation, 8, 16, 32, 64, whole
+ * column; *best_zchunk gets it, 8 or 16 where the one by the sizes is
+ * fastest and no longer than that), then the tile shape and steps per pass
+ * per (stencil order, size class) -- the instances of one class (order D,
+ * interior width <= 64, <= 128 or wider) try each tile shape and, at radius
+ * 1, the two-step units, while the others keep theirs -- then the z-chunk
+ * cap again. */
 b2r_status b2r_batch_autotune(b2r_batch* b, void* cuda_stream, int* best_zchunk, double* best_ms);
 
 /* ---- batched elastic-wave instances (no reference counterpart) ----------- */
