@@ -45,9 +45,13 @@ struct b2r_handle {
     int small_ctas = 0;
     double small_gain = 0;
     // several blocks, or heat on a torus: the domain as one block, which runs of
-    // many steps go to (null: no room, or already one); blocks_of: its owner
+    // many steps go to (null: none, or already one), in this handle's own buffers
+    // (step_joined) and the spare ones; blocks_of: its owner
     b2r_handle* joined = nullptr;
     const b2r_handle* blocks_of = nullptr;
+    float* spare[kMaxFields] = {};
+    int nspare = 0;
+    size_t spare_bytes = 0;      // counted in the process's share (take_spare)
     // elastic wave: fields and material
     float* fld[kMaxFields] = {};
     int nfld = 0;
@@ -184,7 +188,7 @@ void fill_layout(BlockLayout& L, const int n[3], const int B[3], const int nb[3]
                  int periodic, int fixed_edge);
 size_t field_bytes(const b2r_handle* h);
 size_t domain_cells(const b2r_handle* h);
-b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined);   // joined: a handle's one-block form
+b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, b2r_handle* owner);   // owner: of a one-block form, or null
 b2r_status ensure_kappa(b2r_handle* h);
 b2r_status ensure_staging(b2r_handle* h, size_t bytes);
 b2r_status build_heat_maps(b2r_handle* h);

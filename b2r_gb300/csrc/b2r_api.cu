@@ -551,41 +551,79 @@ bool small_runs(const b2r_handle* h, int n)
 // between exchanges: 250x186x132, radius 2, 819 / 671 / 670 / 702 us, 128^3 495 /
 // 434 / 422 / 439; radius 1, 256^3 1661 / 1065 / 885 / 1003, 120^3 436 / 345 / 328 /
 // 299; radius 3, 128^3 536 /
-// 503 / 529 / 525; radius 4, 250x100x100 650 / 587 / 639 / 660.  Made where what it
-// allocates takes at most an eighth of the free memory: two buffers for heat,
-// ten fields for the collocated wave, the material for the staggered one, whose
-// fields lie in the second field set.
-void make_joined(b2r_handle* h)
+// 503 / 529 / 525; radius 4, 250x100x100 650 / 587 / 639 / 660.  False: none.
+bool joined_config(const b2r_handle* h, b2r_config& c)
 {
-    size_t room = 0, all = 0;
-    b2r_config c = h->cfg;
+    c = h->cfg;
     for (int a = 0; a < 3; ++a) c.blocks[a] = 1;
     const int least = std::min(c.env[0], std::min(c.env[1], c.env[2]));
     c.R = 1;
     if (h->L.periodic) {
+        if (c.model != B2R_MODEL_HEAT) return false;
         const BlockLayout one = one_block(h);
         const int period = c.D >= 3 ? 2 : c.D == 1 && heat2_us(one) / 2 <= heat_rows_us(one) / 3 ? 4 : 3;
         c.R = std::max(1, std::min(period, least / 2 / c.D));
     }
-    if (h->L.nblk == 1 && c.R <= h->cfg.R) return;
-    const int nf = c.model == B2R_MODEL_HEAT ? 2 : c.model == B2R_MODEL_EQWP_REF ? 10 : 3;
-    const int H = c.R * halo_per_step(c);
-    const double cells = (double)(c.env[0] + 2 * H + 64) * (c.env[1] + 2 * H) * (c.env[2] + 2 * H);
-    if (cudaMemGetInfo(&room, &all) != cudaSuccess || 4.0 * nf * cells > (double)(room / 8)) {
-        cudaGetLastError();
-        return;
+    return h->L.nblk > 1 || c.R > h->cfg.R;
+}
+
+// It lives in the buffers of the blocks, which hold nothing else meanwhile
+// (step_joined), so these have to be large enough.  Those of heat are made so
+// (room: bytes of a buffer) where that takes a quarter more at most, which only
+// a torus with shallower halos of its own needs.  A small domain gets spare
+// buffers instead, which save moving the blocks' shells or material: 10 steps of
+// heat on 130x63x70 in 2x3x1 blocks 45 us, in the blocks' buffers 86; 12 of the
+// staggered wave on 128^3 in 2x2x2 730 and 762.  All spare buffers of a process
+// take 1 GB at most, beside one field of each collocated domain, which is updated
+// in place and cannot do without.
+constexpr size_t kSpareOne = 256u << 20, kSpareAll = 1u << 30;
+std::atomic<size_t> g_spare{0};
+// n buffers of fb bytes: all of them, or as many as there is room for
+int take_spare(b2r_handle* h, int n, size_t fb, bool all)
+{
+    while (n > 0 && n * fb > kSpareOne) n = all ? 0 : n - 1;
+    if (!n) return 0;
+    if (g_spare.fetch_add(n * fb) + n * fb > kSpareAll) {
+        g_spare.fetch_sub(n * fb);
+        return 0;
     }
-    if (create_handle(&c, &h->joined, true) != B2R_OK) {
-        h->joined = nullptr;
-        return;
+    h->spare_bytes = n * fb;
+    while (h->nspare < n && cudaMalloc(&h->spare[h->nspare], fb) == cudaSuccess) cudaMemset(h->spare[h->nspare++], 0, fb);
+    cudaGetLastError();
+    while (all && h->nspare < n && h->nspare > 0) cudaFree(h->spare[--h->nspare]), h->spare[h->nspare] = nullptr;
+    return h->nspare;
+}
+
+void make_joined(b2r_handle* h, const b2r_config& c, size_t room)
+{
+    b2r_handle* j = nullptr;
+    if (create_handle(&c, &j, h) != B2R_OK) return;
+    const size_t fb = field_bytes(j);
+    bool ok = true;
+    switch (c.model) {
+    case B2R_MODEL_HEAT:
+        if (take_spare(h, 2, fb, true))
+            for (int b = 0; b < 2; ++b) j->buf[b] = h->spare[b];
+        else
+            ok = fb <= room;
+        ok = ok && build_heat_maps(j) == B2R_OK;
+        break;
+    case B2R_MODEL_EQWP_STAG:
+        ok = fb <= room;
+        if (ok && take_spare(h, 3, fb, true))
+            for (int m = 0; m < 3; ++m) j->mat[m] = h->spare[m];
+        break;
+    default:
+        ok = fb <= room;
+        if (ok && !take_spare(h, h->nfld, fb, false)) {
+            h->nspare = cudaMalloc(&h->spare[0], fb) == cudaSuccess;
+            ok = h->nspare > 0;
+            cudaGetLastError();
+        }
+        for (int f = 0; f < h->nfld && ok; ++f) j->fld[f] = f < h->nspare ? h->spare[f] : h->fld[f - h->nspare];
     }
-    if (c.model == B2R_MODEL_EQWP_STAG && field_bytes(h->joined) > field_bytes(h)) {
-        b2r_destroy(h->joined);
-        h->joined = nullptr;
-        return;
-    }
-    h->joined->blocks_of = h;
-    h->joined->d_status = h->d_status;
+    if (ok) h->joined = j;
+    else b2r_destroy(j);
 }
 
 // The collocated wave's force patch (interior coordinates of a block) acts on
@@ -603,9 +641,12 @@ bool force_is_inside(const b2r_handle* h)
 
 // Whether a run of n steps goes to the one-block form.  Joining and splitting
 // cost about as much as eight exchanges and ragged block sweeps of heat: us for
-// 8 and 48 steps in blocks and joined, 512^3 in 2x2x2, R = 2, 1030, 6305 and
-// 1125, 4279; the torus above 212, 1242 and 162, 725; a torus of radius 4, 100^3
-// in 1x2x1, 76, 388 and 85, 366.
+// 8 and 48 steps in blocks and joined, the torus above 212, 1242 and 162, 725; a
+// torus of radius 4, 100^3 in 1x2x1, 76, 388 and 85, 366.  In the blocks' own
+// buffers twelve, for 10 and 14 steps: 512^3 in 2x2x2, R = 2, 1320, 1846 and 1474,
+// 1737 (48: 6305 and 4401), 400x360x380 torus in 2x1x1, radius 2, 1153, 1614 and
+// 1199, 1594; not where every exchange is for one step of radius 1: 400x360x380 in
+// 2x1x1, R = 1, 1022 and 707 for 10.
 // The elastic wave pays about 1.4 steps for it; us per step in blocks and joined:
 // 512x512x256 in 2x2x1, R = 2, 1547 and 1334 (even at 9 steps), 256^3 in 2x1x1,
 // R = 1, 485 and 355 (5), 128^3 in 2x2x2 90 and 51 (4), 64^3 in 2x1x1 18.8 and
@@ -614,39 +655,95 @@ bool force_is_inside(const b2r_handle* h)
 bool joins(const b2r_handle* h, int n)
 {
     if (!h->joined) return false;
-    if (h->cfg.model == B2R_MODEL_HEAT) return h->tune.own && n >= (h->L.periodic && h->cfg.D >= 3 ? 20 : 10);
+    if (h->cfg.model == B2R_MODEL_HEAT) {
+        const bool soon = h->nspare > 0 || (h->cfg.D == 1 && (h->L.periodic || h->cfg.R == 1));
+        return h->tune.own && n >= (h->L.periodic && h->cfg.D >= 3 ? 20 : soon ? 10 : 14);
+    }
     if (n < (h->L.nb[0] * h->L.nb[1] > 1 ? 12 : 24)) return false;
     if (h->cfg.model == B2R_MODEL_EQWP_REF) return force_is_inside(h);
     return !h->eqwp_fused && !h->eqwp_tma && !h->eqwp_overlap;
 }
 
+// The blocks give their storage to the one-block form for the run, where it has
+// none.  Heat: the domain goes from the current buffer into the other, steps
+// between the two, and goes back into whichever does not hold it in the end.
+// Staggered wave: the fields go into the second field set, then the material into
+// the first three fields.  Collocated wave: a group of fields into the spare
+// ones, the next group into the storage of the group before, and back in the
+// opposite order.  Storage that held something else meanwhile gets whole blocks,
+// halos and shell, on the way back, the rest its interior.
 b2r_status step_joined(b2r_handle* h, int n)
 {
-    b2r_handle* j = h->joined;
-    const int nf = std::max(1, h->nfld);
+    b2r_handle* const j = h->joined;
+    const int shell = h->shell, c = h->cur, nf = h->nfld;
+    const bool heat = h->cfg.model == B2R_MODEL_HEAT, stag = h->cfg.model == B2R_MODEL_EQWP_STAG;
+    const bool borrows = h->nspare == 0;   // heat, staggered wave
     RegridFields F{};
-    for (int f = 0; f < nf; ++f) {
-        F.m[f] = h->nfld ? h->fld[f] : static_cast<float*>(h->buf[h->cur]);
-        if (h->cfg.model == B2R_MODEL_EQWP_STAG) {
-            j->fld[f] = h->fld2[f];
-            h->fld2_stale = true;
+    auto fields = [&](int at, int count) {   // fields at .. at + count
+        for (int f = 0; f < count; ++f) {
+            F.m[f] = h->fld[at + f];
+            F.s[f] = j->fld[at + f];
         }
-        F.s[f] = h->nfld ? j->fld[f] : static_cast<float*>(j->buf[j->cur]);
-        F.s2[f] = static_cast<float*>(j->buf[1 - j->cur]);
+        return count;
+    };
+    if (heat) {
+        if (borrows) j->cur = 1 - c;
+        F.m[0] = static_cast<float*>(h->buf[c]);
+        F.s[0] = static_cast<float*>(j->buf[j->cur]);
+        F.s2[0] = borrows ? nullptr : static_cast<float*>(j->buf[1 - j->cur]);   // both buffers carry the shell
+        CK(h, launch_join(F, 1, h->L, j->L, shell, h->stream));
+        if (borrows && shell) CK(h, launch_outside(F.s[0], F.m[0], j->L, h->stream));
+    } else if (stag) {
+        for (int f = 0; f < nf; ++f) j->fld[f] = h->fld2[f];
+        h->fld2_stale = true;
+        CK(h, launch_join(F, fields(0, nf), h->L, j->L, shell, h->stream));
+        if (borrows) {
+            for (int m = 0; m < 3; ++m) {
+                F.m[m] = h->mat[m];
+                F.s[m] = j->mat[m] = h->fld[m];
+            }
+            CK(h, launch_join(F, 3, h->L, j->L, shell, h->stream));
+        }
+    } else {
+        for (int at = 0; at < nf; at += h->nspare)
+            CK(h, launch_join(F, fields(at, std::min(h->nspare, nf - at)), h->L, j->L, shell, h->stream));
     }
-    CK(h, launch_join(F, nf, h->L, j->L, h->shell, h->stream));
     j->stream = h->stream;
     j->graphs = h->graphs;
-    j->ts = h->nfld ? h->ts : 0;
+    const long long from = j->ts = nf ? h->ts : 0;
     j->halos_fresh = false;
-    if (b2r_status st = b2r_step(j, n); st != B2R_OK) return fail(h, st, "%s", j->err.c_str());
-    if (!h->nfld) F.s[0] = static_cast<float*>(j->buf[j->cur]);
-    CK(h, launch_split(F, nf, h->L, j->L, h->stream));
-    h->ts += n;
+    const b2r_status st = b2r_step(j, n);   // whatever it did goes back into the blocks
+    h->halos_lost = !(heat && borrows);     // of some field at least
+    if (heat && borrows) {
+        float* const s = F.s[0] = static_cast<float*>(j->buf[j->cur]);
+        float* const m = F.m[0] = static_cast<float*>(j->buf[1 - j->cur]);
+        CK(h, launch_split_whole(F, 1, h->L, j->L, shell, h->stream));
+        h->cur = 1 - j->cur;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(h->stream, &cap) != cudaSuccess) cudaGetLastError();
+        if (cap != cudaStreamCaptureStatusNone && h->cur != c) {   // a graph may be replayed: it ends where it began
+            CK(h, cudaMemcpyAsync(s, m, field_bytes(h), cudaMemcpyDeviceToDevice, h->stream));
+            h->cur = c;
+        } else if (shell) {
+            CK(h, launch_outside(m, s, h->L, h->stream));
+        }
+    } else if (heat) {
+        F.s[0] = static_cast<float*>(j->buf[j->cur]);
+        CK(h, launch_split(F, 1, h->L, j->L, h->stream));
+    } else if (stag) {
+        if (borrows) CK(h, launch_split_whole(F, fields(0, 3), h->L, j->L, shell, h->stream));
+        const int first = borrows ? 3 : 0;
+        CK(h, launch_split(F, fields(first, nf - first), h->L, j->L, h->stream));
+    } else {
+        int at = (nf - 1) / h->nspare * h->nspare;
+        CK(h, launch_split(F, fields(at, nf - at), h->L, j->L, h->stream));
+        while ((at -= h->nspare) >= 0)
+            CK(h, launch_split_whole(F, fields(at, h->nspare), h->L, j->L, shell, h->stream));
+    }
+    h->ts += j->ts - from;
     h->upmask = 0;
-    h->halos_fresh = false;
-    h->halos_lost = true;   // the interiors are current, the halos are not
-    return B2R_OK;
+    h->halos_fresh = !h->halos_lost && h->ts % h->cfg.R == 0;
+    return st == B2R_OK ? st : fail(h, st, "%s", j->err.c_str());
 }
 
 // Game of Life over several generations runs on the domain's bit grid unless
@@ -744,7 +841,7 @@ bool make_block_tmap(CUtensorMap* map, const void* base, const BlockLayout& L, i
 
 namespace b2r_api {
 
-b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined)
+b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, b2r_handle* owner)
 {
     if (!cfg || !out) return fail(nullptr, B2R_ERR_ARG, "null argument");
     *out = nullptr;
@@ -781,6 +878,7 @@ b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined)
     b2r_handle* h = new (std::nothrow) b2r_handle();
     if (!h) return fail(nullptr, B2R_ERR_OOM, "host allocation failed");
     h->cfg = c;
+    h->blocks_of = owner;
     h->cell_bytes = (c.model == B2R_MODEL_GOL) ? 1 : 4;
     h->shell = (c.boundary == B2R_BC_PERIODIC) ? 0 : halo_per_step(c) / (c.model >= B2R_MODEL_EQWP_REF ? 2 : 1);
     int n[3];
@@ -793,16 +891,46 @@ b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined)
         cudaGetLastError();   // a failed allocation must not surface in the caller's next launch check
         return s;
     };
-    if (!joined) {                       // a one-block form reports to its owner's
-        if (cudaMalloc(&h->d_status, sizeof(int)) != cudaSuccess)
-            return bail(fail(nullptr, B2R_ERR_CUDA, "cudaMalloc(status) failed"));
-        cudaMemset(h->d_status, 0, sizeof(int));
+    if (owner) {                       // a one-block form has its owner's memory and status word
+        h->d_status = owner->d_status;
+        if (c.model == B2R_MODEL_HEAT) {
+            h->hc = owner->hc;
+            for (int b = 0; b < 2; ++b) h->buf[b] = owner->buf[b];
+            std::lock_guard<std::mutex> lock(g_tune_mu);
+            auto it = g_tune_cache.find(key_of(h));
+            if (it != g_tune_cache.end()) h->tune = it->second;
+        } else {
+            h->nfld = owner->nfld;
+        }
+        *out = h;
+        return B2R_OK;
     }
+    if (cudaMalloc(&h->d_status, sizeof(int)) != cudaSuccess)
+        return bail(fail(nullptr, B2R_ERR_CUDA, "cudaMalloc(status) failed"));
+    cudaMemset(h->d_status, 0, sizeof(int));
     const size_t fb = field_bytes(h);
+    b2r_config jc;
     if (c.model == B2R_MODEL_HEAT || c.model == B2R_MODEL_GOL) {
+        bool join = false;
+        size_t room = fb;
+        if (c.model == B2R_MODEL_HEAT) {
+            make_small(h);
+            join = !h->small_ctas && joined_config(h, jc);
+            if (join) {
+                BlockLayout one;
+                const int JH = jc.R * c.D, nb[3] = {1, 1, 1}, jn[3] = {c.env[0] + 2 * JH, c.env[1] + 2 * JH, c.env[2] + 2 * JH};
+                fill_layout(one, jn, c.env, nb, JH, 4, h->L.periodic, -1);
+                const size_t need = (size_t)one.bstride * sizeof(float);
+                if (2 * need > kSpareOne && need <= fb + fb / 4) room = std::max(fb, need);
+            }
+        }
         for (int b = 0; b < 2; ++b) {
-            if (cudaMalloc(&h->buf[b], fb) != cudaSuccess)
-                return bail(fail(nullptr, B2R_ERR_OOM, "cudaMalloc of %zu bytes failed", fb));
+            if (room == fb || cudaMalloc(&h->buf[b], room) != cudaSuccess) {
+                cudaGetLastError();
+                room = fb;
+                if (cudaMalloc(&h->buf[b], fb) != cudaSuccess)
+                    return bail(fail(nullptr, B2R_ERR_OOM, "cudaMalloc of %zu bytes failed", fb));
+            }
             cudaMemset(h->buf[b], 0, fb);
         }
         if (c.model == B2R_MODEL_GOL &&
@@ -821,12 +949,11 @@ b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined)
                 g_err = h->err;
                 return bail(st);
             }
-            if (!joined) make_small(h);
-            if (!joined && !h->small_ctas && (h->L.nblk > 1 || h->L.periodic)) make_joined(h);
+            if (join) make_joined(h, jc, room);
         }
     } else {
         h->nfld = (c.model == B2R_MODEL_EQWP_REF) ? 10 : 9;
-        for (int f = 0; f < h->nfld && !(joined && c.model == B2R_MODEL_EQWP_STAG); ++f) {
+        for (int f = 0; f < h->nfld; ++f) {
             if (cudaMalloc(&h->fld[f], fb) != cudaSuccess)
                 return bail(fail(nullptr, B2R_ERR_OOM, "cudaMalloc of %zu bytes failed", fb));
             cudaMemset(h->fld[f], 0, fb);
@@ -837,20 +964,20 @@ b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined)
                     return bail(fail(nullptr, B2R_ERR_OOM, "cudaMalloc of %zu bytes failed", fb));
                 cudaMemset(h->mat[m], 0, fb);
             }
-            for (int f = 0; f < h->nfld && !joined; ++f) {
+            for (int f = 0; f < h->nfld; ++f) {
                 if (cudaMalloc(&h->fld2[f], fb) != cudaSuccess)
                     return bail(fail(nullptr, B2R_ERR_OOM, "cudaMalloc of %zu bytes failed", fb));
                 cudaMemset(h->fld2[f], 0, fb);
             }
             const int box = eqwp_fused_box();
-            for (int f = 0; f < 6 && !joined; ++f)
+            for (int f = 0; f < 6; ++f)
                 if (!make_block_tmap(&h->smaps[0].m[f], h->fld[B2R_F_SXX + f], h->L, 4, box, box, 1) ||
                     !make_block_tmap(&h->smaps[1].m[f], h->fld2[B2R_F_SXX + f], h->L, 4, box, box, 1))
                     return bail(fail(nullptr, B2R_ERR_CUDA, "cuTensorMapEncodeTiled failed"));
         }
-        if (!joined && h->L.nblk > 1 && !h->L.periodic) make_joined(h);
+        if (joined_config(h, jc)) make_joined(h, jc, fb);
     }
-    if (!joined && cudaDeviceSynchronize() != cudaSuccess)
+    if (cudaDeviceSynchronize() != cudaSuccess)
         return bail(fail(nullptr, B2R_ERR_CUDA, "device initialisation failed"));
     *out = h;
     return B2R_OK;
@@ -860,18 +987,20 @@ b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, bool joined)
 
 extern "C" {
 
-b2r_status b2r_create(const b2r_config* cfg, b2r_handle** out) { return create_handle(cfg, out, false); }
+b2r_status b2r_create(const b2r_config* cfg, b2r_handle** out) { return create_handle(cfg, out, nullptr); }
 
 b2r_status b2r_destroy(b2r_handle* h)
 {
     if (!h) return B2R_OK;
-    if (h->joined) {
-        h->joined->d_status = nullptr;   // this handle's
-        if (h->cfg.model == B2R_MODEL_EQWP_STAG)
-            for (float*& f : h->joined->fld) f = nullptr;   // so are these
-        b2r_destroy(h->joined);
-    }
     drop_graphs(h);
+    if (h->blocks_of) {   // a one-block form: the memory is its owner's
+        delete h;
+        return B2R_OK;
+    }
+    b2r_destroy(h->joined);
+    for (float* p : h->spare)
+        if (p) cudaFree(p);
+    g_spare.fetch_sub(h->spare_bytes);
     if (h->adj_ws) cudaFree(h->adj_ws);
     for (int b = 0; b < 2; ++b)
         if (h->buf[b]) cudaFree(h->buf[b]);
@@ -972,7 +1101,7 @@ b2r_status b2r_upload(b2r_handle* h, int field, const void* src, int src_is_devi
     void* dst2 = nullptr;   // written with the same cells in the same pass
     if (is_mat) {
         dst = h->mat[field - B2R_F_LAMBDA];
-        if (h->joined)
+        if (h->joined && h->nspare)
             CK(h, launch_scatter<float>(static_cast<const float*>(dsrc), h->joined->mat[field - B2R_F_LAMBDA], nullptr,
                                         h->joined->L, h->shell, h->stream));
     } else if (eq) {

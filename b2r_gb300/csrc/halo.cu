@@ -253,23 +253,22 @@ gather_kernel(T* __restrict__ dom, const T* __restrict__ blocks, const BlockLayo
 
 // ---------------------------------------------------------------- blocks <-> one block
 // Domain cells between the blocks of layout M and one block of layout S that
-// holds the whole domain (same interior, same fixed shell or torus).  JOIN:
-// every cell, shell included, from M to S, the shell also into S's second
-// buffer if it has one; else the interior from S to M.  blockIdx.y: field.  A
-// warp copies one row, x-block by x-block, four loads in flight per lane.
-template <bool JOIN>
+// holds the whole domain (same interior, same fixed shell or torus); blockIdx.y:
+// field.  Join: every cell, shell included, the shell also into s2 unless that is
+// null; a warp per row, x-block by x-block, four loads in flight per lane.
+template <bool TWO>
 __global__ void __launch_bounds__(kRowWarps * 32)
-regrid_kernel(const RegridFields F, const BlockLayout M, const BlockLayout S, int shell)
+join_kernel(const RegridFields F, const BlockLayout M, const BlockLayout S, int shell)
 {
-    float* const m = F.m[blockIdx.y];
+    const float* const m = F.m[blockIdx.y];
     float* const s = F.s[blockIdx.y];
-    float* const s2 = F.s2[blockIdx.y];
-    const int lane = threadIdx.x & 31, edge = JOIN ? shell : 0;
+    float* const s2 = TWO ? F.s2[blockIdx.y] : nullptr;
+    const int lane = threadIdx.x & 31;
     const int e0 = S.B[0], e1 = S.B[1], e2 = S.B[2];
-    const long long rows = (long long)(e1 + 2 * edge) * (e2 + 2 * edge);
+    const long long rows = (long long)(e1 + 2 * shell) * (e2 + 2 * shell);
     for (long long r = (long long)blockIdx.x * kRowWarps + (threadIdx.x >> 5); r < rows;
          r += (long long)gridDim.x * kRowWarps) {
-        const int g1 = (int)(r % (e1 + 2 * edge)) - edge, g2 = (int)(r / (e1 + 2 * edge)) - edge;
+        const int g1 = (int)(r % (e1 + 2 * shell)) - shell, g2 = (int)(r / (e1 + 2 * shell)) - shell;
         const bool out = g1 < 0 || g1 >= e1 || g2 < 0 || g2 >= e2;      // a row of the shell
         const int b1 = owner_of(g1, M.B[1], M.nb[1]), b2 = owner_of(g2, M.B[2], M.nb[2]);
         const long long so = (long long)(g2 + S.H) * S.plane + (long long)(g1 + S.H) * S.P + S.xoff + S.H;
@@ -277,28 +276,159 @@ regrid_kernel(const RegridFields F, const BlockLayout M, const BlockLayout S, in
                              M.xoff + M.H;
         const int blk_yz = M.nb[0] * (b1 + M.nb[1] * b2);
         for (int b0 = 0; b0 < M.nb[0]; ++b0) {
-            const int lo = b0 == 0 ? -edge : b0 * M.B[0];
-            const int hi = b0 == M.nb[0] - 1 ? e0 + edge : (b0 + 1) * M.B[0];
+            const int lo = b0 == 0 ? -shell : b0 * M.B[0];
+            const int hi = b0 == M.nb[0] - 1 ? e0 + shell : (b0 + 1) * M.B[0];
             const long long o = (blk_yz + b0) * M.bstride + mo - (long long)b0 * M.B[0];
             for (int xb = lo; xb < hi; xb += 32 * kRowUnroll) {
                 float v[kRowUnroll];
 #pragma unroll
                 for (int u = 0; u < kRowUnroll; ++u) {
                     const int x = xb + u * 32 + lane;
-                    v[u] = x < hi ? (JOIN ? m[o + x] : s[so + x]) : 0.f;
+                    v[u] = x < hi ? m[o + x] : 0.f;
                 }
 #pragma unroll
                 for (int u = 0; u < kRowUnroll; ++u) {
                     const int x = xb + u * 32 + lane;
                     if (x >= hi) continue;
-                    if (JOIN) {
-                        s[so + x] = v[u];
-                        if (s2 && (out || x < 0 || x >= e0)) s2[so + x] = v[u];
-                    } else {
-                        m[o + x] = v[u];
-                    }
+                    s[so + x] = v[u];
+                    if (TWO && (out || x < 0 || x >= e0)) s2[so + x] = v[u];
                 }
             }
+        }
+    }
+}
+// Split, interiors: the way back, as join.
+__global__ void __launch_bounds__(kRowWarps * 32)
+split_kernel(const RegridFields F, const BlockLayout M, const BlockLayout S)
+{
+    float* const m = F.m[blockIdx.y];
+    const float* const s = F.s[blockIdx.y];
+    const int lane = threadIdx.x & 31;
+    const long long rows = (long long)S.B[1] * S.B[2];
+    for (long long r = (long long)blockIdx.x * kRowWarps + (threadIdx.x >> 5); r < rows;
+         r += (long long)gridDim.x * kRowWarps) {
+        int g1;
+        const int g2 = (int)div_row(r, S.B[1], g1);
+        const int b1 = owner_of(g1, M.B[1], M.nb[1]), b2 = owner_of(g2, M.B[2], M.nb[2]);
+        const long long so = (long long)(g2 + S.H) * S.plane + (long long)(g1 + S.H) * S.P + S.xoff + S.H;
+        const long long mo = (long long)(g2 - b2 * M.B[2] + M.H) * M.plane + (long long)(g1 - b1 * M.B[1] + M.H) * M.P +
+                             M.xoff + M.H;
+        const int blk_yz = M.nb[0] * (b1 + M.nb[1] * b2);
+        for (int b0 = 0; b0 < M.nb[0]; ++b0) {
+            const int lo = b0 * M.B[0], hi = lo + M.B[0];
+            const long long o = (blk_yz + b0) * M.bstride + mo - lo;
+            for (int xb = lo; xb < hi; xb += 32 * kRowUnroll) {
+                float v[kRowUnroll];
+#pragma unroll
+                for (int u = 0; u < kRowUnroll; ++u) {
+                    const int x = xb + u * 32 + lane;
+                    v[u] = x < hi ? s[so + x] : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < kRowUnroll; ++u) {
+                    const int x = xb + u * 32 + lane;
+                    if (x < hi) m[o + x] = v[u];
+                }
+            }
+        }
+    }
+}
+// Split, whole: the padded blocks, halos and shell as an upload fills them.  A
+// warp per row: the interior, which starts on 128 bytes, and as many cells as the
+// halo, rounded up to 8, on each side, so that whole sectors are written (the
+// row's padding holds nothing).
+__global__ void __launch_bounds__(kRowWarps * 32)
+split_whole_kernel(const RegridFields F, const BlockLayout M, const BlockLayout S, int shell)
+{
+    float* const m = F.m[blockIdx.y];
+    const float* const s = F.s[blockIdx.y] + S.H * (S.plane + S.P + 1) + S.xoff;   // cell (0, 0, 0)
+    const int lane = threadIdx.x & 31, end = (M.H + 7) & ~7;
+    const int e0 = S.B[0], e1 = S.B[1], e2 = S.B[2];
+    const long long rows = (long long)M.n[1] * M.n[2] * M.nblk;
+    for (long long r = (long long)blockIdx.x * kRowWarps + (threadIdx.x >> 5); r < rows;
+         r += (long long)gridDim.x * kRowWarps) {
+        int y, z;
+        const int blk = (int)div_row(div_row(r, M.n[1], y), M.n[2], z);
+        const int b0 = blk % M.nb[0], b1 = (blk / M.nb[0]) % M.nb[1], b2 = blk / (M.nb[0] * M.nb[1]);
+        int g1 = b1 * M.B[1] + y - M.H, g2 = b2 * M.B[2] + z - M.H;
+        if (M.periodic) {
+            g1 = wrap_once(g1, e1);
+            g2 = wrap_once(g2, e2);
+        }
+        // outside the domain and its shell (none on a torus) a block row holds zeros
+        const bool has = g1 >= -shell && g1 < e1 + shell && g2 >= -shell && g2 < e2 + shell;
+        const float* const row = s + g2 * S.plane + (long long)g1 * S.P;
+        float* const out = m + blk * M.bstride + (long long)z * M.plane + (long long)y * M.P + M.xoff + M.H;
+        const int x0 = b0 * M.B[0];
+        float v[kRowUnroll], w[2];
+        auto end_cell = [&](int i) { return i < end ? i - end : M.B[0] + i - end; };   // of the block, i < 2 end
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = u * 32 + lane, x = end_cell(i);
+            int g0 = x0 + x;
+            if (M.periodic) g0 = wrap_once(g0, e0);
+            w[u] = has && i < 2 * end && x >= -M.H && x < M.B[0] + M.H && g0 >= -shell && g0 < e0 + shell ? row[g0] : 0.f;
+        }
+        for (int xb = 0; xb < M.B[0]; xb += 32 * kRowUnroll) {
+#pragma unroll
+            for (int u = 0; u < kRowUnroll; ++u) {
+                const int x = xb + u * 32 + lane;
+                v[u] = has && x < M.B[0] ? row[x0 + x] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < kRowUnroll; ++u) {
+                const int x = xb + u * 32 + lane;
+                if (x < M.B[0]) out[x] = v[u];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (u * 32 + lane < 2 * end) out[end_cell(u * 32 + lane)] = w[u];
+        for (int i = 64 + lane; i < 2 * end; i += 32) {   // halos of more than 32 cells
+            const int x = end_cell(i);
+            int g0 = x0 + x;
+            if (M.periodic) g0 = wrap_once(g0, e0);
+            out[x] = has && x >= -M.H && x < M.B[0] + M.H && g0 >= -shell && g0 < e0 + shell ? row[g0] : 0.f;
+        }
+    }
+}
+// The cells of the blocks outside the domain's interior from src to dst: whole
+// rows beyond the y and z faces (a warp each), and whole 8-cell groups of the
+// others' ends (a lane a row; the groups hold halo and padding alone, but for one
+// that the interior may end in).
+__global__ void __launch_bounds__(kRowWarps * 32)
+outside_kernel(const float* __restrict__ src, float* __restrict__ dst, const BlockLayout M)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long rows = (long long)M.n[1] * M.n[2] * M.nblk;
+    auto find = [&](long long r, int& edge, bool& out) {   // element of the row's cell x = 0
+        int y, z;
+        const int blk = (int)div_row(div_row(r, M.n[1], y), M.n[2], z);
+        edge = edge_bits(M, blk);
+        out = ((edge & 4) && y < M.H) || ((edge & 8) && y >= M.H + M.B[1]) || ((edge & 16) && z < M.H) ||
+              ((edge & 32) && z >= M.H + M.B[2]);
+        return blk * M.bstride + (long long)z * M.plane + (long long)y * M.P + M.xoff;
+    };
+    int edge;
+    bool out;
+    for (long long r = (long long)blockIdx.x * kRowWarps + warp; r < rows; r += (long long)gridDim.x * kRowWarps) {
+        const long long o = find(r, edge, out);
+        if (out)
+            for (int x = lane; x < M.n[0]; x += 32) dst[o + x] = src[o + x];
+    }
+    const int end = (M.H + 7) & ~7;
+    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < rows;
+         r += (long long)gridDim.x * blockDim.x) {
+        const long long o = find(r, edge, out) + M.H;
+        if (out) continue;
+        if (edge & 1)
+            for (int x = -end; x < 0; x += 4)
+                *reinterpret_cast<float4*>(dst + o + x) = *reinterpret_cast<const float4*>(src + o + x);
+        if (edge & 2) {
+            int x = M.B[0];
+            for (; x & 3; ++x) dst[o + x] = src[o + x];
+            for (const int stop = (M.B[0] + M.H + 7) & ~7; x < stop; x += 4)
+                *reinterpret_cast<float4*>(dst + o + x) = *reinterpret_cast<const float4*>(src + o + x);
         }
     }
 }
@@ -532,7 +662,8 @@ cudaError_t launch_join(const RegridFields& F, int nf, const BlockLayout& M, con
                         cudaStream_t st)
 {
     const long long rows = (long long)(S.B[1] + 2 * shell) * (S.B[2] + 2 * shell);
-    regrid_kernel<true><<<dim3(grid_for(rows * 32, kRowWarps * 32), nf), kRowWarps * 32, 0, st>>>(F, M, S, shell);
+    const auto kernel = F.s2[0] ? join_kernel<true> : join_kernel<false>;
+    kernel<<<dim3(grid_for(rows * 32, kRowWarps * 32), nf), kRowWarps * 32, 0, st>>>(F, M, S, shell);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -540,7 +671,24 @@ cudaError_t launch_join(const RegridFields& F, int nf, const BlockLayout& M, con
 cudaError_t launch_split(const RegridFields& F, int nf, const BlockLayout& M, const BlockLayout& S, cudaStream_t st)
 {
     const long long rows = (long long)S.B[1] * S.B[2];
-    regrid_kernel<false><<<dim3(grid_for(rows * 32, kRowWarps * 32), nf), kRowWarps * 32, 0, st>>>(F, M, S, 0);
+    split_kernel<<<dim3(grid_for(rows * 32, kRowWarps * 32), nf), kRowWarps * 32, 0, st>>>(F, M, S);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_split_whole(const RegridFields& F, int nf, const BlockLayout& M, const BlockLayout& S, int shell,
+                               cudaStream_t st)
+{
+    const long long rows = (long long)M.n[1] * M.n[2] * M.nblk;
+    split_whole_kernel<<<dim3(grid_for(rows * 32, kRowWarps * 32), nf), kRowWarps * 32, 0, st>>>(F, M, S, shell);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_outside(const float* src, float* dst, const BlockLayout& M, cudaStream_t st)
+{
+    const long long rows = (long long)M.n[1] * M.n[2] * M.nblk;
+    outside_kernel<<<grid_for(rows * 32, kRowWarps * 32), kRowWarps * 32, 0, st>>>(src, dst, M);
     count_launches(1);
     return cudaGetLastError();
 }

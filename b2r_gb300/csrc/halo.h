@@ -36,8 +36,12 @@ cudaError_t launch_gather(T* dom, const T* blocks, const BlockLayout& L, int she
                           cudaStream_t st);
 
 // nf fields of a domain between the blocks of layout M (m) and one block of
-// layout S that holds the whole domain (s): every cell into S, its shell also
-// into the second buffer s2 unless that is null, and the interior back.
+// layout S that holds the whole domain (s).  launch_join: every cell, the fixed
+// shell included, into S (what lies beyond is left as it is), and the shell into
+// s2 unless that is null; launch_split: the
+// interiors back; launch_split_whole: every cell of the padded blocks, halos and
+// shell as an upload fills them.  launch_outside: the cells of the blocks
+// outside the domain's interior from src to dst.
 struct RegridFields {
     float* m[kMaxFields];
     float* s[kMaxFields];
@@ -46,5 +50,8 @@ struct RegridFields {
 cudaError_t launch_join(const RegridFields& F, int nf, const BlockLayout& M, const BlockLayout& S, int shell,
                         cudaStream_t st);
 cudaError_t launch_split(const RegridFields& F, int nf, const BlockLayout& M, const BlockLayout& S, cudaStream_t st);
+cudaError_t launch_split_whole(const RegridFields& F, int nf, const BlockLayout& M, const BlockLayout& S, int shell,
+                               cudaStream_t st);
+cudaError_t launch_outside(const float* src, float* dst, const BlockLayout& M, cudaStream_t st);
 
 }  // namespace b2r

@@ -80,7 +80,9 @@ typedef struct b2r_handle b2r_handle;
 
 /* ---- life cycle ------------------------------------------------------- */
 /* Validates cfg as simu_env_init does (b2r.cpp:47-67, 154-159) and allocates
- * every device field.  Replaces b2r_sync_init (b2r_halo_sync.cu:74) and
+ * every device field: the blocks, and for long runs on the domain as one block
+ * (see TBLOCK) one field more (collocated wave) or, in small domains, spare
+ * buffers, 1 GB at most over all handles.  Replaces b2r_sync_init (b2r_halo_sync.cu:74) and
  * eqwp_cuda_init (eqwp.cu:515). */
 b2r_status b2r_create(const b2r_config* cfg, b2r_handle** out);
 /* Replaces b2r_sync_finalize (b2r_halo_sync.cu:121) / eqwp_cuda_finalize
