@@ -107,7 +107,7 @@ struct AdjS {
     float* g_mu;
     float k;
     // the residuals of step n-1, added to vb_y at the receivers (rec: element
-    // offsets) by the first CTA: the stress adjoint does not touch vb, and a
+    // offsets) by the first CTAs: the stress adjoint does not touch vb, and a
     // launch of its own took 2.5 us of a 150 us reverse step at 128^3
     float* vby;
     const long long* rec;
@@ -116,8 +116,9 @@ struct AdjS {
 };
 __device__ __forceinline__ void inject(const AdjS& A)
 {
-    if (blockIdx.x || blockIdx.y || blockIdx.z) return;
-    for (int r = threadIdx.y * blockDim.x + threadIdx.x; r < A.nrec; r += blockDim.x * blockDim.y)
+    const long long threads = blockDim.x * blockDim.y;
+    for (long long r = grid_cta() * threads + threadIdx.y * blockDim.x + threadIdx.x; r < A.nrec;
+         r += threads * gridDim.x * gridDim.y * gridDim.z)
         atomicAdd(&A.vby[A.rec[r]], A.res[r]);
 }
 

@@ -342,6 +342,12 @@ __device__ __forceinline__ void st4(float* f, const Cell& c, const float (&v)[4]
     }
 }
 
+// the CTA's number in the launch
+__device__ __forceinline__ long long grid_cta()
+{
+    return blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
+}
+
 // Tile origin of a stage launch: the first tile starts at the lowest window
 // cell of any block (x rounded down to a float4 boundary), so that no tile
 // column or row lies wholly outside every window.

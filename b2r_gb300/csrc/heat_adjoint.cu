@@ -15,7 +15,7 @@
 // u^n is replayed from checkpoints every K steps.
 //
 // Measured (radius 2, 160x144x128, 200 steps, checkpoints every 50, 64
-// receivers, the whole gradient call): 10.1 ms, from 61 with a thread per
+// receivers, the whole gradient call): 9.1 ms, from 61 with a thread per
 // column over the whole z axis, the reverse step in two sweeps, and a
 // separate launch for every receiver sample.
 #include <algorithm>
@@ -84,9 +84,12 @@ heat_kappa_step_kernel(const float* __restrict__ in, float* __restrict__ out, co
                        float* __restrict__ rec_out)
 {
     pdl_begin();
-    if (rec_out && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
-        for (int r = threadIdx.y * blockDim.x + threadIdx.x; r < nrec; r += blockDim.x * blockDim.y)
+    if (rec_out) {
+        const long long threads = blockDim.x * blockDim.y;
+        for (long long r = grid_cta() * threads + threadIdx.y * blockDim.x + threadIdx.x; r < nrec;
+             r += threads * gridDim.x * gridDim.y * gridDim.z)
             rec_out[r] = in[rec[r]];
+    }
     const Win w = window(L, 0, blockIdx.z, T.nzc, L.H);
     Cell cell;
     if (!cell_setup(L, w, 0, cell, T.x0, T.y0)) return;
@@ -161,16 +164,21 @@ heat_adj_step_kernel(float* __restrict__ lam, const float* __restrict__ y, float
     }
 }
 
-// The residuals of a step into lam at the receivers, and y = kappa lam there
-// (one CTA: receivers that share a cell are all added before y is formed).
-__global__ void heat_adj_inject_kernel(float* lam, float* y, const float* kappa, const long long* rec, int nrec,
-                                       const float* res)
+// The residuals of a step into lam at the receivers, and y = kappa lam there:
+// receivers that share a cell are all added before y is formed, by a barrier
+// where one CTA does both, by two launches where there are many receivers (on
+// 128^3, 40 steps, the whole gradient with one CTA for this and the samples, and
+// now: 16384 receivers 4.4 and 2.1 ms, 262144 58 and 17).
+constexpr int kInjectCta = 1024;
+template <bool ADD, bool FORM>
+__global__ void __launch_bounds__(kInjectCta)
+heat_adj_inject_kernel(float* lam, float* y, const float* kappa, const long long* rec, int nrec, const float* res)
 {
     pdl_begin();
-    for (int r = threadIdx.x; r < nrec; r += blockDim.x) atomicAdd(&lam[rec[r]], res[r]);
-    __syncthreads();
-    for (int r = threadIdx.x; r < nrec; r += blockDim.x)
-        y[rec[r]] = __fmul_rn(kappa[rec[r]], *(volatile float*)&lam[rec[r]]);
+    const int r = blockIdx.x * kInjectCta + threadIdx.x;
+    if (ADD && r < nrec) atomicAdd(&lam[rec[r]], res[r]);
+    if (ADD && FORM) __syncthreads();
+    if (FORM && r < nrec) y[rec[r]] = __fmul_rn(kappa[rec[r]], *(volatile float*)&lam[rec[r]]);
 }
 
 // The fixed shell of `src` (the D cells around the window on every axis, the
@@ -289,8 +297,12 @@ cudaError_t launch_heat_adjoint_step(float* lam, const float* y, float* y_next, 
 cudaError_t launch_heat_adjoint_inject(float* lam, float* y, const float* kappa, const long long* rec, int nrec,
                                        const float* res, cudaStream_t st)
 {
-    return launch_pdl(heat_adj_inject_kernel, 1, std::min(1024, (nrec + 31) / 32 * 32), 0, st, lam, y, kappa, rec, nrec,
-                      res);
+    const int ctas = (nrec + kInjectCta - 1) / kInjectCta;
+    if (ctas == 1)
+        return launch_pdl(heat_adj_inject_kernel<true, true>, 1, (nrec + 31) / 32 * 32, 0, st, lam, y, kappa, rec, nrec, res);
+    if (cudaError_t e = launch_pdl(heat_adj_inject_kernel<true, false>, ctas, kInjectCta, 0, st, lam, y, kappa, rec, nrec, res))
+        return e;
+    return launch_pdl(heat_adj_inject_kernel<false, true>, ctas, kInjectCta, 0, st, lam, y, kappa, rec, nrec, res);
 }
 
 cudaError_t launch_heat_shell(const float* src, float* dst, long long stride, int n, const BlockLayout& L, int D,
