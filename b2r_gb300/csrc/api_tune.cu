@@ -11,18 +11,18 @@ b2r_status b2r_set_tuning(b2r_handle* h, int key, int value)
 {
     if (!h) return fail(nullptr, B2R_ERR_ARG, "null handle");
     switch (key) {
-    case B2R_TUNE_ZCHUNK: h->tune.zchunk = value; h->tune.own = false; break;
-    case B2R_TUNE_CTAS_PER_SM: h->tune.ctas_per_sm = value; h->tune.own = false; break;
-    case B2R_TUNE_PDL: h->tune.pdl = value != 0; h->tune.own = false; break;
-    case B2R_TUNE_TBLOCK: h->tune.tblock = value; h->tune.own = false; break;
-    case B2R_TUNE_ZCHUNK2: h->tune.zchunk2 = value; h->tune.own = false; break;
+    case B2R_TUNE_ZCHUNK: h->tune.zchunk = value; break;
+    case B2R_TUNE_CTAS_PER_SM: h->tune.ctas_per_sm = value; break;
+    case B2R_TUNE_PDL: h->tune.pdl = value != 0; break;
+    case B2R_TUNE_TBLOCK: h->tune.tblock = value; break;
+    case B2R_TUNE_ZCHUNK2: h->tune.zchunk2 = value; break;
     case B2R_TUNE_EQWP_FUSED: h->eqwp_fused = value != 0; break;
     case B2R_TUNE_GOL_BYTES: h->gol_bytes = value != 0; break;
     case B2R_TUNE_ADJ_FUSED: h->adj_fused = value != 0; break;
     case B2R_TUNE_GOL_PUSH: h->gol_push = value != 0; break;
-    case B2R_TUNE_TB16: h->tune.tb16 = value != 0; h->tune.own = false; break;
-    case B2R_TUNE_TB_NARROW: h->tune.tbn = value != 0; h->tune.own = false; break;
-    case B2R_TUNE_TB_R2: h->tune.r2 = value != 0; h->tune.own = false; break;
+    case B2R_TUNE_TB16: h->tune.tb16 = value != 0; break;
+    case B2R_TUNE_TB_NARROW: h->tune.tbn = value != 0; break;
+    case B2R_TUNE_TB_R2: h->tune.r2 = value != 0; break;
     case B2R_TUNE_EQWP_TMA: h->eqwp_tma = value != 0; break;
     case B2R_TUNE_EQWP_OVERLAP: h->eqwp_overlap = value != 0; break;
     case B2R_TUNE_GOL_ROWS: h->gol_rows = value < 0 ? 0 : value; break;
@@ -278,7 +278,6 @@ b2r_status b2r_autotune(b2r_handle* h, int trial_steps, int best[3], double* bes
         h->tune.tb16 = cd.tb16;
         h->tune.tbn = cd.tbn;
         h->tune.r2 = cd.r2;
-        h->tune.own = cd.tb == 0;
         h->tune.tblock = cd.tb == 0 ? 2 : cd.tb;
         h->tune.zchunk2 = cd.zc2;
         h->tune.zchunk = cd.zc;

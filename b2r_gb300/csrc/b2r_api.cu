@@ -139,7 +139,7 @@ int heat_own_steps(const b2r_handle* h)
 int heat_max_pass_steps(const b2r_handle* h)
 {
     if (h->cfg.model != B2R_MODEL_HEAT || h->tune.tblock < 2) return 1;
-    if (h->cfg.D == 1) return h->tune.own ? heat_own_steps(h) : std::min(h->tune.tblock, 4);
+    if (h->cfg.D == 1) return h->tune.own() ? heat_own_steps(h) : std::min(h->tune.tblock, 4);
     return h->cfg.D == 2 && h->tune.r2 ? 2 : 1;
 }
 
@@ -321,7 +321,7 @@ b2r_status substep(b2r_handle* h, int i, bool xnext)
     h->upmask = 0;
     switch (h->cfg.model) {
     case B2R_MODEL_HEAT:
-        if (h->tune.own)
+        if (h->tune.own())
             CK(h, launch_heat_far(h->tmapf[h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L, h->cfg.D, i, h->hc,
                                   h->d_status, h->stream));
         else
@@ -486,7 +486,7 @@ b2r_status advance(b2r_handle* h, int n)
                 CK(h, launch_heat_substep_tb2(&h->tmap3[h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L, i,
                                               h->hc, h->d_status, h->stream, h->tune.zchunk2));
                 h->cur = 1 - h->cur;
-            } else if (h->tune.own && heat_own_steps(h) > 2) {
+            } else if (h->tune.own() && heat_own_steps(h) > 2) {
                 CK(h, launch_heat_rows(k, &h->tmapr[k - 2][h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L, i,
                                        h->hc, h->d_status, h->stream));
                 h->cur = 1 - h->cur;
@@ -540,7 +540,7 @@ void make_small(b2r_handle* h)
 // exchanges and ragged sweeps of several blocks or a torus save.
 bool small_runs(const b2r_handle* h, int n)
 {
-    return h->small_ctas && h->tune.own && n >= 4 && (h->L.nblk > 1 || h->L.periodic || n * h->small_gain > 8.0);
+    return h->small_ctas && h->tune.own() && n >= 4 && (h->L.nblk > 1 || h->L.periodic || n * h->small_gain > 8.0);
 }
 
 // The one-block form of a domain of several blocks, or of a heat domain on a
@@ -657,7 +657,7 @@ bool joins(const b2r_handle* h, int n)
     if (!h->joined) return false;
     if (h->cfg.model == B2R_MODEL_HEAT) {
         const bool soon = h->nspare > 0 || (h->cfg.D == 1 && (h->L.periodic || h->cfg.R == 1));
-        return h->tune.own && n >= (h->L.periodic && h->cfg.D >= 3 ? 20 : soon ? 10 : 14);
+        return h->tune.own() && n >= (h->L.periodic && h->cfg.D >= 3 ? 20 : soon ? 10 : 14);
     }
     if (n < (h->L.nb[0] * h->L.nb[1] > 1 ? 12 : 24)) return false;
     if (h->cfg.model == B2R_MODEL_EQWP_REF) return force_is_inside(h);

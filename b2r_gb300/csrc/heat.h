@@ -47,13 +47,18 @@ struct HeatTune {
     int zchunk = 0;        // output planes per work unit; 0 = 16 (fewer for small grids)
     int ctas_per_sm = 0;   // 0 = one CTA per unit; k > 0 = persistent, k CTAs per SM
     int pdl = 1;           // programmatic dependent launch on the stream
-    bool own = true;       // the library's own rule for the kernel (heat_far.cu, on large blocks of radius 1
-                           // heat_rows.cu) and the steps per pass; false once one of the knobs below is set
     int tblock = 2;        // time steps per HBM pass: radius 1 (2 = heat2.cu, 3-4 = heat_tb.cu), radius 2 (2 = heat_tb2.cu, with r2)
     int zchunk2 = 0;       // output planes per unit of the several-step kernels (0 = 16 / 64)
     int tb16 = 0;          // two steps per pass: 0 = heat2.cu (8-warp CTAs), 1 = heat_tb.cu (16 warps)
     int tbn = 0;           // heat_tb.cu tiles: 0 = 128 x 32 cells, 1 = 64 x 64 cells
     int r2 = 0;            // radius 2: 1 = two steps per pass (heat_tb2.cu) when tblock >= 2
+    // The library's own rule for the kernel and the steps per pass, while every
+    // knob has its default: so knobs read from one handle and set on another
+    // choose the same there, and set back they choose the rule again.
+    bool own() const
+    {
+        return zchunk == 0 && ctas_per_sm == 0 && pdl && tblock == 2 && zchunk2 == 0 && !tb16 && !tbn && !r2;
+    }
 };
 
 // One sub-step of every block: units (block, z-chunk, tile row, tile column)

@@ -131,16 +131,16 @@ b2r_status b2r_step(b2r_handle* h, int nsteps);
  * CUDA graphs captured on first use (heat and Game of Life, when the handle
  * has a non-default stream).  Default on; results are identical either way. */
 b2r_status b2r_set_graphs(b2r_handle* h, int enable);
-/* Launch-schedule knobs (the autotuner's search space).  Until one of the heat
- * knobs is set, a heat domain runs on the kernel that the library's own rule
- * picks; setting one selects the sweep that the knob belongs to. */
+/* Launch-schedule knobs (the autotuner's search space).  While every heat knob
+ * has its default value, a heat domain runs on the kernel that the library's own
+ * rule picks; another value selects the sweep that the knob belongs to. */
 enum {
     B2R_TUNE_ZCHUNK = 1,       /* planes per work unit of the one-step sweep (0 = 16) */
     B2R_TUNE_CTAS_PER_SM = 2,  /* 0 = one CTA per unit, k = persistent k CTAs per SM */
     B2R_TUNE_PDL = 3,          /* programmatic dependent launch on / off */
     B2R_TUNE_TBLOCK = 4,       /* time steps per pass: heat of radius 1 takes up to tblock (2, 3
-                                  or 4; default 2) steps per HBM pass.  Until a heat knob is set
-                                  the library chooses: two or three steps by the block size, long
+                                  or 4; default 2) steps per HBM pass.  While every heat
+                                  knob has its default the library chooses: two or three steps by the block size, long
                                   runs on several blocks as one block, small domains in one
                                   cluster's shared memory.  Game of Life (bit-sliced cells, tblock
                                   >= 2): several generations per pass, on the whole domain's bit
