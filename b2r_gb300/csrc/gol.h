@@ -1,6 +1,7 @@
 // gol.h -- internal interface of the Game of Life kernel (gol.cu).
 #pragma once
 #include "b2r_common.cuh"
+#include "gol_plan.h"
 
 namespace b2r {
 
@@ -37,19 +38,6 @@ int gol_bits_max_generations_per_pass();
 // halos between blocks are neither read nor written.  plans: the tiles and
 // generations per pass chosen for this domain, kept by the caller (zeroed at
 // first).
-constexpr int kGolDomainMaxGen = 8;   // generations per pass at most
-struct GolPass {
-    int nx, ny, nz, W;     // cells per axis of the bit grid (shell included), words per row
-    int periodic;
-    int G;                 // generations of this pass
-    int WX, XO, split;     // region words per row, output words, 1: a row is cut into x tiles
-    int Ty, Tz, PR, PZ;    // output rows / planes of a tile, region rows (even) / planes
-    int RP, RPZ;           // shared pitch of a row and of a plane (words)
-    int nzs;               // z segments of a CTA
-    int ntx, nty;
-    int threads;
-    size_t smem;
-};
 struct GolDomainPlans {
     GolPass p[kGolDomainMaxGen + 1] = {};   // by generations to go (at most kGolDomainMaxGen); G = 0: not made yet
 };

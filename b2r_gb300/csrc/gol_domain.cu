@@ -31,6 +31,8 @@
 // measured: 4.9, 4.4, 3.8, 4.1, 4.6, 4.8 us per generation); the integer pipe
 // is 55 % busy over the whole pass.
 #include <algorithm>
+#include <array>
+#include <map>
 #include <mutex>
 
 #include "b2r_common.cuh"
@@ -41,9 +43,8 @@ namespace b2r {
 namespace {
 
 constexpr int kMaxG = kGolDomainMaxGen;
-constexpr int kNR = 2;                    // rows per thread
-constexpr int kMaxThreads = 1024;
-constexpr int kMaxPR = 96, kMaxPZ = 96;   // region rows / planes at most
+constexpr int kNR = kGolRows, kMaxThreads = kGolMaxThreads;
+constexpr int kMaxPR = kGolMaxRegion, kMaxPZ = kGolMaxRegion;
 
 
 // One three-input logic instruction each, by its truth table (bit 4a + 2b + c).  Written out because the compiler
@@ -366,83 +367,23 @@ gol_unpack_kernel(uint8_t* __restrict__ blocks, const uint32_t* __restrict__ bit
     }
 }
 
-// Shared pitch of a row: 2 more than a multiple of 4, so that the rows of
-// the threads of a warp (words fastest, then pairs of rows) spread over the
-// banks; a template argument, so that a thread's loads of a plane share
-// three addresses.
-int row_pitch(int WX) { return WX <= 2 ? 2 : (WX - 2 + 3) / 4 * 4 + 2; }
-
-// Tile and generations of a pass by a cost model (cycles per generation of
-// the busiest SM).  Each generation of a CTA costs its logic operations
-// (about 22 per word, and 20 more for the x and y sums, which a z segment
-// computes for two extra planes), at 64 lanes per cycle and SM, or the chain
-// of one thread where few threads are in flight; a pass costs a launch and
-// the load of its regions on top.
-GolPass plan_pass(const GolPass& base, int left, int sms)
+// The plan of a pass, once per domain and generations to go: kept for the process
+// (512 at most), so that a new domain of a known size has it at hand.
+GolPass plan_of(const GolPass& base, int left, int sms)
 {
-    GolPass best = base;
-    double best_cost = 1e300;
-    for (int G : {4, 6, 8, 3, 5, 2, 1}) {
-        if (G > left) continue;
-        for (int PR = 4; PR <= kMaxPR; PR += PR < 24 ? kNR : 4) {
-            const int Ty = PR - 2 * G;
-            if (Ty < 1) continue;
-            if (Ty >= base.ny + 4) break;
-            const int RP = row_pitch(base.WX);
-            const int nty = (base.ny + Ty - 1) / Ty;
-            for (int nzt = 1; nzt <= base.nz; ++nzt) {
-                const int Tz = (base.nz + nzt - 1) / nzt;
-                if (nzt > 1 && Tz == (base.nz + nzt - 2) / (nzt - 1)) continue;   // same tile as fewer chunks
-                const int PZ = Tz + 2 * G;
-                if (PZ > kMaxPZ) continue;
-                if (Tz < 3 && base.nz > 8) break;
-                // no z split of this tile can beat the best so far
-                const double ctas_all = (double)base.ntx * nty * ((base.nz + Tz - 1) / Tz);
-                const double least = 6000.0 + 150.0 * G + ctas_all / sms * PR * base.WX *
-                                                              ((39.0 / 56.0) * (G * PZ - G * (G + 1)) + 0.55 * PZ);
-                if (least / G >= best_cost) continue;
-                for (int nzs : {4, 2, 3, 6, 8, 12, 16, 1}) {
-                    const int th = base.WX * (PR / kNR) * nzs;
-                    if (th > kMaxThreads || (nzs > 1 && Tz < nzs)) continue;
-                    const size_t bytes = (size_t)2 * PZ * (PR + 2) * RP * 4;
-                    if (bytes > 200 * 1024) continue;
-                    const long long ctas = (long long)base.ntx * nty * ((base.nz + Tz - 1) / Tz);
-                    const int warps = (th + 31) / 32;
-                    const int fit = (int)std::min<size_t>(std::min(2048 / (warps * 32), 65536 / (warps * 32 * 64)),
-                                                          (220 * 1024) / (bytes + 1024));
-                    if (fit < 1) continue;
-                    const long long busiest = (ctas + sms - 1) / sms;
-                    auto together = [&](int n) {   // n CTAs resident on the SM
-                        double c = (double)n * PZ * PR * base.WX * 0.55;               // the load
-                        for (int g = 1; g <= G; ++g) {
-                            const int sz = (PZ - 2 * g + nzs - 1) / nzs;
-                            const double per = kNR * (25.0 * sz + 14.0 * (sz + 2)) + 12.0 * sz;   // per thread
-                            c += std::max(n * warps * 32 * per / 56.0, per * 9.5) + 150.0;
-                        }
-                        return c;
-                    };
-                    double cost = (double)(busiest / fit) * together(fit);
-                    if (busiest % fit) cost += together((int)(busiest % fit));
-                    cost = (cost + 6000.0) / G;
-                    if (cost < best_cost) {
-                        best_cost = cost;
-                        best.G = G;
-                        best.Ty = Ty;
-                        best.Tz = Tz;
-                        best.PR = PR;
-                        best.PZ = PZ;
-                        best.nzs = nzs;
-                        best.nty = nty;
-                    }
-                }
-            }
-        }
+    static std::mutex mu;
+    static std::map<std::array<int, 6>, GolPass> known;
+    const std::array<int, 6> key{base.nx, base.ny, base.nz, base.periodic, left, sms};
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        auto it = known.find(key);
+        if (it != known.end()) return it->second;
     }
-    best.RP = row_pitch(best.WX);
-    best.RPZ = (best.PR + 2) * best.RP;
-    best.smem = (size_t)2 * best.PZ * best.RPZ * 4;
-    best.threads = (best.WX * (best.PR / kNR) * best.nzs + 31) / 32 * 32;
-    return best;
+    const GolPass p = gol_plan_pass(base, left, sms);
+    std::lock_guard<std::mutex> lock(mu);
+    if (known.size() >= 512) known.clear();
+    known[key] = p;
+    return p;
 }
 
 }  // namespace
@@ -459,16 +400,7 @@ cudaError_t launch_gol_domain(uint8_t* blocks, uint32_t* bits, const int env[3],
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    GolPass P{};
-    P.nx = env[0] + 2 * shell;
-    P.ny = env[1] + 2 * shell;
-    P.nz = env[2] + 2 * shell;
-    P.W = (P.nx + 31) / 32;
-    P.periodic = shell ? 0 : 1;
-    P.split = P.W > 32;
-    P.XO = P.split ? 30 : P.W;
-    P.WX = P.split ? 32 : P.W;
-    P.ntx = P.split ? (P.W + P.XO - 1) / P.XO : 1;
+    const GolPass P = gol_pass_rows(env[0] + 2 * shell, env[1] + 2 * shell, env[2] + 2 * shell, shell == 0);
     const bool rag = P.periodic && !P.split && P.nx % 32 != 0;
     uint32_t* grid[2] = {bits, bits + gol_domain_words(env, shell)};
 
@@ -485,12 +417,12 @@ cudaError_t launch_gol_domain(uint8_t* blocks, uint32_t* bits, const int env[3],
     static const Kern kerns[2][9] = {B2R_GOL_PITCHES(false), B2R_GOL_PITCHES(true)};
 #undef B2R_GOL_PITCHES
     static SmemLimit limit[2][9];
-    const int pitch = row_pitch(P.WX) / 4;
+    const int pitch = gol_row_pitch(P.WX) / 4;
     const Kern kern = kerns[rag][pitch];
     int cur = 0;
     for (int left = gens; left > 0;) {
         GolPass& plan = plans.p[std::min(left, kMaxG)];
-        if (plan.G == 0) plan = plan_pass(P, std::min(left, kMaxG), sms);
+        if (plan.G == 0) plan = plan_of(P, std::min(left, kMaxG), sms);
         if ((e = raise_smem_limit(limit[rag][pitch], (const void*)kern, std::max<size_t>(plan.smem, 48 * 1024)))) return e;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(plan.ntx * plan.nty * ((plan.nz + plan.Tz - 1) / plan.Tz)));
