@@ -40,6 +40,8 @@ struct b2r_handle {
     CUtensorMap tmapf[2][3];    // boxes of heat_far.cu's three tile heights
     HeatCoef hc{};
     HeatTune tune{};
+    int own_steps = 1;          // steps per HBM pass by the library's own rule (radius 1)
+    std::map<std::pair<int, int>, HeatTiles> tiles;   // of heat_far.cu (steps 1) and heat_rows.cu, by steps and sub-step
     // heat: the cluster of heat_small.cu that holds the domain and steps it faster
     // (0: none), and the us per step that it saves
     int small_ctas = 0;
@@ -193,7 +195,6 @@ b2r_status ensure_kappa(b2r_handle* h);
 b2r_status ensure_staging(b2r_handle* h, size_t bytes);
 b2r_status build_heat_maps(b2r_handle* h);
 int heat_pass_steps(const b2r_handle* h, int i, int left);
-int heat_own_steps(const b2r_handle* h);
 int gol_pass_gens(const b2r_handle* h, int i, int left);
 b2r_status check_status(b2r_handle* h);
 b2r_status exchange_all(b2r_handle* h, bool staged, cudaStream_t xst = nullptr);   // xst: another stream than the handle's

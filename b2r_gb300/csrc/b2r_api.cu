@@ -126,8 +126,9 @@ b2r_status build_heat_maps(b2r_handle* h)
 // rows per thread (heat_rows.cu, whose tiles are 120 x 44 cells), or two in
 // two-row tiles (heat2.cu) where too few of those fill the GPU, by the
 // estimates of a pass of either.
-int heat_own_steps(const b2r_handle* h)
+static int heat_own_steps(const b2r_handle* h)
 {
+    if (h->cfg.D != 1) return 1;
     if (heat2_us(h->L) / 2 <= heat_rows_us(h->L) / 3) return 2;
     // a period of four steps between exchanges is one pass of four, not three
     // and one (512^3 torus in 2x2x2 blocks: 136 us per step, 157 as 3 + 1)
@@ -139,7 +140,7 @@ int heat_own_steps(const b2r_handle* h)
 int heat_max_pass_steps(const b2r_handle* h)
 {
     if (h->cfg.model != B2R_MODEL_HEAT || h->tune.tblock < 2) return 1;
-    if (h->cfg.D == 1) return h->tune.own() ? heat_own_steps(h) : std::min(h->tune.tblock, 4);
+    if (h->cfg.D == 1) return h->tune.own() ? h->own_steps : std::min(h->tune.tblock, 4);
     return h->cfg.D == 2 && h->tune.r2 ? 2 : 1;
 }
 
@@ -323,7 +324,7 @@ b2r_status substep(b2r_handle* h, int i, bool xnext)
     case B2R_MODEL_HEAT:
         if (h->tune.own())
             CK(h, launch_heat_far(h->tmapf[h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L, h->cfg.D, i, h->hc,
-                                  h->d_status, h->stream));
+                                  h->d_status, h->stream, h->tiles[{1, i}]));
         else
             CK(h, launch_heat_substep(&h->tmap[h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L,
                                   h->cfg.D, i, h->hc, h->d_status, h->stream, h->tune));
@@ -486,9 +487,9 @@ b2r_status advance(b2r_handle* h, int n)
                 CK(h, launch_heat_substep_tb2(&h->tmap3[h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L, i,
                                               h->hc, h->d_status, h->stream, h->tune.zchunk2));
                 h->cur = 1 - h->cur;
-            } else if (h->tune.own() && heat_own_steps(h) > 2) {
+            } else if (h->tune.own() && h->own_steps > 2) {
                 CK(h, launch_heat_rows(k, &h->tmapr[k - 2][h->cur], static_cast<float*>(h->buf[1 - h->cur]), h->L, i,
-                                       h->hc, h->d_status, h->stream));
+                                       h->hc, h->d_status, h->stream, h->tiles[{k, i}]));
                 h->cur = 1 - h->cur;
             } else if (k == 2 && !h->tune.tb16) {
                 if ((st = substep2(h, i)) != B2R_OK) return st;
@@ -891,6 +892,7 @@ b2r_status create_handle(const b2r_config* cfg, b2r_handle** out, b2r_handle* ow
         cudaGetLastError();   // a failed allocation must not surface in the caller's next launch check
         return s;
     };
+    if (c.model == B2R_MODEL_HEAT) h->own_steps = heat_own_steps(h);
     if (owner) {                       // a one-block form has its owner's memory and status word
         h->d_status = owner->d_status;
         if (c.model == B2R_MODEL_HEAT) {

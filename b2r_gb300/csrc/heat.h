@@ -101,19 +101,28 @@ int heat_tb_box_h(int narrow);
 cudaError_t launch_heat_substep_tb(int T, int narrow, const CUtensorMap* tin, float* out, const BlockLayout& L,
                                    int step_i, const HeatCoef& c, int* status, cudaStream_t st, int zchunk);
 
+// The tiles of a launch over the union of the blocks' windows; kept by the
+// caller for the same layout and sub-step (rows = 0: not made yet), since the
+// search goes through every block and z chunk.
+struct HeatTiles {
+    int rows = 0;                   // computed rows of a tile
+    int ntx, nty, nzc, Lz;
+    int x0, y0, z0;                 // storage x, row and plane of the windows' first cells
+};
+
 // T = 2, 3 or 4 sub-steps (step_i .. step_i+T-1) of radius 1 per launch, four
 // rows per thread (heat_rows.cu).  The tensor map must have the box
 // heat_rows_box_w() x heat_rows_box_h(T).
 int heat_rows_box_w();
 int heat_rows_box_h(int T);
 cudaError_t launch_heat_rows(int T, const CUtensorMap* tin, float* out, const BlockLayout& L, int step_i,
-                             const HeatCoef& c, int* status, cudaStream_t st);
+                             const HeatCoef& c, int* status, cudaStream_t st, HeatTiles& tiles);
 
 // One sub-step of radius D = 1 .. 4 (heat_far.cu).  tin: three tensor maps
 // over the input, with boxes of heat_far_box_w() x heat_far_box_h(D, k) cells.
 int heat_far_box_w();
 int heat_far_box_h(int D, int k);
 cudaError_t launch_heat_far(const CUtensorMap* tin, float* out, const BlockLayout& L, int D, int step_i,
-                            const HeatCoef& c, int* status, cudaStream_t st);
+                            const HeatCoef& c, int* status, cudaStream_t st, HeatTiles& tiles);
 
 }  // namespace b2r

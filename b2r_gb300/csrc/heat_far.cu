@@ -43,15 +43,10 @@ struct FCfg {
     static constexpr size_t SMEM = (size_t)S * SLOT * 4 + 2 * S * 8 + 128;
 };
 
-struct FSched {
-    int ntx, nty, nzc, Lz;
-    int x0, y0, z0;     // storage x, row and plane of the first tile: the windows' first cells
-};
-
 template <int D, int NC>
 __global__ void __launch_bounds__(32 * (NC + 1), NC <= 7 ? 2 : 1)
 heat_far_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ out, const BlockLayout L,
-                const int step_i, const HeatCoef C, const FSched sch, int* __restrict__ status)
+                const int step_i, const HeatCoef C, const HeatTiles sch, int* __restrict__ status)
 {
     using Cfg = FCfg<D, NC>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -158,30 +153,26 @@ FPlan f_plan(int nblk, int D, int ntx, int NY, int NZ, int sms)
 }
 
 template <int D, int NC>
-cudaError_t launch_f(const CUtensorMap* tin, float* out, const BlockLayout& L, FSched sch, int NY, int NZ, int step_i,
+cudaError_t launch_f(const CUtensorMap* tin, float* out, const BlockLayout& L, const HeatTiles& sch, int step_i,
                      const HeatCoef& c, int* status, cudaStream_t st)
 {
     using Cfg = FCfg<D, NC>;
     static KernelSetup setup;
     if (cudaError_t e = kernel_setup(setup, heat_far_kernel<D, NC>, Cfg::THR, Cfg::SMEM, nullptr, nullptr)) return e;
-    sch.nty = (NY + Cfg::TH - 1) / Cfg::TH;
-    sch.nzc = (NZ + sch.Lz - 1) / sch.Lz;
     return launch_pdl(heat_far_kernel<D, NC>, (unsigned)((long long)sch.ntx * sch.nty * sch.nzc * L.nblk), Cfg::THR,
                       Cfg::SMEM, st, *tin, out, L, step_i, c, sch, status);
 }
 
-template <int D>
-cudaError_t launch_d(const CUtensorMap* tin, float* out, const BlockLayout& L, int step_i, const HeatCoef& c,
-                     int* status, cudaStream_t st)
+// Tiles over the union of the blocks' windows, which shrink from sub-step to
+// sub-step: 250 cells take two tile columns where 258 take three
+// (250x186x132 torus as one block, radius 2, three steps between exchanges:
+// 670 us for 48 steps against 716 with tiles over all that a period computes).
+cudaError_t f_tiles(const BlockLayout& L, int D, int step_i, HeatTiles& sch)
 {
     int dev = 0, sms = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    // tiles over the union of the blocks' windows, which shrink from sub-step to
-    // sub-step: 250 cells take two tile columns where 258 take three
-    // (250x186x132 torus as one block, radius 2, three steps between exchanges:
-    // 670 us for 48 steps against 716 with tiles over all that a period computes)
     int lo[3] = {1 << 30, 1 << 30, 1 << 30}, hi[3] = {-1, -1, -1};
     for (int b = 0; b < L.nblk; ++b)
         for (int a = 0; a < 3; ++a) {
@@ -190,20 +181,36 @@ cudaError_t launch_d(const CUtensorMap* tin, float* out, const BlockLayout& L, i
             lo[a] = std::min(lo[a], l);
             hi[a] = std::max(hi[a], h);
         }
-    if (hi[0] < lo[0] || hi[1] < lo[1] || hi[2] < lo[2]) return cudaSuccess;
-    FSched sch;
+    sch = HeatTiles{};
     sch.x0 = (L.xoff + lo[0]) & ~3;
     sch.y0 = lo[1];
     sch.z0 = lo[2];
-    sch.ntx = (L.xoff + hi[0] - sch.x0) / kTW + 1;
     const int NY = hi[1] - lo[1] + 1, NZ = hi[2] - lo[2] + 1;
+    if (hi[0] < lo[0] || NY < 1 || NZ < 1) {
+        sch.rows = 1;        // nothing to compute
+        return cudaSuccess;
+    }
+    sch.ntx = (L.xoff + hi[0] - sch.x0) / kTW + 1;
     const FPlan p = f_plan(L.nblk, D, sch.ntx, NY, NZ, sms);
+    sch.rows = p.rows;
     sch.Lz = p.lz;
+    sch.nty = (NY + p.rows - 1) / p.rows;
+    sch.nzc = (NZ + p.lz - 1) / p.lz;
+    return cudaSuccess;
+}
+
+template <int D>
+cudaError_t launch_d(const CUtensorMap* tin, float* out, const BlockLayout& L, int step_i, const HeatCoef& c,
+                     int* status, cudaStream_t st, HeatTiles& sch)
+{
+    if (!sch.rows)
+        if (cudaError_t e = f_tiles(L, D, step_i, sch)) return e;
     // rows of the tile by the tensor map's box: tin[0], [1], [2] for 30, 22, 14
-    switch (p.rows) {
-    case 30: return launch_f<D, 15>(&tin[0], out, L, sch, NY, NZ, step_i, c, status, st);
-    case 22: return launch_f<D, 11>(&tin[1], out, L, sch, NY, NZ, step_i, c, status, st);
-    default: return launch_f<D, 7>(&tin[2], out, L, sch, NY, NZ, step_i, c, status, st);
+    switch (sch.rows) {
+    case 30: return launch_f<D, 15>(&tin[0], out, L, sch, step_i, c, status, st);
+    case 22: return launch_f<D, 11>(&tin[1], out, L, sch, step_i, c, status, st);
+    case 14: return launch_f<D, 7>(&tin[2], out, L, sch, step_i, c, status, st);
+    default: return cudaSuccess;
     }
 }
 
@@ -213,13 +220,13 @@ int heat_far_box_w() { return kTW + 8; }
 int heat_far_box_h(int D, int k) { return (k == 0 ? 30 : k == 1 ? 22 : 14) + 2 * D; }
 
 cudaError_t launch_heat_far(const CUtensorMap* tin, float* out, const BlockLayout& L, int D, int step_i,
-                            const HeatCoef& c, int* status, cudaStream_t st)
+                            const HeatCoef& c, int* status, cudaStream_t st, HeatTiles& tiles)
 {
     switch (D) {
-    case 1: return launch_d<1>(tin, out, L, step_i, c, status, st);
-    case 2: return launch_d<2>(tin, out, L, step_i, c, status, st);
-    case 3: return launch_d<3>(tin, out, L, step_i, c, status, st);
-    case 4: return launch_d<4>(tin, out, L, step_i, c, status, st);
+    case 1: return launch_d<1>(tin, out, L, step_i, c, status, st, tiles);
+    case 2: return launch_d<2>(tin, out, L, step_i, c, status, st, tiles);
+    case 3: return launch_d<3>(tin, out, L, step_i, c, status, st, tiles);
+    case 4: return launch_d<4>(tin, out, L, step_i, c, status, st, tiles);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -48,11 +48,6 @@ struct RCfg {
     static constexpr size_t SMEM = (size_t)kSlots * SLOT * 4 + (size_t)(T - 1) * 2 * XE * 4 + kSlots * 8 + 128;
 };
 
-struct RSched {
-    int ntx, nty, nzc, Lz;
-    int x0, y0, z0;     // storage x, row and plane of the first stored cells: the windows' first
-};
-
 __device__ __forceinline__ float4 rld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void rst4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 
@@ -178,7 +173,7 @@ __device__ __forceinline__ bool r_iter(RCtx<T, NW>& c, int pr)
 template <int T, int NW>
 __global__ void __launch_bounds__(32 * NW, 1)
 heat_rows_kernel(const __grid_constant__ CUtensorMap tin, float* __restrict__ out, const BlockLayout L,
-                 const int step_i, const HeatCoef C, const RSched sch, int* __restrict__ status)
+                 const int step_i, const HeatCoef C, const HeatTiles sch, int* __restrict__ status)
 {
     using Cfg = RCfg<T, NW>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -297,7 +292,7 @@ int r_chunk(long long tiles, int NZ, int T, int sms, long long& least)
 }
 
 template <int T, int NW>
-RSched r_sched(const BlockLayout& L, int step_i, int sms, long long& cost)
+HeatTiles r_sched(const BlockLayout& L, int step_i, int sms, long long& cost)
 {
     // tiles over the union of the blocks' windows after the pass
     int lo[3] = {1 << 30, 1 << 30, 1 << 30}, hi[3] = {-1, -1, -1};
@@ -308,7 +303,8 @@ RSched r_sched(const BlockLayout& L, int step_i, int sms, long long& cost)
             lo[a] = std::min(lo[a], l);
             hi[a] = std::max(hi[a], h);
         }
-    RSched sch;
+    HeatTiles sch;
+    sch.rows = RCfg<T, NW>::ROWS;
     sch.x0 = (L.xoff + lo[0]) & ~3;
     sch.y0 = lo[1];
     sch.z0 = lo[2];
@@ -322,16 +318,16 @@ RSched r_sched(const BlockLayout& L, int step_i, int sms, long long& cost)
 
 template <int T, int NW>
 cudaError_t launch_r(const CUtensorMap* tin, float* out, const BlockLayout& L, int step_i, const HeatCoef& c,
-                     int* status, cudaStream_t st)
+                     int* status, cudaStream_t st, HeatTiles& sch)
 {
     using Cfg = RCfg<T, NW>;
     static KernelSetup setup;
     int total = 0;      // one CTA per SM
     if (cudaError_t e = kernel_setup(setup, heat_rows_kernel<T, NW>, 32 * NW, Cfg::SMEM, nullptr, &total)) return e;
     long long cost;
-    const RSched sch = r_sched<T, NW>(L, step_i, total, cost);
-    return launch_pdl(heat_rows_kernel<T, NW>, (unsigned)((long long)sch.ntx * sch.nty * L.nblk * sch.nzc), 32 * NW, Cfg::SMEM, st, *tin, out, L, step_i,
-                      c, sch, status);
+    if (!sch.rows) sch = r_sched<T, NW>(L, step_i, total, cost);
+    return launch_pdl(heat_rows_kernel<T, NW>, (unsigned)((long long)sch.ntx * sch.nty * L.nblk * sch.nzc), 32 * NW,
+                      Cfg::SMEM, st, *tin, out, L, step_i, c, sch, status);
 }
 
 constexpr int kNW2 = 12, kNW3 = 12, kNW4 = 8;   // warps by steps per pass
@@ -349,12 +345,12 @@ double heat_rows_us(const BlockLayout& L)
 int heat_rows_box_h(int T) { return kRY * (T == 2 ? kNW2 : T == 3 ? kNW3 : kNW4) + 2; }
 
 cudaError_t launch_heat_rows(int T, const CUtensorMap* tin, float* out, const BlockLayout& L, int step_i,
-                             const HeatCoef& c, int* status, cudaStream_t st)
+                             const HeatCoef& c, int* status, cudaStream_t st, HeatTiles& tiles)
 {
     switch (T) {
-    case 2: return launch_r<2, kNW2>(tin, out, L, step_i, c, status, st);
-    case 3: return launch_r<3, kNW3>(tin, out, L, step_i, c, status, st);
-    case 4: return launch_r<4, kNW4>(tin, out, L, step_i, c, status, st);
+    case 2: return launch_r<2, kNW2>(tin, out, L, step_i, c, status, st, tiles);
+    case 3: return launch_r<3, kNW3>(tin, out, L, step_i, c, status, st, tiles);
+    case 4: return launch_r<4, kNW4>(tin, out, L, step_i, c, status, st, tiles);
     default: return cudaErrorInvalidValue;
     }
 }
