@@ -767,12 +767,12 @@ b2r_status capture_graph(b2r_handle* h, int c, int periods)
 {
     const int save_cur = h->cur;
     const long long save_ts = h->ts;
-    const bool save_fresh = h->halos_fresh;
-    h->cur = c;
-    h->ts = 0;
-    h->halos_fresh = false;
+    const bool save_fresh = h->halos_fresh, save_lost = h->halos_lost;
     const long long k0 = b2r_kernel_launches();
     CK(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+    h->cur = c;
+    h->ts = 0;
+    h->halos_fresh = h->halos_lost = false;
     b2r_status st = advance(h, periods * h->cfg.R);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
@@ -782,14 +782,22 @@ b2r_status capture_graph(b2r_handle* h, int c, int periods)
     h->cur = save_cur;
     h->ts = save_ts;
     h->halos_fresh = save_fresh;
+    h->halos_lost = save_lost;
     if (st != B2R_OK) {
         if (g) cudaGraphDestroy(g);
         return st;
     }
-    if (e != cudaSuccess) return fail(h, B2R_ERR_CUDA, "stream capture: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(h, B2R_ERR_CUDA, "stream capture: %s", cudaGetErrorString(e));
+    }
     e = cudaGraphInstantiate(&h->gexec[c], g, 0);
     cudaGraphDestroy(g);
-    if (e != cudaSuccess) return fail(h, B2R_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        h->gexec[c] = nullptr;
+        return fail(h, B2R_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
+    }
     h->gkernels = nk;
     return B2R_OK;
 }
