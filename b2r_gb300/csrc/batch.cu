@@ -216,13 +216,14 @@ __global__ void __launch_bounds__(kQThreads, 2) batch_far_kernel(const BatchArgs
                 for (int c = max(0, zc - reach) + lane; ok && c <= min(in.nzc - 1, zc + reach); c += 32)
                     ok = wq::wait_done(&a.done[in.done0 + c], (unsigned)q.t * (unsigned)tiles * (unsigned)kQC);
                 ok = __all_sync(0xffffffffu, ok);
+                __syncwarp();                // a vote orders no memory: what the other lanes acquired, before lane 0's loads
             }
             if (lane == 0) {
                 const int zs = D + zc * in.Lz, ze = min(D + (zc + 1) * in.Lz - 1, in.L.n[2] - 1 - D);
                 const int np = ze - zs + 1 + 2 * D, xs0 = ((in.L.xoff + D) & ~3) + tx * 4 * in.lpr;
                 const unsigned bytes = (unsigned)(bw * (th + 2 * D)) * 4u;
                 const CUtensorMap* map = &a.maps[2 * q.k + (q.t & 1)];
-                asm volatile("fence.proxy.async.global;" ::: "memory");   // what the other lanes waited for, too
+                asm volatile("fence.proxy.async.global;" ::: "memory");
                 for (int p = 0; p < np && ok; ++p, ++i) {
                     if (i >= kQS) ok = mbar_wait_bounded(&empty[slot], phase ^ 1);
                     if (!ok) break;
