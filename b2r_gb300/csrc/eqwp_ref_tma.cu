@@ -290,7 +290,7 @@ cudaError_t launch_stage(const EqwpRefMaps& maps, RefArgs A, const BlockLayout& 
     }
     // z chunks: the fewest planes on the busiest SM, four of them to start a chunk
     double least = 1e300;
-    for (int k = 1; k <= std::max(1, nz / 8); ++k) {
+    for (int k = 1; k <= std::max(1, std::min(nz / 8, 65535 / L.nblk)); ++k) {
         const double cost = (double)((tiles * k + sms - 1) / sms) * ((nz + k - 1) / k + 4);
         if (cost < least - 1e-9) {
             least = cost;

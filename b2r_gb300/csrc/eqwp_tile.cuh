@@ -439,7 +439,7 @@ inline Grid stage_grid(const BlockLayout& L, int shrink, int per_sm = B2R_EQWP_M
     const long long tiles = (long long)tx * ty * L.nblk;
     const int nz = std::max(1, hi[2] - lo[2] + 1);
     const int lz = chunk(tiles, nz, per_sm);
-    const int nzc = (nz + lz - 1) / lz;
+    const int nzc = std::max(1, std::min((nz + lz - 1) / lz, 65535 / L.nblk));   // a grid has at most 65535 along z
     r.t.nzc = nzc;
     r.g = dim3(tx, ty, L.nblk * nzc);
     return r;
