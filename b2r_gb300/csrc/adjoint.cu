@@ -116,10 +116,7 @@ struct AdjS {
 };
 __device__ __forceinline__ void inject(const AdjS& A)
 {
-    const long long threads = blockDim.x * blockDim.y;
-    for (long long r = grid_cta() * threads + threadIdx.y * blockDim.x + threadIdx.x; r < A.nrec;
-         r += threads * gridDim.x * gridDim.y * gridDim.z)
-        atomicAdd(&A.vby[A.rec[r]], A.res[r]);
+    for (unsigned r = grid_thread(); r < (unsigned)A.nrec; r += grid_threads()) atomicAdd(&A.vby[A.rec[r]], A.res[r]);
 }
 
 // Adjoint of the stress stage of step n followed by the velocity-stage

@@ -342,10 +342,16 @@ __device__ __forceinline__ void st4(float* f, const Cell& c, const float (&v)[4]
     }
 }
 
-// the CTA's number in the launch
-__device__ __forceinline__ long long grid_cta()
+// the thread's number in a stage launch, and its threads (fewer than 2^31: they
+// have four cells each at least)
+__device__ __forceinline__ unsigned grid_thread()
 {
-    return blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
+    return ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * (blockDim.x * blockDim.y) +
+           threadIdx.y * blockDim.x + threadIdx.x;
+}
+__device__ __forceinline__ unsigned grid_threads()
+{
+    return gridDim.x * gridDim.y * gridDim.z * (blockDim.x * blockDim.y);
 }
 
 // Tile origin of a stage launch: the first tile starts at the lowest window

@@ -84,12 +84,8 @@ heat_kappa_step_kernel(const float* __restrict__ in, float* __restrict__ out, co
                        float* __restrict__ rec_out)
 {
     pdl_begin();
-    if (rec_out) {
-        const long long threads = blockDim.x * blockDim.y;
-        for (long long r = grid_cta() * threads + threadIdx.y * blockDim.x + threadIdx.x; r < nrec;
-             r += threads * gridDim.x * gridDim.y * gridDim.z)
-            rec_out[r] = in[rec[r]];
-    }
+    if (rec_out)
+        for (unsigned r = grid_thread(); r < (unsigned)nrec; r += grid_threads()) rec_out[r] = in[rec[r]];
     const Win w = window(L, 0, blockIdx.z, T.nzc, L.H);
     Cell cell;
     if (!cell_setup(L, w, 0, cell, T.x0, T.y0)) return;
