@@ -380,7 +380,7 @@ struct Grid {
 // neighbouring chunks cost more (512x512x256 in four blocks: 154 ms per 100
 // steps with 16 planes, 155.6 with 8).  Measured us per
 // elastic-wave step (two stages) against chunks of at least 16 planes: 32^3
-// 12.5 from 45, 64^3 13 from 49, 96^3 23 from 49, 128^3 56 from 82, 192^3 172
+// 6.9 from 45, 64^3 9.0 from 49, 96^3 18 from 49, 128^3 51 from 82, 192^3 168
 // from 194, 256^3 361 from 388 (by planes 1, 2, 3, 4, 6, 8, 12, 16 there:
 // 426, 402, 370, 360, 354, 361, 373, 388).  per_sm: resident CTAs per SM.
 inline int stage_chunk(long long tiles, int nz, int per_sm)

@@ -25,7 +25,7 @@
 //
 // Measured, 256^3 torus in 2x2x2 blocks, R = 4: 3.8 us per generation against
 // 17.1 for the several-generation block pass with its halo gather (400
-// generations with upload and download 1.57 ms against 7.02); 512^3 with a
+// generations with upload and download 1.63 ms against 7.02); 512^3 with a
 // shell 27 against 56; 64^3 torus 1.3 against 14.7.  A pass of four
 // generations takes 15.5 us, about 5 of them launch and load (G = 2 to 8
 // measured: 4.9, 4.4, 3.8, 4.1, 4.6, 4.8 us per generation); the integer pipe

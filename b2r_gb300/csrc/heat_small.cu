@@ -1,5 +1,5 @@
 // heat_small.cu -- any number of heat time steps of a small domain in one
-// launch, radius 1..4: the domain lives in the shared memory of one cluster.
+// launch, radius 1 and 2: the domain lives in the shared memory of one cluster.
 //
 // A step of a small domain is all latency: a launch, its loads and its drain
 // (1.86 us at 48x40x32, two steps per launch) for 0.1 us of arithmetic.  Here a

@@ -78,7 +78,7 @@ WORKLOADS = {
                        nrec=64, ckpt=50, f0=12.0, bytes_per_cell=84, kernel="adjoint"),
     # the reference's collocated elastic-wave model, 512x512x256, one block, R = 1
     "eqwp_ref": dict(model=3, env=(512, 512, 256), blocks=(1, 1, 1), R=1, D=2, sub_steps=100,
-                     bytes_per_cell=80, kernel="eqwp_ref_stress+velocity"),
+                     bytes_per_cell=80, kernel="eqwp_ref_tma_kernel (both stages)"),
     # staggered elastic wave 512x512x256, 2x2x1 subdomains, R = 2, 100 steps per pass
     "eqwp_stag": dict(model=4, env=(512, 512, 256), blocks=(2, 2, 1), R=2, D=2, sub_steps=100,
                       bytes_per_cell=84, kernel="eqwp_stag_velocity+stress"),
@@ -450,6 +450,7 @@ def run_batch(args, wl):
         bt.upload(i, a)
     tuned = bt.autotune()
     widths = bt.instance_tiles()
+    kernel = wl["kernel"] if 2 in bt.instance_pass_steps() else "batch_far_kernel<1..4>, a launch per radius"
     # instances per tile width and on two-step units, as the autotuner left
     # them (per order and size class)
     tuned_tile = {str(w): widths.count(w) for w in (128, 64, 32) if w in widths}
@@ -532,7 +533,7 @@ def run_batch(args, wl):
             "e2e": None, "gpu_launches": int(launches),
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "traffic": None, "peak_source": peak_src,
-                         "kernel": "batch_kernel", "note": "8 B per lattice-site update, whole run"},
+                         "kernel": kernel, "note": "8 B per lattice-site update, whole run"},
             "cpu_baseline": None, "clocks": clk, "parity": parity}
     return line
 
@@ -971,7 +972,7 @@ def run_ours(args, wl):
         # the library's own rule: no knob of the heat schedules set
         knobs = tuned or tune or {}
         own = knobs.get("tblock", 2) == 2 and not any(knobs.get(k) for k in ("zchunk", "ctas_per_sm", "zchunk2", "tb16",
-                                                                             "tb_narrow", "tb_r2"))
+                                                                             "tb_narrow", "tb_r2")) and knobs.get("pdl", 1)
         rows = own and steps_per_launch > 2
         kern = ("heat_rows_kernel (three time steps per launch, 120 x 44-cell tiles)" if rows else
                 f"heat_far_kernel<{wl['D']}>" if own and steps_per_launch < 1.5 else
