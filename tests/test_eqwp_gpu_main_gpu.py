@@ -1,4 +1,4 @@
-"""The collocated model's own period driver (b2r_eqwp_gpu_main) between steps of
+"""The collocated model's own entry for a period (b2r_eqwp_gpu_main) between steps of
 several blocks: the fields move on without an exchange, so the next step has to
 start with one, whether the halos were fresh from an upload, from the caller's
 exchange, or brought up to date after a long run."""
