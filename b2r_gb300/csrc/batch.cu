@@ -735,34 +735,26 @@ b2r_status b2r_batch_create(const b2r_batch_item* items, int n, b2r_batch** out)
         cudaMalloc(&b->d_status, sizeof(int)) != cudaSuccess)
         return bail(bfail(B2R_ERR_OOM, "batch table allocation failed"));
     cudaMemset(b->d_status, 0, sizeof(int));
-    for (int k = 0; k < 3; ++k)
+    // a launch per radius, the first on the caller's stream
+    bool has[5] = {};
+    for (const b2r_batch_item& it : b->items) has[it.D] = true;
+    const int sides = has[1] + has[2] + has[3] + has[4] - 1;
+    for (int k = 0; k < sides; ++k)
         if (cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming) != cudaSuccess)
             return bail(bfail(B2R_ERR_CUDA, "batch streams"));
-    if (cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess)
+    if (sides > 0 && cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess)
         return bail(bfail(B2R_ERR_CUDA, "batch streams"));
     // persistent grid: every resident slot
     b->smem = kSmem + 16 + kSmemS1;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    {
-        // the limit is per function and device: only ever raised, so that a
-        // batch with a smaller schedule does not lower it under one created
-        // before it
-        static SmemLimit limit[5];
-        const void* fns[5] = {(const void*)batch_far_kernel<1>, (const void*)batch_far_kernel<2>,
-                              (const void*)batch_far_kernel<3>, (const void*)batch_far_kernel<4>,
-                              (const void*)batch_kernel};
-        for (int v = 0; v < 5; ++v) {
-            int occ = 0;
-            const size_t smem = v < 4 ? kQSmem : b->smem;
-            if (raise_smem_limit(limit[v], fns[v], smem) != cudaSuccess)
-                return bail(bfail(B2R_ERR_CUDA, "smem attribute"));
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fns[v], v < 4 ? kQThreads : kThreads, smem);
-            b->grid[v] = std::max(1, occ) * std::max(1, sms);
-        }
-    }
+    static KernelSetup setup[5];
+    using Kernel = void (*)(BatchArgs);
+    static const Kernel kerns[5] = {batch_far_kernel<1>, batch_far_kernel<2>, batch_far_kernel<3>, batch_far_kernel<4>,
+                                    batch_kernel};
+    for (int v = 0; v < 5; ++v)
+        if (kernel_setup(setup[v], kerns[v], v < 4 ? kQThreads : kThreads, v < 4 ? kQSmem : b->smem, nullptr, &b->grid[v]) !=
+            cudaSuccess)
+            return bail(bfail(B2R_ERR_CUDA, "smem attribute"));
     b2r_status st = apply_shapes(b, default_shapes(b, false));
     if (st != B2R_OK) return bail(st);
     if (cudaDeviceSynchronize() != cudaSuccess) return bail(bfail(B2R_ERR_CUDA, "batch set-up failed"));
