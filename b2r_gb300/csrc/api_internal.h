@@ -51,6 +51,7 @@ struct b2r_handle {
     // (step_joined) and the spare ones; blocks_of: its owner
     b2r_handle* joined = nullptr;
     const b2r_handle* blocks_of = nullptr;
+    void* spare_mem = nullptr;
     float* spare[kMaxFields] = {};
     int nspare = 0;
     size_t spare_bytes = 0;      // counted in the process's share (take_spare)

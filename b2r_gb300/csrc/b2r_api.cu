@@ -579,20 +579,24 @@ bool joined_config(const b2r_handle* h, b2r_config& c)
 // in place and cannot do without.
 constexpr size_t kSpareOne = 256u << 20, kSpareAll = 1u << 30;
 std::atomic<size_t> g_spare{0};
-// n buffers of fb bytes: all of them, or as many as there is room for
+// n buffers of fb bytes in one allocation, or
+// unless `all` as many as a domain may have; 0: none.  What lies outside the cells
+// that a run copies into them is never used.
 int take_spare(b2r_handle* h, int n, size_t fb, bool all)
 {
+    fb = (fb + 255) & ~(size_t)255;
     while (n > 0 && n * fb > kSpareOne) n = all ? 0 : n - 1;
     if (!n) return 0;
-    if (g_spare.fetch_add(n * fb) + n * fb > kSpareAll) {
+    if (g_spare.fetch_add(n * fb) + n * fb > kSpareAll || cudaMalloc(&h->spare_mem, n * fb) != cudaSuccess) {
+        cudaGetLastError();
+        h->spare_mem = nullptr;
         g_spare.fetch_sub(n * fb);
         return 0;
     }
     h->spare_bytes = n * fb;
-    while (h->nspare < n && cudaMalloc(&h->spare[h->nspare], fb) == cudaSuccess) cudaMemset(h->spare[h->nspare++], 0, fb);
-    cudaGetLastError();
-    while (all && h->nspare < n && h->nspare > 0) cudaFree(h->spare[--h->nspare]), h->spare[h->nspare] = nullptr;
-    return h->nspare;
+    for (h->nspare = 0; h->nspare < n; ++h->nspare)
+        h->spare[h->nspare] = reinterpret_cast<float*>(static_cast<char*>(h->spare_mem) + h->nspare * fb);
+    return n;
 }
 
 void make_joined(b2r_handle* h, const b2r_config& c, size_t room)
@@ -617,9 +621,13 @@ void make_joined(b2r_handle* h, const b2r_config& c, size_t room)
     default:
         ok = fb <= room;
         if (ok && !take_spare(h, h->nfld, fb, false)) {
-            h->nspare = cudaMalloc(&h->spare[0], fb) == cudaSuccess;
-            ok = h->nspare > 0;
-            cudaGetLastError();
+            ok = cudaMalloc(&h->spare_mem, fb) == cudaSuccess;
+            if (!ok) {
+                cudaGetLastError();
+                h->spare_mem = nullptr;
+            }
+            h->spare[0] = static_cast<float*>(h->spare_mem);
+            h->nspare = ok;
         }
         for (int f = 0; f < h->nfld && ok; ++f) j->fld[f] = f < h->nspare ? h->spare[f] : h->fld[f - h->nspare];
     }
@@ -1008,8 +1016,7 @@ b2r_status b2r_destroy(b2r_handle* h)
         return B2R_OK;
     }
     b2r_destroy(h->joined);
-    for (float* p : h->spare)
-        if (p) cudaFree(p);
+    if (h->spare_mem) cudaFree(h->spare_mem);
     g_spare.fetch_sub(h->spare_bytes);
     if (h->adj_ws) cudaFree(h->adj_ws);
     for (int b = 0; b < 2; ++b)
